@@ -234,10 +234,11 @@ typedef struct {
   int32_t bp_kernel;      /* matched backprojection of det_v-along-z angles:
                              1: z-lane warps over a column-major weighted
                              sinogram, 0: voxel-pair threads over a row-major one */
-  int32_t bp_shape;       /* z-lane warp shape (voxels along the in-plane axis x
-                             voxels along z per lane x warps per block):
-                             0: 4x8x4, 1: 4x8x8, 2: 4x16x8, 3: 4x16x16,
-                             4: 3x16x8, 5: 4x4x4, 6: 4x2x4 */
+  int32_t bp_shape;       /* z-lane warp shape: 0, 1, 2: chosen from the volume's
+                             z extent (at most 8 voxels along z per lane);
+                             3: 4-voxel windows, 16 planes per block and 4:
+                             3-voxel windows, where lanes hold 8 voxels; 5, 6:
+                             at most 4 and 2 voxels along z per lane */
   int32_t bp_general;     /* matched backprojection of the other angles (tilted
                              detectors): 0: blocks over voxel boxes that stage
                              each angle's detector region in shared memory,

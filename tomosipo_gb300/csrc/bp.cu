@@ -1382,9 +1382,13 @@ int launch_bp_sep_multi(const BpMulti& m, bool a_is_x, void* stream_) {
 
 bool bp_batch_multi_eligible(const tsgb_projector* p) {
   int gx = 0, gy = 0;
-  return !p->fine && !bp_uses_zlane(p) && !p->fine_rows && p->n_general_bp == 0 &&
-         p->n_separable_bp > 0 && bp_sep_blocks(p, true, &gx, &gy) >= 0 &&
-         bp_sep_blocks(p, false, &gx, &gy) >= 0;
+  if (p->fine || p->n_general_bp > 0 || p->n_separable_bp == 0) return false;
+  return bp_uses_zlane(p) || (!p->fine_rows && bp_sep_blocks(p, true, &gx, &gy) >= 0 &&
+                              bp_sep_blocks(p, false, &gx, &gy) >= 0);
+}
+
+int64_t bp_batch_item_bytes(const tsgb_projector* p) {
+  return bp_pairs_bytes(p->g) + (bp_uses_zlane(p) ? bp_scratch_bytes(p) : 0);
 }
 
 int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* sino, int64_t n,
@@ -1397,6 +1401,17 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
   const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - p->n_sep_ax;
   for (int64_t i0 = 0; i0 < n; i0 += group) {
     const int m = int(std::min<int64_t>(group, n - i0));
+    if (bp_uses_zlane(p)) {
+      for (int k = 0; k < m; ++k)
+        launch_bp_weight_z(p, sino + (i0 + k) * sino_elems,
+                           reinterpret_cast<float*>(workspace + k * item_bytes), 0, g.nangles,
+                           stream);
+      launch_bp_zlane_separable(p, 0, n_ax, n_ax, n_ay, reinterpret_cast<const float*>(workspace),
+                                reinterpret_cast<float*>(workspace + bp_pairs_bytes(g)),
+                                vol + i0 * vol_elems, additive ? 1 : 0, nullptr, stream, m,
+                                item_bytes);
+      continue;
+    }
     for (int k = 0; k < m; ++k)
       launch_bp_weight_rows(p, sino + (i0 + k) * sino_elems,
                             reinterpret_cast<float2*>(workspace + k * item_bytes), 0, g.nangles,

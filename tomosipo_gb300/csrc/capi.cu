@@ -28,6 +28,7 @@ void free_device(tsgb_projector* p) {
   if (p->d_params) cudaFree(p->d_params);
   if (p->d_columns) cudaFree(p->d_columns);
   if (p->d_sep_angles) cudaFree(p->d_sep_angles);
+  if (p->d_solve) cudaFree(p->d_solve);
   if (p->d_gen_angles) cudaFree(p->d_gen_angles);
   if (p->d_bil_fast) cudaFree(p->d_bil_fast);
   if (p->d_bil_slow) cudaFree(p->d_bil_slow);
@@ -36,6 +37,7 @@ void free_device(tsgb_projector* p) {
   p->d_params = nullptr;
   p->d_columns = nullptr;
   p->d_sep_angles = nullptr;
+  p->d_solve = nullptr;
   p->d_gen_angles = nullptr;
 }
 
@@ -121,7 +123,13 @@ int tsgb_projector_create(const tsgb_volume_desc* vol, const tsgb_projection_des
   if (e == cudaSuccess) e = upload(&p->d_columns, columns);
   p->host_sep_angles = sep;
   p->host_gen_angles = gen;
+  std::vector<tsgb::SolveEntry> solve;
+  for (int t : sep) {
+    const tsgb::AngleParams& ap = p->host_params[t];
+    solve.push_back({ap.ca[0], ap.ca[1], ap.ma[0], ap.ma[1], ap.e[0], ap.e[1], t, 0});
+  }
   if (e == cudaSuccess) e = upload(&p->d_sep_angles, sep);
+  if (e == cudaSuccess) e = upload(&p->d_solve, solve);
   if (e == cudaSuccess) e = upload(&p->d_gen_angles, gen);
   if (e == cudaSuccess) e = upload(&p->d_bil_fast, bfast);
   if (e == cudaSuccess) e = upload(&p->d_bil_slow, bslow);
@@ -162,7 +170,10 @@ int64_t fine_sino_bytes(const tsgb_projector* p) {
 int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p) {
   if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
   if (p->fine) return fine_sino_bytes(p) + tsgb_fp_workspace_bytes(p->fine);
-  return p->fp_workspace_elems * int64_t(2 * sizeof(float));  // pairs of floats
+  // volume copies (pairs of floats); batched SIRT also keeps its sum volume and
+  // the backprojection's scratch volumes there
+  return std::max(p->fp_workspace_elems * int64_t(2 * sizeof(float)),
+                  tsgb::bp_volume_bytes(p->g) + tsgb::bp_scratch_bytes(p));
 }
 
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
@@ -175,9 +186,8 @@ int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
   if (bp_kind != TSGB_BP_MATCHED) return fail(TSGB_ERR_INVALID, "unknown bp_kind");
   if (p->fine) return fine_sino_bytes(p) + tsgb_bp_workspace_bytes(p->fine, bp_kind);
   // row-pair weighted sinogram (two floats per pixel, kRowPad padding rows),
-  // then the z-lane kernel's [y][x][z] scratch volume (either kernel may run)
-  return tsgb::bp_pairs_bytes(p->g) +
-         (p->n_separable_bp > 0 ? tsgb::bp_volume_bytes(p->g) : int64_t(0));
+  // then the z-lane kernel's [y][x][z] scratch volumes (either kernel may run)
+  return tsgb::bp_pairs_bytes(p->g) + tsgb::bp_scratch_bytes(p);
 }
 
 int tsgb_projector_shapes(const tsgb_projector* p, int64_t vol_shape[3], int64_t sino_shape[3]) {
@@ -294,7 +304,7 @@ int64_t tsgb_bp_batch_workspace_bytes(const tsgb_projector* p, int64_t n, int32_
   const int64_t one = tsgb_bp_workspace_bytes(p, bp_kind);
   if (one < 0 || n <= 1 || bp_kind != TSGB_BP_MATCHED || !tsgb::bp_batch_multi_eligible(p))
     return one;
-  const int64_t item = tsgb::bp_pairs_bytes(p->g), group = tsgb::batch_group(n, item);
+  const int64_t item = tsgb::bp_batch_item_bytes(p), group = tsgb::batch_group(n, item);
   return group > 1 ? std::max<int64_t>(one, group * item) : one;
 }
 
@@ -307,7 +317,7 @@ int tsgb_direct_bp_batch(tsgb_projector* p, float* vol, const float* sino, int64
   const size_t sino_elems = size_t(p->g.rows) * p->g.nangles * p->g.cols;
   // multi-job launches when the workspace holds a weighted sinogram per item
   // of a group (tsgb_bp_batch_workspace_bytes); else one item after another
-  const int64_t item = tsgb::bp_pairs_bytes(p->g);
+  const int64_t item = tsgb::bp_batch_item_bytes(p);
   const int64_t group = workspace ? std::min<int64_t>({n, int64_t(tsgb::kMaxMultiJobs),
                                                        workspace_bytes / item})
                                   : 0;

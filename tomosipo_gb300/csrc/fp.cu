@@ -583,12 +583,10 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   t.fp_patch_rows = 256 / kFpRows;
   t.fp_patch_cols = 32 / kFpCols;
   t.fp_group_pairs = 32;
-  // Matched backprojection: z-lane warps of 4 voxels x 16 z per lane x 8
-  // planes for volumes of 448 or more voxels along z (512^3 / 1024 angles:
-  // 124.8 ms against 144.5 ms for the voxel-pair kernel); below that a warp's
-  // 512 z would leave lanes idle, and the voxel-pair kernel is faster at 256^3
-  // (6.76 ms against 7.2 ms for the best z-lane shape).
-  t.bp_kernel = p->g.nz >= 448 ? 1 : 0;
+  // Matched backprojection: the z-lane kernel for every size (ms per call
+  // against the voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360
+  // 4.56 / 6.52, 8 x 128^3 / 128 2.0 / 2.6).
+  t.bp_kernel = 1;
   t.bp_shape = 2;
   return t;
 }

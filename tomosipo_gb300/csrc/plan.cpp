@@ -336,9 +336,8 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   }
   p->fp_workspace_elems = off;
   // At least a quarter of the separable work on rows finer than the voxels (a
-  // supersampled or fine detector; about 0.6 % of it for the cone scans of the
-  // benchmark): the matched backprojection takes the voxel-pair kernel's
-  // fine-row variant.
+  // supersampled or fine detector; about 0.6 % of it for the benchmark's cone
+  // scans): the voxel-pair kernel then runs as its fine-row variant.
   p->fine_rows = all_planes > 0.0 && fine_planes >= 0.25 * all_planes;
   // Detector region of a 16 x 8 x 16 voxel box at the anchor for each general
   // angle (its corners widened by one voxel along a and b, as the kernel

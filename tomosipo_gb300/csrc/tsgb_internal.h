@@ -72,6 +72,15 @@ struct alignas(16) ColumnEntry {
   float R, S, pad0, pad1;
 };
 
+// Per separable angle, in the order of the angle list: the coefficients of
+// q_a(kt, u) = (ca0 + kt ma0 + u (ca1 + kt ma1)) / (e0 + e1 u), for finding the
+// detector columns that cross a plane within a window, and the angle's id.
+struct alignas(16) SolveEntry {
+  float ca0, ca1, ma0, ma1;
+  float e0, e1;
+  int theta, pad;
+};
+
 struct Layout {
   int d, a, b;
   int64_t n_d, n_a, n_b;   // unpadded extents
@@ -122,8 +131,7 @@ struct tsgb_projector {
   int n_sep_ax = 0;             // of those, the first n_sep_ax have a = x (the rest a = y)
   // On at least a quarter of the (separable angle, column, plane) triples the
   // detector rows lie closer than one voxel apart (|q_b step per row| < 1):
-  // the matched backprojection then runs the voxel-pair kernel's fine-row
-  // variant.
+  // the voxel-pair kernel then runs as its fine-row variant.
   bool fine_rows = false;
   // The general backprojector's voxel boxes may be 16 wide along x: the
   // detector region a 16 x 8 x 16 box at the volume's centre projects to, for
@@ -135,6 +143,7 @@ struct tsgb_projector {
   tsgb::AngleParams* d_params = nullptr;
   tsgb::ColumnEntry* d_columns = nullptr;  // [nangles][cols]
   int* d_sep_angles = nullptr;             // angle ids for the separable BP kernel
+  tsgb::SolveEntry* d_solve = nullptr;     // the same angles' column-range coefficients
   std::vector<int> host_sep_angles;        // the same lists on the host (angle ranges)
   std::vector<int> host_gen_angles;
   int* d_gen_angles = nullptr;             // angle ids for the general BP kernel
@@ -272,25 +281,25 @@ int launch_fp_batch(const tsgb_projector* p, const float* vol, float* sino, int6
 // the multi-job launch of that pass over several jobs (bp.cu).
 long long bp_sep_blocks(const tsgb_projector* p, bool a_is_x, int* gx, int* gy);
 int launch_bp_sep_multi(const BpMulti& m, bool a_is_x, void* stream);
-// Whether a projector's batched matched backprojection can run on multi-job
-// launches (voxel-pair kernel, separable angles only, 32-bit offsets, no
-// supersampling or fine-row variant), and that batched backprojection:
-// `group` items per launch (<= kMaxMultiJobs), item k's weighted sinogram at
-// workspace + (k % group) * item_bytes (item_bytes >= bp_pairs_bytes) (bp.cu).
+// Whether a projector's batched matched backprojection can run on launches
+// shared by several items (separable angles only, no supersampling; voxel-pair
+// kernel: 32-bit offsets, no fine-row variant), the workspace of an item
+// (weighted sinogram; z-lane kernel: its scratch volumes too), and that batched
+// backprojection: `group` items per launch (<= kMaxMultiJobs), item k's part at
+// workspace + (k % group) * item_bytes (bp.cu).
 bool bp_batch_multi_eligible(const tsgb_projector* p);
+int64_t bp_batch_item_bytes(const tsgb_projector* p);
 int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* sino, int64_t n,
                             bool additive, char* workspace, int64_t item_bytes, int group,
                             void* stream);
 
 // The matched backprojector of det_v-along-z angles is the z-lane kernel
 // (bp_zlane.cu, column-major weighted sinogram) unless the tuning picks the
-// voxel-pair kernel (bp.cu, row-major), the volume's (y, x) plane is too
-// large for the z-lane grid (fewer than 2^32 voxel columns keep it below 2^31
-// blocks for every shape, which hold at least 8 columns per block), or the
-// detector rows are mostly finer than the voxels (fine_rows: the voxel-pair
-// kernel has a fast path for that).
+// voxel-pair kernel (bp.cu, row-major) or the volume's (y, x) plane is too
+// large for the z-lane grid (fewer than 2^32 voxel columns keep its two passes
+// below 2^31 blocks for every shape, which hold at least 16 columns per block).
 inline bool bp_uses_zlane(const tsgb_projector* p) {
-  return p->tuning.bp_kernel == 1 && !p->fine_rows &&
+  return p->tuning.bp_kernel == 1 &&
          int64_t(p->g.nx) * p->g.ny < (int64_t(1) << 32);
 }
 inline int zlane_shape(const tsgb_projector* p) { return p->tuning.bp_shape; }
@@ -299,17 +308,26 @@ inline int zlane_shape(const tsgb_projector* p) { return p->tuning.bp_shape; }
 // rounded up to 256; the z-lane kernel's [y][x][z] scratch volume follows it.
 int64_t bp_pairs_bytes(const DeviceGeometry& g);
 int64_t bp_volume_bytes(const DeviceGeometry& g);
+// The z-lane kernel's scratch volumes, one per pass that has angles (they follow
+// one another, bp_volume_bytes each).
+inline int bp_scratch_volumes(const tsgb_projector* p) {
+  return (p->n_sep_ax > 0) + (p->n_separable_bp > p->n_sep_ax);
+}
+int64_t bp_scratch_bytes(const tsgb_projector* p);
 
 // Column-major row-pair weighted sinogram (float pairs) of angles
 // angle_begin .. angle_end - 1 (bp_zlane.cu).
 int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz, int angle_begin,
                        int angle_end, void* stream);
 // Both z-lane passes over the separable angle lists (offsets into
-// p->d_sep_angles) into the [y][x][z] scratch volt, then vol (=, +=, SIRT)
-// from it (out_mode 0 / 1 / 2; C for SIRT). False if there are no such angles.
+// p->d_sep_angles) in one launch into the [y][x][z] scratch volumes at volt
+// (bp_scratch_bytes), then vol (=, +=, SIRT) from their sum (out_mode 0 / 1 / 2;
+// C for SIRT). items > 1: stacked items, item k's sinoz and volt k * item_bytes
+// further on and its vol k volumes (no SIRT). False if there are no such angles.
 bool launch_bp_zlane_separable(const tsgb_projector* p, int off_x, int n_ax, int off_y, int n_ay,
                                const float* sinoz, float* volt, float* vol, int out_mode,
-                               const float* C, void* stream);
+                               const float* C, void* stream, int items = 1,
+                               int64_t item_bytes = 0);
 
 // Kernel launchers (fp.cu, bp.cu). All return cudaGetLastError() as int.
 // With `sirt` the forward projection writes the SIRT residual instead of sino.
