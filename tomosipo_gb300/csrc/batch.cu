@@ -54,7 +54,7 @@ struct Unit {
 bool multi_eligible(const tsgb_projector* p) {
   const tsgb::DeviceGeometry& g = p->g;
   int gx = 0, gy = 0;
-  return (long long)g.nz * g.ny * g.nx <= kMultiMaxVoxels && !tsgb::bp_uses_zlane(p) &&
+  return (long long)g.nz * g.ny * g.nx <= kMultiMaxVoxels && !p->flat && !tsgb::bp_uses_zlane(p) &&
          p->n_general_bp == 0 && tsgb::fp_multi_eligible(p) &&
          tsgb::bp_sep_blocks(p, true, &gx, &gy) >= 0;
 }
@@ -178,7 +178,8 @@ namespace {
 
 // One SIRT iteration of job J on its own launches.
 cudaError_t iterate_job(const tsgb_sirt_job& J, cudaStream_t s) {
-  const tsgb::FpSirt sirt{J.sino, J.R, J.residual, tsgb::bp_uses_zlane(J.projector) ? 1 : 0};
+  const tsgb::FpSirt sirt{J.sino, J.R, J.residual, tsgb::bp_uses_zlane(J.projector) ? 1 : 0,
+                          tsgb::flat_bp(J.projector) ? 1 : 0};
   cudaError_t e = cudaError_t(tsgb::launch_fp(J.projector, J.vol, nullptr, false, J.fp_workspace, s, &sirt));
   // the forward workspace is free once the residual is written: it holds the
   // first backprojection pass's sum

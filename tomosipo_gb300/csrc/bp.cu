@@ -1260,6 +1260,9 @@ int launch_bp_matched(const tsgb_projector* p, float* vol, const float* sino, bo
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const DeviceGeometry& g = p->g;
   if (angle_end < 0) angle_end = g.nangles;
+  if (flat_bp(p))
+    return launch_flat_bp(p, vol, sino, false, additive ? 1 : 0, nullptr, workspace, stream,
+                          angle_begin, angle_end, 1, 0);
   // the angles of [angle_begin, angle_end) in each of the three angle lists
   int off_x, n_ax, off_y, n_ay, off_g, n_g;
   angle_sub_range(p->host_sep_angles, 0, p->n_sep_ax, angle_begin, angle_end, off_x, n_ax);
@@ -1311,6 +1314,8 @@ int launch_bp_sirt(const tsgb_projector* p, float* vol, const float* C, const fl
   const float2* pairs = reinterpret_cast<const float2*>(res);
   const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - p->n_sep_ax;
   const DeviceGeometry& g = p->g;
+  if (flat_bp(p))  // the residual is a plain sinogram of W y
+    return launch_flat_bp(p, vol, res, true, 2, C, scratch, stream, 0, g.nangles, 1, 0);
   if (p->n_general_bp > 0) {
     // Angles outside the separable backprojector (tilted detectors): the whole
     // backprojection goes into a sum volume as launch_bp_matched computes it
@@ -1383,11 +1388,12 @@ int launch_bp_sep_multi(const BpMulti& m, bool a_is_x, void* stream_) {
 bool bp_batch_multi_eligible(const tsgb_projector* p) {
   int gx = 0, gy = 0;
   if (p->fine || p->n_general_bp > 0 || p->n_separable_bp == 0) return false;
-  return bp_uses_zlane(p) || (!p->fine_rows && bp_sep_blocks(p, true, &gx, &gy) >= 0 &&
+  return flat_bp(p) || bp_uses_zlane(p) || (!p->fine_rows && bp_sep_blocks(p, true, &gx, &gy) >= 0 &&
                               bp_sep_blocks(p, false, &gx, &gy) >= 0);
 }
 
 int64_t bp_batch_item_bytes(const tsgb_projector* p) {
+  if (flat_bp(p)) return flat_bp_bytes(p);
   return bp_pairs_bytes(p->g) + (bp_uses_zlane(p) ? bp_scratch_bytes(p) : 0);
 }
 
@@ -1401,6 +1407,13 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
   const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - p->n_sep_ax;
   for (int64_t i0 = 0; i0 < n; i0 += group) {
     const int m = int(std::min<int64_t>(group, n - i0));
+    if (flat_bp(p)) {
+      const int rc = launch_flat_bp(p, vol + i0 * vol_elems, sino + i0 * sino_elems, false,
+                                    additive ? 1 : 0, nullptr, reinterpret_cast<float*>(workspace),
+                                    stream, 0, g.nangles, m, item_bytes);
+      if (rc != 0) return rc;
+      continue;
+    }
     if (bp_uses_zlane(p)) {
       for (int k = 0; k < m; ++k)
         launch_bp_weight_z(p, sino + (i0 + k) * sino_elems,

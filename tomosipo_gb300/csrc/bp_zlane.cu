@@ -98,62 +98,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Two fp32 values in one 64-bit register pair, and the packed operations on
-// them (one issue slot for both halves; each half rounds as the scalar does).
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2_rd(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-// Window accumulation: a column between voxels f0 and f0 + 1 of the window
-// (f0 in -1 .. kX - 1) adds wl V(z) to voxel f0 and wr V(z) to voxel f0 + 1,
-// with V(z) of the lane's voxels z0 + 32 j in pairs: profile(jj) holds those of
-// j = 2 jj and 2 jj + 1. The uniform branch on f0 sits outside the z loop, so
-// each profile pair goes straight into the two accumulators it feeds.
-template <int kX, int kPairs, int kM, typename F>
-__device__ __forceinline__ void window_apply(f32x2 (&acc)[kX][kPairs], const F& profile, f32x2 wl2,
-                                             f32x2 wr2) {
-#pragma unroll
-  for (int jj = 0; jj < kPairs; ++jj) {
-    const f32x2 V = profile(jj);
-    if constexpr (kM >= 0) acc[kM][jj] = fma2(wl2, V, acc[kM][jj]);
-    if constexpr (kM + 1 < kX) acc[kM + 1][jj] = fma2(wr2, V, acc[kM + 1][jj]);
-  }
-}
-
-template <int kX, int kPairs, int kM, typename F>
-__device__ __forceinline__ void window_dispatch(f32x2 (&acc)[kX][kPairs], int f0, const F& profile,
-                                                f32x2 wl2, f32x2 wr2) {
-  if constexpr (kM + 1 < kX) {
-    if (f0 == kM)
-      window_apply<kX, kPairs, kM>(acc, profile, wl2, wr2);
-    else
-      window_dispatch<kX, kPairs, kM + 1>(acc, f0, profile, wl2, wr2);
-  } else {
-    window_apply<kX, kPairs, kM>(acc, profile, wl2, wr2);  // f0 = kX - 1
-  }
-}
-
 // The columns of a list whose rows are at least a voxel apart (|Sl| >= 1).
 // Row pair v0 = floor((z - B) / Sl) and v0 + 1 (tent half-width 1/|Sl| <= 1
 // row). For voxel z: row v0's ray crosses the plane at t0 = v0 Sl + B - z from
@@ -214,7 +158,7 @@ __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
                    fmaf(__saturatef(1.0f - tb), S.yb[jj].x, __saturatef(e3.y + tb) * S.yb[jj].y));
     }
     const auto profile = [&](int jj) { return V[jj]; };
-    window_dispatch<kX, kPairs, -1>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
+    window_dispatch<kX, kPairs, -1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
                                     pack2(e2.z, e2.w));
   };
   if (n == 0) return;
@@ -287,39 +231,13 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
     for (int j = 0; j < kPairs; ++j) acc[m][j] = 0ull;
 
   for (int n0 = 0; n0 < n_angles; n0 += 32) {
-    // lane: detector columns of angle n0 + lane whose ray crosses this plane
-    // within (i0 - 1, i0 + kX): q_a(u) = (A0 + A1 u) / (e0 + e1 u); only the
-    // range uses this solve
-    int lo = 0, cnt = 0, theta = 0;
-    if (n0 + lane < n_angles) {
-      const float4 s0 = __ldg(solve + 2 * (n0 + lane));      // ca0, ca1, ma0, ma1
-      const float4 s1 = __ldg(solve + 2 * (n0 + lane) + 1);  // e0, e1, theta, -
-      const float A0 = fmaf(kt, s0.z, s0.x), A1 = fmaf(kt, s0.w, s0.y);
-      const float tl = i0t - 1.0f, th = i0t + float(kX);
-      const float u1 = __fdividef(fmaf(tl, s1.x, -A0), fmaf(-tl, s1.y, A1));
-      const float u2 = __fdividef(fmaf(th, s1.x, -A0), fmaf(-th, s1.y, A1));
-      lo = max(0, (int)floorf(clamp_coord(fminf(u1, u2))) + 1 + g.ou);
-      const int hi = min(g.cols - 1, (int)ceilf(clamp_coord(fmaxf(u1, u2))) - 1 + g.ou);
-      cnt = max(0, hi - lo + 1);
-      theta = __float_as_int(s1.z);
-    }
-    int end = cnt;  // running total of the ranges
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, end, o);
-      if (lane >= o) end += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, end, 31);
-    for (int t0 = 0; t0 < total; t0 += 32) {
-      // lane: list entry t0 + lane, of the angle m whose range holds it
+    const ColumnRanges cr = column_ranges(solve, n0 + lane, n_angles, kt, i0t - 1.0f,
+                                          i0t + float(kX), g);
+    for (int t0 = 0; t0 < cr.total; t0 += 32) {
       const int t = t0 + lane;
-      int m = 0;
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1)
-        if (__shfl_sync(0xffffffffu, end, m + o - 1) <= t) m += o;
-      const int iu = __shfl_sync(0xffffffffu, lo - (end - cnt), m) + t;
-      const int th = __shfl_sync(0xffffffffu, theta, m);
-      bool ok = t < total;
+      int iu, th;
+      column_of(cr, t, iu, th);
+      bool ok = t < cr.total;
       float4 e0, e1, e2, e3;
       int path = 0;
       if (ok) {
@@ -396,7 +314,7 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
             return fmaf(__saturatef(1.0f - at), y.x, __saturatef(c1s + at) * y.y);
           };
           const auto clamped = [&](int jj) { return pack2(row_pair(2 * jj), row_pair(2 * jj + 1)); };
-          window_dispatch<kX, kPairs, -1>(acc, f0, clamped, wl2, wr2);
+          window_dispatch<kX, kPairs, -1, kX>(acc, f0, clamped, wl2, wr2);
         } else if (rpath == 2) {
           // Rows finer than voxels: the tent (half-width 1/|Sl| <= 2 rows)
           // covers at most four rows, from the first above its lower end: two
@@ -420,7 +338,7 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
             return fmaf(__saturatef(1.0f - fabsf(fmaf(v0 + 3.0f, Sl, Bj))), y23.y, V);
           };
           const auto fine = [&](int jj) { return pack2(fine1(2 * jj), fine1(2 * jj + 1)); };
-          window_dispatch<kX, kPairs, -1>(acc, f0, fine, wl2, wr2);
+          window_dispatch<kX, kPairs, -1, kX>(acc, f0, fine, wl2, wr2);
         } else {
           // finer still: every row whose tent reaches the voxel
           const float2* col = reinterpret_cast<const float2*>(
@@ -436,7 +354,7 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
             return V;
           };
           const auto rows_loop = [&](int jj) { return pack2(rows1(2 * jj), rows1(2 * jj + 1)); };
-          window_dispatch<kX, kPairs, -1>(acc, f0, rows_loop, wl2, wr2);
+          window_dispatch<kX, kPairs, -1, kX>(acc, f0, rows_loop, wl2, wr2);
         }
       }
       __syncwarp();  // the list is rewritten
@@ -549,9 +467,12 @@ void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaS
   }
 }
 
+}  // namespace
+
 void launch_zlane_out(const DeviceGeometry& g, int mode, const float* volt0, const float* volt1,
                       long long item_volt, int zs, float* vol, const float* C, int items,
-                      cudaStream_t stream) {
+                      void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const dim3 grid(unsigned((g.nz + 31) / 32) * items, unsigned((g.nx + 31) / 32),
                   unsigned(std::min(g.ny, 65535)));
   const dim3 block(32, 8);
@@ -562,8 +483,6 @@ void launch_zlane_out(const DeviceGeometry& g, int mode, const float* volt0, con
   else
     bp_zlane_out_kernel<kOutSirt><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, vol, C, g);
 }
-
-}  // namespace
 
 int64_t bp_pairs_bytes(const DeviceGeometry& g) {
   return (int64_t(g.rows + 2 * kRowPad) * g.nangles * g.cols * 8 + 255) / 256 * 256;

@@ -170,10 +170,13 @@ int64_t fine_sino_bytes(const tsgb_projector* p) {
 int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p) {
   if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
   if (p->fine) return fine_sino_bytes(p) + tsgb_fp_workspace_bytes(p->fine);
+  // (batched SIRT backprojects in the forward workspace)
+  const int64_t sirt_bytes = tsgb::flat_bp(p) ? tsgb::flat_bp_bytes(p)
+                                              : tsgb::bp_volume_bytes(p->g) + tsgb::bp_scratch_bytes(p);
+  if (p->flat) return std::max(tsgb::flat_fp_bytes(p), sirt_bytes);
   // volume copies (pairs of floats); batched SIRT also keeps its sum volume and
   // the backprojection's scratch volumes there
-  return std::max(p->fp_workspace_elems * int64_t(2 * sizeof(float)),
-                  tsgb::bp_volume_bytes(p->g) + tsgb::bp_scratch_bytes(p));
+  return std::max(p->fp_workspace_elems * int64_t(2 * sizeof(float)), sirt_bytes);
 }
 
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
@@ -185,6 +188,7 @@ int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
                              : 0;
   if (bp_kind != TSGB_BP_MATCHED) return fail(TSGB_ERR_INVALID, "unknown bp_kind");
   if (p->fine) return fine_sino_bytes(p) + tsgb_bp_workspace_bytes(p->fine, bp_kind);
+  if (tsgb::flat_bp(p)) return tsgb::flat_bp_bytes(p);
   // row-pair weighted sinogram (two floats per pixel, kRowPad padding rows),
   // then the z-lane kernel's [y][x][z] scratch volumes (either kernel may run)
   return tsgb::bp_pairs_bytes(p->g) + tsgb::bp_scratch_bytes(p);
@@ -421,14 +425,20 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
   const int64_t extra = p->fine ? 1 : 0;
   const int64_t chunks = (f->g.nangles + 65534) / 65535;
   const int64_t chunk = tsgb::fp_angle_chunk(f->g);
+  // (parallel beams through flat.cu: copy, line sums, rows; resample, windows, out)
   const int64_t fp_launches =
-      int64_t(f->layouts.size()) + (f->g.nangles + chunk - 1) / chunk + extra;
-  // weight pass, one launch per separable pass, the z-lane kernel's transpose
-  // out of its scratch, the general kernel
-  const int64_t bp_launches = chunks + (f->n_sep_ax > 0 ? 1 : 0) +
-                              (f->n_separable_bp - f->n_sep_ax > 0 ? 1 : 0) +
-                              (tsgb::bp_uses_zlane(f) && f->n_separable_bp > 0 ? 1 : 0) +
-                              ((f->n_general_bp > 0 || f->n_separable_bp == 0) ? 1 : 0) + extra;
+      f->flat ? 3 + extra
+              : int64_t(f->layouts.size()) + (f->g.nangles + chunk - 1) / chunk + extra;
+  // weight pass, both z-lane passes and the transpose out of their scratch (or
+  // one launch per voxel-pair pass), the general kernel
+  const int64_t sep_launches =
+      f->n_separable_bp == 0        ? 0
+      : tsgb::bp_uses_zlane(f) ? 2
+                               : (f->n_sep_ax > 0) + (f->n_separable_bp > f->n_sep_ax);
+  const int64_t bp_launches =
+      (tsgb::flat_bp(f) ? 3
+               : chunks + sep_launches + ((f->n_general_bp > 0 || f->n_separable_bp == 0) ? 1 : 0)) +
+      extra;
   const int64_t vals[8] = {int64_t(f->layouts.size()),
                            f->n_separable_bp,
                            f->n_general_bp,

@@ -106,6 +106,159 @@ __device__ __forceinline__ bool finite_ray(const Ray& r) {
   return isfinite(r.Xa) && isfinite(r.ma) && isfinite(r.Xb) && isfinite(r.mb);
 }
 
+// Narrow [klo, khi] (plane coordinates) to planes where X + k m lies in (lo, hi).
+__device__ __forceinline__ void clip_planes(float X, float m, float lo, float hi, float& klo,
+                                            float& khi) {
+  if (m != 0.0f) {
+    const float inv = 1.0f / m;
+    const float t1 = (lo - X) * inv, t2 = (hi - X) * inv;
+    klo = fmaxf(klo, fminf(t1, t2));
+    khi = fminf(khi, fmaxf(t1, t2));
+  } else if (!(X > lo && X < hi)) {
+    klo = 1.0f;
+    khi = 0.0f;
+  }
+}
+
+// The detector columns whose rays cross a plane within an interval, for 32
+// angles at a time with one lane per angle: lane l's angle has columns lo ..
+// lo + cnt - 1, entries end - cnt .. end - 1 of the flattened list of all of them.
+struct ColumnRanges {
+  int lo, cnt, end, theta;
+  int total;  // entries of all lanes
+};
+
+// solve: the pass's SolveEntry table (two float4 per angle), n the lane's angle;
+// the ray of column u crosses plane kt at (A0 + A1 u) / (e0 + e1 u), solved for
+// tl and th. Every lane of the warp calls it.
+__device__ __forceinline__ ColumnRanges column_ranges(const float4* __restrict__ solve, int n,
+                                                      int n_angles, float kt, float tl, float th,
+                                                      const DeviceGeometry& g) {
+  const int lane = threadIdx.x & 31;
+  ColumnRanges r{0, 0, 0, 0, 0};
+  if (n < n_angles) {
+    const float4 s0 = __ldg(solve + 2 * n);      // ca0, ca1, ma0, ma1
+    const float4 s1 = __ldg(solve + 2 * n + 1);  // e0, e1, theta, -
+    const float A0 = fmaf(kt, s0.z, s0.x), A1 = fmaf(kt, s0.w, s0.y);
+    const float u1 = __fdividef(fmaf(tl, s1.x, -A0), fmaf(-tl, s1.y, A1));
+    const float u2 = __fdividef(fmaf(th, s1.x, -A0), fmaf(-th, s1.y, A1));
+    r.lo = max(0, (int)floorf(clamp_coord(fminf(u1, u2))) + 1 + g.ou);
+    const int hi = min(g.cols - 1, (int)ceilf(clamp_coord(fmaxf(u1, u2))) - 1 + g.ou);
+    r.cnt = max(0, hi - r.lo + 1);
+    r.theta = __float_as_int(s1.z);
+  }
+  r.end = r.cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, r.end, o);
+    if (lane >= o) r.end += v;
+  }
+  r.total = __shfl_sync(0xffffffffu, r.end, 31);
+  return r;
+}
+
+// Column iu of angle theta that list entry t stands for (t < total; else some
+// valid or invalid column). Every lane of the warp calls it.
+__device__ __forceinline__ void column_of(const ColumnRanges& r, int t, int& iu, int& theta) {
+  int m = 0;  // the lane whose range holds t: the number of ranges that end at or before it
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1)
+    if (__shfl_sync(0xffffffffu, r.end, m + o - 1) <= t) m += o;
+  iu = __shfl_sync(0xffffffffu, r.lo - (r.end - r.cnt), m) + t;
+  theta = __shfl_sync(0xffffffffu, r.theta, m);
+}
+
+// SIRT epilogue: residual W * (R * (y - A x)) of pixel idx, written where the
+// backprojector reads it. s.res is the row-pair sinogram of bp_weight_kernel
+// (kRowPad padding rows above and below the detector, zeroed once by the
+// caller and never written): the pixel is the first value of its own row's
+// pair and the second of the pair one row up. The plain recipe computes the
+// same products with separate operations (y - A(x), times R, then the
+// backprojector's W pass), rounded the same way.
+// With s.zlayout the pairs are column-major (bp_weight_z_kernel): pixel
+// (iv, theta, iu) is the first value of pair (theta, iu, iv + kRowPad) and the
+// second of the pair before it. Without pairs (s.plain, parallel beams through
+// flat.cu) the residual is a plain sinogram.
+__device__ __forceinline__ void sirt_residual(const FpSirt& s, const DeviceGeometry& g,
+                                              long long idx, float total, float W) {
+  const float r = __fmul_rn(__fsub_rn(__ldg(s.y + idx), total), __ldg(s.R + idx));
+  const float v = __fmul_rn(W, r);
+  if (s.plain) {
+    s.res[idx] = v;
+    return;
+  }
+  if (s.zlayout) {
+    const long long iu = idx % g.cols, rest = idx / g.cols;
+    const long long theta = rest % g.nangles, iv = rest / g.nangles;
+    float* e = s.res + 2 * ((theta * g.cols + iu) * (g.rows + 2 * kRowPad) + iv + kRowPad);
+    e[0] = v;
+    e[-1] = v;
+    return;
+  }
+  const long long rs = (long long)g.nangles * g.cols;
+  float* e = s.res + 2 * (idx + kRowPad * rs);
+  e[0] = v;
+  e[1 - 2 * rs] = v;
+}
+
+// Two fp32 values in one 64-bit register pair, and the packed operations on
+// them (one issue slot for both halves; each half rounds as the scalar does).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2_rd(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// Window accumulation: a column between voxels f0 and f0 + 1 of the window
+// (f0 in -1 .. kX - 1) adds wl V(z) to voxel f0 and wr V(z) to voxel f0 + 1,
+// with V(z) of the lane's voxels z0 + 32 j in pairs: profile(jj) holds those of
+// j = 2 jj and 2 jj + 1. The uniform branch on f0 sits outside the z loop, so
+// each profile pair goes straight into the two accumulators it feeds.
+template <int kX, int kPairs, int kM, typename F>
+__device__ __forceinline__ void window_apply(f32x2 (&acc)[kX][kPairs], const F& profile, f32x2 wl2,
+                                             f32x2 wr2) {
+#pragma unroll
+  for (int jj = 0; jj < kPairs; ++jj) {
+    const f32x2 V = profile(jj);
+    if constexpr (kM >= 0) acc[kM][jj] = fma2(wl2, V, acc[kM][jj]);
+    if constexpr (kM + 1 < kX) acc[kM + 1][jj] = fma2(wr2, V, acc[kM + 1][jj]);
+  }
+}
+
+// (kLo <= f0 < kHi: halves the candidates at each branch)
+template <int kX, int kPairs, int kLo, int kHi, typename F>
+__device__ __forceinline__ void window_dispatch(f32x2 (&acc)[kX][kPairs], int f0, const F& profile,
+                                                f32x2 wl2, f32x2 wr2) {
+  if constexpr (kHi - kLo == 1) {
+    window_apply<kX, kPairs, kLo>(acc, profile, wl2, wr2);
+  } else {
+    constexpr int kMid = kLo + (kHi - kLo) / 2;
+    if (f0 < kMid)
+      window_dispatch<kX, kPairs, kLo, kMid>(acc, f0, profile, wl2, wr2);
+    else
+      window_dispatch<kX, kPairs, kMid, kHi>(acc, f0, profile, wl2, wr2);
+  }
+}
+
 // ------------------------------------------------------------ FP tile order
 // Tile (row block, column block, angle pair) of linear block b under s. The
 // blocks of a group of pairs come first, inside a group the patches strip by

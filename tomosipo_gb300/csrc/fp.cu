@@ -115,20 +115,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Narrow [klo, khi] (plane coordinates) to planes where X + k m lies in (lo, hi).
-__device__ __forceinline__ void clip_planes(float X, float m, float lo, float hi, float& klo,
-                                            float& khi) {
-  if (m != 0.0f) {
-    const float inv = 1.0f / m;
-    const float t1 = (lo - X) * inv, t2 = (hi - X) * inv;
-    klo = fmaxf(klo, fminf(t1, t2));
-    khi = fminf(khi, fmaxf(t1, t2));
-  } else if (!(X > lo && X < hi)) {
-    klo = 1.0f;
-    khi = 0.0f;
-  }
-}
-
 // floor(q) as an int and q - floor(q), without the conversion unit
 // (kFloorMagic); identical to floorf. The sampled positions stay within a few
 // voxels of the volume, far inside its |q| < 2^22 range.
@@ -310,34 +296,6 @@ __device__ __forceinline__ void fp_ray_pair(const AngleParams& apa, const AngleP
   if (Wb) *Wb = ray_weight(apb, b.r);
 }
 
-// SIRT epilogue: residual W * (R * (y - A x)) of pixel idx, written where the
-// backprojector reads it. s.res is the row-pair sinogram of bp_weight_kernel
-// (kRowPad padding rows above and below the detector, zeroed once by the
-// caller and never written): the pixel is the first value of its own row's
-// pair and the second of the pair one row up. The plain recipe computes the
-// same products with separate operations (y - A(x), times R, then the
-// backprojector's W pass), rounded the same way.
-// With s.zlayout the pairs are column-major (bp_weight_z_kernel): pixel
-// (iv, theta, iu) is the first value of pair (theta, iu, iv + kRowPad) and the
-// second of the pair before it.
-__device__ __forceinline__ void sirt_residual(const FpSirt& s, const DeviceGeometry& g,
-                                              long long idx, float total, float W) {
-  const float r = __fmul_rn(__fsub_rn(__ldg(s.y + idx), total), __ldg(s.R + idx));
-  const float v = __fmul_rn(W, r);
-  if (s.zlayout) {
-    const long long iu = idx % g.cols, rest = idx / g.cols;
-    const long long theta = rest % g.nangles, iv = rest / g.nangles;
-    float* e = s.res + 2 * ((theta * g.cols + iu) * (g.rows + 2 * kRowPad) + iv + kRowPad);
-    e[0] = v;
-    e[-1] = v;
-    return;
-  }
-  const long long rs = (long long)g.nangles * g.cols;
-  float* e = s.res + 2 * (idx + kRowPad * rs);
-  e[0] = v;
-  e[1 - 2 * rs] = v;
-}
-
 // One thread per pixel and pair of adjacent angles; the linear block index
 // is mapped to a tile by the projector's schedule. The output offset and the
 // pair flag wait in shared memory during the walk (volatile, so they are not
@@ -505,6 +463,13 @@ int launch_fp_batch(const tsgb_projector* p, const float* vol, float* sino, int6
   const size_t sino_elems = size_t(g.rows) * g.nangles * g.cols;
   for (int64_t i0 = 0; i0 < n; i0 += group) {
     const int m = int(std::min<int64_t>(group, n - i0));
+    if (p->flat) {
+      const int rc = launch_flat_fp(p, vol + i0 * vol_elems, sino + i0 * sino_elems, additive,
+                                    reinterpret_cast<float*>(workspace), stream, nullptr, 0,
+                                    g.nangles, false, m, item_bytes);
+      if (rc != 0) return rc;
+      continue;
+    }
     FpMulti fm{};
     for (int k = 0; k < m; ++k) {
       float* ws = reinterpret_cast<float*>(workspace + k * item_bytes);
@@ -539,6 +504,9 @@ int launch_fp(const tsgb_projector* p, const float* vol, float* sino, bool addit
               int angle_end, bool copies_ready) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (angle_end < 0) angle_end = p->g.nangles;
+  if (p->flat)
+    return launch_flat_fp(p, vol, sino, additive, workspace, stream, sirt, angle_begin, angle_end,
+                          copies_ready, 1, 0);
   if (p->tuning.fp_pair_layout)
     launch_fp_elems(p, vol, sino, additive, reinterpret_cast<float2*>(workspace), stream, sirt,
                     angle_begin, angle_end, copies_ready);
@@ -583,10 +551,12 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   t.fp_patch_rows = 256 / kFpRows;
   t.fp_patch_cols = 32 / kFpCols;
   t.fp_group_pairs = 32;
-  // Matched backprojection: the z-lane kernel for every size (ms per call
-  // against the voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360
-  // 4.56 / 6.52, 8 x 128^3 / 128 2.0 / 2.6).
-  t.bp_kernel = 1;
+  // Matched backprojection: the z-lane kernel (ms per call against the
+  // voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360 4.56 / 6.52,
+  // 64^3 / 96 0.057 / 0.241), except for thin, wide volumes, whose few voxels
+  // along z leave its lanes idle (256^2 x 16 / 360 1.79 / 0.86, 256^2 x 40 1.95 /
+  // 1.57).
+  t.bp_kernel = thin_volume(p, 48) ? 0 : 1;
   t.bp_shape = 2;
   return t;
 }

@@ -174,6 +174,8 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   columns->assign(size_t(g.nangles) * g.cols, ColumnEntry{});
   sep_angles->clear();
   p->fine_rows = false;
+  // (the flat kernels' column lists hold 32-bit column indexes)
+  p->flat = !cone && int64_t(g.nangles) * g.cols < (int64_t(1) << 32);
   double fine_planes = 0.0, all_planes = 0.0;  // (separable angle, column, plane) triples
   gen_angles->clear();
   bil_fast->clear();
@@ -289,6 +291,8 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
       }
     }
     ap.bp_general = (separable && b == 0) ? 0 : 1;
+    // rays within one slice, all columns' rows at the same heights
+    if (ap.bp_general || mb[0] != 0.0 || cb[1] != 0.0) p->flat = false;
     if (ap.bp_general)
       gen_angles->push_back(t);
     else
