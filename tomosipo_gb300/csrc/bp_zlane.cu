@@ -30,7 +30,7 @@
 //    Several stacked items (batched backprojection) share the launch.
 //
 // Measured (GB300; the matched backprojection, weight pass and transpose
-// included): 512^3 / 1024 angles 99.7 ms, 256^3 / 360 4.56 ms. 256^3 in ncu:
+// included): 512^3 / 1024 angles 94.0 ms, 256^3 / 360 4.30 ms. 256^3 in ncu:
 // 20 thread instructions per voxel-angle, issue 64 %, 5.8 warps per scheduler
 // before the loads were issued a column ahead, waiting mostly for them.
 //
@@ -113,15 +113,15 @@ __global__ void __launch_bounds__(256)
 // (116 ms at 512^3 / 1024 angles, against 100 ms for two ranges of 8).
 template <int kX, int kRun, bool kClamp>
 __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
-                                              const float4 (&list)[32][4], int n, float zt,
+                                              const float4 (&list)[34][4], int n, float zt,
                                               float vmin, float vmax) {
   constexpr int kPairs = (kRun + 1) / 2;
   struct Stage {
     f32x2 t[kPairs];
     float2 ya[kPairs], yb[kPairs];
   } st[2];
-  const auto stage = [&](Stage& S, int k) {
-    const float4 e0 = list[k][0], e1 = list[k][1];
+  const auto stage = [&](Stage& S, const float4(&entry)[4]) {
+    const float4 e0 = entry[0], e1 = entry[1];
     const f32x2 Sl2 = pack2(e0.x, e0.y), Bl2 = pack2(e0.z, e0.w);
     const char* colb = reinterpret_cast<const char*>(
         size_t(__float_as_uint(e1.z)) | (size_t(__float_as_uint(e1.w)) << 32));
@@ -144,9 +144,9 @@ __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
       S.yb[jj] = __ldg(reinterpret_cast<const float2*>(colb + size_t(__float_as_uint(fb)) * sizeof(float2)));
     }
   };
-  const auto finish = [&](const Stage& S, int k) {
-    const float4 e2 = list[k][2];
-    const float2 e3 = *reinterpret_cast<const float2*>(&list[k][3]);
+  const auto finish = [&](const Stage& S, const float4(&entry)[4]) {
+    const float4 e2 = entry[2];
+    const float2 e3 = *reinterpret_cast<const float2*>(&entry[3]);
     f32x2 V[kPairs];
 #pragma unroll
     for (int jj = 0; jj < kPairs; ++jj) {
@@ -162,13 +162,14 @@ __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
                                     pack2(e2.z, e2.w));
   };
   if (n == 0) return;
-  stage(st[0], 0);
-  for (int k = 0; k < n; k += 2) {
-    stage(st[1], min(k + 1, n - 1));
-    finish(st[0], k);
+  const float4(*entry)[4] = list;
+  stage(st[0], entry[0]);
+  for (int k = 0; k < n; k += 2, entry += 2) {
+    stage(st[1], entry[1]);
+    finish(st[0], entry[0]);
     if (k + 1 < n) {
-      stage(st[0], min(k + 2, n - 1));
-      finish(st[1], k + 1);
+      stage(st[0], entry[2]);
+      finish(st[1], entry[1]);
     }
   }
 }
@@ -204,7 +205,7 @@ template <int kX, int kRun, int kPlanes, int kMinBlocks>
 __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
     bp_zlane_kernel(const __grid_constant__ ZlaneArgs A) {
   constexpr int kPairs = (kRun + 1) / 2;
-  __shared__ float4 s_list[kPlanes][32][4];
+  __shared__ float4 s_list[kPlanes][34][4];
   const DeviceGeometry& g = A.g;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int pass = blockIdx.x < A.blocks0 ? 0 : 1;
@@ -281,6 +282,10 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
         s_list[w][slot][1] = e1;
         s_list[w][slot][2] = e2;
         s_list[w][slot][3] = e3;
+        if ((mask >> lane) == 1u) {  // the last: loads a column ahead find it again
+          s_list[w][slot + 1][0] = s_list[w][slot + 2][0] = e0;
+          s_list[w][slot + 1][1] = s_list[w][slot + 2][1] = e1;
+        }
       }
       __syncwarp();
       const int columns_in = __popc(mask);
@@ -442,11 +447,12 @@ void launch_zlane_shape(ZlaneArgs& A, int items, cudaStream_t stream) {
 // most 8, ranges of near-equal length along z). Wider windows share a column's
 // profile between more voxels ((kX + 1) / kX columns per voxel), as long as the
 // accumulators and the two load stages fit the registers. Measured (GB300):
-// run 8, 512^3 / 1024 angles: 5 x 8 warps 99.7 ms, 3 x 8 101.0, 4 x 8 102.2,
-// 4 x 16 100.5, 6 x 8 108.3; run 6, helical 170 x 190 x 181 / 257: 6 x 4 warps
+// run 8, 512^3 / 1024 angles: 5 x 8 warps 94.0 ms, 3 x 8 101.0, 4 x 8 95.5,
+// 6 x 8 over 100; run 6, helical 170 x 190 x 181 / 257: 6 x 4 warps
 // 2.76 ms (forward projection included), 5 x 4 2.80, 4 x 4 2.88; run 3, SIRT at
 // 96^3: 8 x 4 warps 1.61 ms, 4 x 4 1.66, 6 x 4 1.71; run 4, 8 x 128^3: all
-// within 2 %. The tuning's bp_shape 3 and 4 force other windows for run 8, 5 and
+// within 2 %,
+// 128^3 / 200: 6 x 4 warps 0.407, 8 x 4 0.431. The tuning's bp_shape 3 and 4 force other windows for run 8, 5 and
 // 6 cap the run at 4 and 2; any other value takes this rule.
 void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaStream_t stream) {
   const int shape = zlane_shape(p);
@@ -456,7 +462,7 @@ void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaS
     case 1: return launch_zlane_shape<4, 1, 8, 4>(A, items, stream);
     case 2: return launch_zlane_shape<4, 2, 8, 4>(A, items, stream);
     case 3: return launch_zlane_shape<8, 3, 4, 4>(A, items, stream);
-    case 4: return launch_zlane_shape<8, 4, 4, 5>(A, items, stream);
+    case 4: return launch_zlane_shape<6, 4, 4, 5>(A, items, stream);
     case 5: return launch_zlane_shape<6, 5, 4, 4>(A, items, stream);
     case 6: return launch_zlane_shape<6, 6, 4, 4>(A, items, stream);
     case 7: return launch_zlane_shape<5, 7, 8, 2>(A, items, stream);
