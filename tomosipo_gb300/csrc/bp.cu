@@ -28,9 +28,9 @@
 // Bilinear backprojection: voxel-driven, bilinear interpolation of the
 // detector at the projected voxel centre, weighted so that it approximates
 // the transpose (voxel volume / pixel area / ray obliquity, times the cone
-// magnification squared). For z-flat geometries a quad copy of the sinogram
-// gives each voxel its four taps in one load; the same kernel with FDK's
-// weights is the backprojection of the FDK reconstruction.
+// magnification squared). Angles whose projection keeps u and the depth along z
+// take bp_bilinear.cu (thin, wide volumes bp_bilinear_z_kernel here), the others
+// bp_bilinear_kernel.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -971,6 +971,9 @@ __device__ __forceinline__ float detector_or_zero(const float* __restrict__ sino
   return __ldg(sino + ((size_t)iv * g.nangles + t) * g.cols + iu);
 }
 
+// Thin, wide volumes (thin_volume(p, 32)): the lanes of bp_bilinear.cu's kernel
+// would idle, so a thread owns a voxel column of 16 voxels along z instead.
+//
 // Quad copy of the sinogram for bp_bilinear_z_kernel: element (iv, t, iu) for
 // iv in -kRowPad .. rows + kRowPad - 1 and iu in -kColPad .. cols + kColPad - 1
 // holds the four taps of a bilinear read, (y[iv][iu], y[iv][iu+1],
@@ -1039,12 +1042,6 @@ __device__ __forceinline__ float bilinear_z_term(const float4* __restrict__ colq
   }
   return fmaf(c, val, acc);
 }
-
-// kWeight: kBilParallel, kBilCone (the bilinear backprojector's weights) or
-// kBilFdk: FDK's backprojection weight angle_w[theta] / w^2, where w is the
-// voxel's depth along the detector normal relative to the volume anchor's
-// (the projective denominator pw . [P, 1]).
-enum BilWeight { kBilParallel = 0, kBilCone = 1, kBilFdk = 2 };
 
 // A block of 128 threads is kTX voxel columns along x times 128 / kTX along y,
 // x-fastest; each thread owns kRun voxels along z.
@@ -1479,6 +1476,32 @@ void launch_bil_z(const tsgb_projector* p, const float4* quads, float* vol, bool
   launch_bil_z_tile<kWeight, 8>(p, quads, vol, additive, angle_w, stream);
 }
 
+// Quad copy and the z-flat kernel of thin, wide volumes.
+void launch_bil_thin(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
+                     bool additive, float* workspace, cudaStream_t stream) {
+  const DeviceGeometry& g = p->g;
+  const long long total = (long long)(g.rows + 2 * kRowPad) * g.nangles * (g.cols + 2 * kColPad);
+  const long long blocks = (total + 255) / 256;
+  float4* quads = reinterpret_cast<float4*>(workspace);
+  bp_bilinear_prep_kernel<<<int(blocks < 152LL * 64 ? blocks : 152LL * 64), 256, 0, stream>>>(
+      sino, quads, g);
+  if (angle_w)
+    launch_bil_z<kBilFdk>(p, quads, vol, additive, angle_w, stream);
+  else if (g.kind == TSGB_CONE)
+    launch_bil_z<kBilCone>(p, quads, vol, additive, nullptr, stream);
+  else
+    launch_bil_z<kBilParallel>(p, quads, vol, additive, nullptr, stream);
+}
+
+// The z-flat angles of the bilinear backprojection (angle_w: FDK's weights).
+void launch_bil_fast(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
+                     bool additive, float* workspace, cudaStream_t stream) {
+  if (bilinear_thin(p))
+    launch_bil_thin(p, vol, sino, angle_w, additive, workspace, stream);
+  else
+    launch_bilinear_zlane(p, vol, sino, angle_w, additive, workspace, stream);
+}
+
 }  // namespace
 
 int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, bool additive,
@@ -1488,15 +1511,7 @@ int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, b
   const dim3 block(kBpX, kBpY);
   bool written = false;
   if (p->n_bil_fast > 0) {
-    const long long total = (long long)(g.rows + 2 * kRowPad) * g.nangles * (g.cols + 2 * kColPad);
-    const long long blocks = (total + 255) / 256;
-    float4* quads = reinterpret_cast<float4*>(workspace);
-    bp_bilinear_prep_kernel<<<int(blocks < 152LL * 64 ? blocks : 152LL * 64), 256, 0, stream>>>(
-        sino, quads, g);
-    if (g.kind == TSGB_CONE)
-      launch_bil_z<kBilCone>(p, quads, vol, additive, nullptr, stream);
-    else
-      launch_bil_z<kBilParallel>(p, quads, vol, additive, nullptr, stream);
+    launch_bil_fast(p, vol, sino, nullptr, additive, workspace, stream);
     written = true;
   }
   if (p->n_bil_slow > 0 || !written) {
@@ -1514,12 +1529,7 @@ int launch_bp_fdk(const tsgb_projector* p, float* vol, const float* sino, const 
   const DeviceGeometry& g = p->g;
   bool written = false;
   if (p->n_bil_fast > 0) {
-    const long long total = (long long)(g.rows + 2 * kRowPad) * g.nangles * (g.cols + 2 * kColPad);
-    const long long blocks = (total + 255) / 256;
-    float4* quads = reinterpret_cast<float4*>(workspace);
-    bp_bilinear_prep_kernel<<<int(blocks < 152LL * 64 ? blocks : 152LL * 64), 256, 0, stream>>>(
-        sino, quads, g);
-    launch_bil_z<kBilFdk>(p, quads, vol, additive, angle_w, stream);
+    launch_bil_fast(p, vol, sino, angle_w, additive, workspace, stream);
     written = true;
   }
   if (p->n_bil_slow > 0 || !written) {

@@ -31,8 +31,10 @@ void free_device(tsgb_projector* p) {
   if (p->d_solve) cudaFree(p->d_solve);
   if (p->d_gen_angles) cudaFree(p->d_gen_angles);
   if (p->d_bil_fast) cudaFree(p->d_bil_fast);
+  if (p->d_bil_table) cudaFree(p->d_bil_table);
   if (p->d_bil_slow) cudaFree(p->d_bil_slow);
   p->d_bil_fast = nullptr;
+  p->d_bil_table = nullptr;
   p->d_bil_slow = nullptr;
   p->d_params = nullptr;
   p->d_columns = nullptr;
@@ -132,6 +134,19 @@ int tsgb_projector_create(const tsgb_volume_desc* vol, const tsgb_projection_des
   if (e == cudaSuccess) e = upload(&p->d_solve, solve);
   if (e == cudaSuccess) e = upload(&p->d_gen_angles, gen);
   if (e == cudaSuccess) e = upload(&p->d_bil_fast, bfast);
+  std::vector<tsgb::BilinearEntry> bil;
+  for (int row = 0; row < 4; ++row)
+    for (int t : bfast) {
+      const tsgb::AngleParams& ap = p->host_params[t];
+      float id;
+      std::memcpy(&id, &t, sizeof(id));
+      const tsgb::BilinearEntry rows[4] = {{{ap.pu[1], ap.pu[2], ap.pu[3], ap.pv[0]}},
+                                           {{ap.pv[1], ap.pv[2], ap.pv[3], ap.pw[1]}},
+                                           {{ap.pw[2], ap.pw[3], ap.bil_scale, id}},
+                                           {{ap.src[0], ap.src[1], ap.src[2], 0.0f}}};
+      bil.push_back(rows[row]);
+    }
+  if (e == cudaSuccess) e = upload(&p->d_bil_table, bil);
   if (e == cudaSuccess) e = upload(&p->d_bil_slow, bslow);
   if (e != cudaSuccess) {
     free_device(p);
@@ -182,10 +197,7 @@ int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p) {
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
   if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
   if (bp_kind == TSGB_BP_BILINEAR)
-    // quad copy of the padded sinogram: four floats per element
-    return p->n_bil_fast > 0 ? int64_t(p->g.rows + 2 * tsgb::kRowPad) * p->g.nangles *
-                                   (p->g.cols + 2 * tsgb::kColPad) * int64_t(4 * sizeof(float))
-                             : 0;
+    return p->n_bil_fast > 0 ? tsgb::bilinear_bytes(p) : 0;
   if (bp_kind != TSGB_BP_MATCHED) return fail(TSGB_ERR_INVALID, "unknown bp_kind");
   if (p->fine) return fine_sino_bytes(p) + tsgb_bp_workspace_bytes(p->fine, bp_kind);
   if (tsgb::flat_bp(p)) return tsgb::flat_bp_bytes(p);
@@ -444,7 +456,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
                            f->n_general_bp,
                            fp_launches,
                            bp_launches,
-                           (p->n_bil_fast > 0 ? 2 : 0) +
+                           (p->n_bil_fast > 0 ? (tsgb::bilinear_thin(p) ? 2 : 3) : 0) +
                                ((p->n_bil_slow > 0 || p->n_bil_fast == 0) ? 1 : 0),
                            tsgb_fp_workspace_bytes(p),
                            tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED)};

@@ -217,6 +217,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -257,6 +262,21 @@ __device__ __forceinline__ void window_dispatch(f32x2 (&acc)[kX][kPairs], int f0
     else
       window_dispatch<kX, kPairs, kMid, kHi>(acc, f0, profile, wl2, wr2);
   }
+}
+
+// Tile (i, j) of linear block b of an ni x nj grid of tiles, run in patches of
+// pi x pj tiles (i fastest inside a patch; only the last patches are smaller).
+__device__ __forceinline__ void patch_tile(unsigned b, int ni, int nj, int pi, int pj, int& i,
+                                           int& j) {
+  const unsigned strip = unsigned(ni) * unsigned(pj);  // a full strip of patches
+  const int s = int(b / strip);
+  b -= unsigned(s) * strip;
+  const int hj = min(pj, nj - s * pj);
+  const int q = int(b / unsigned(pi * hj));
+  b -= unsigned(q) * unsigned(pi * hj);
+  const int wi = min(pi, ni - q * pi);
+  i = q * pi + int(b % unsigned(wi));
+  j = s * pj + int(b / unsigned(wi));
 }
 
 // ------------------------------------------------------------ FP tile order

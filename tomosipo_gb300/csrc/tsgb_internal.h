@@ -31,6 +31,11 @@ namespace tsgb {
 constexpr int kPad = 2;        // zero padding of the forward-projection volume copies
 constexpr int kRowPad = 2;     // zero detector rows above and below the weighted sinogram
 constexpr int kColPad = 2;     // zero detector columns left and right (bilinear BP copy)
+// Weights of the bilinear kernels: the bilinear backprojector's (parallel, cone) or
+// FDK's backprojection weight angle_w[theta] / w^2, where w is the voxel's depth
+// along the detector normal relative to the volume anchor's (the projective
+// denominator pw . [P, 1]).
+enum BilWeight { kBilParallel = 0, kBilCone = 1, kBilFdk = 2 };
 constexpr int kMaxLayouts = 6; // axis permutations (d, a, b)
 
 // Per-angle parameters, read uniformly by all threads of a block.
@@ -79,6 +84,14 @@ struct alignas(16) SolveEntry {
   float ca0, ca1, ma0, ma1;
   float e0, e1;
   int theta, pad;
+};
+
+// Per z-flat angle of the bilinear backprojector, structure of arrays (row k of
+// n entries): projection coefficients of a voxel column (y, x) and its weights:
+//   row 0: pu[1], pu[2], pu[3], pv[0]   row 1: pv[1], pv[2], pv[3], pw[1]
+//   row 2: pw[2], pw[3], bil_scale, theta   row 3: src (z, y, x), -
+struct BilinearEntry {
+  float v[4];
 };
 
 struct Layout {
@@ -150,7 +163,8 @@ struct tsgb_projector {
   std::vector<int> host_sep_angles;        // the same lists on the host (angle ranges)
   std::vector<int> host_gen_angles;
   int* d_gen_angles = nullptr;             // angle ids for the general BP kernel
-  int* d_bil_fast = nullptr;               // angle ids, bilinear z-flat kernel
+  int* d_bil_fast = nullptr;               // angle ids, bilinear z-flat kernels
+  tsgb::BilinearEntry* d_bil_table = nullptr;  // 4 rows of n_bil_fast entries
   int* d_bil_slow = nullptr;               // angle ids, bilinear general kernel
 };
 
@@ -340,16 +354,28 @@ void launch_zlane_out(const DeviceGeometry& g, int out_mode, const float* volt0,
                       const float* volt1, long long item_volt, int zs, float* vol, const float* C,
                       int items, void* stream);
 
+// Volumes of at most nz voxels along z and 2^15 or more in the slice: they leave
+// most of the z-lane kernels' lanes idle, and fill the GPU without them.
+inline bool thin_volume(const tsgb_projector* p, int nz) {
+  return p->g.nz <= nz && int64_t(p->g.nx) * p->g.ny >= (int64_t(1) << 15);
+}
+// Bilinear backprojection of the z-flat angles (bp_bilinear.cu): vol (= or +=),
+// with FDK's weights angle_w (by angle id) or, if null, the bilinear ones; its
+// workspace (padded row pairs, scratch volume).
+int64_t bilinear_bytes(const tsgb_projector* p);
+// Thin, wide volumes keep one thread per voxel column (bp.cu) and a quad copy of
+// the sinogram (256^2 slice, 360 cone angles: 16 voxels along z 0.79 ms against
+// 1.09, 32 0.92 / 1.06, 48 1.84 / 1.69).
+inline bool bilinear_thin(const tsgb_projector* p) { return thin_volume(p, 32); }
+int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino,
+                          const float* angle_w, bool additive, float* workspace, void* stream);
+
 // Parallel beams through flat.cu (p->flat). Workspace bytes of one item's
 // forward projection (volume copy, per-slice line sums) and backprojection
 // (sinogram resampled to the slices, scratch volumes); the projections of
 // `items` stacked items with their workspaces item_bytes apart.
-// Thin, wide volumes leave most z lanes idle: up to 16 voxels along z, 2^15 or
-// more in the slice, the backprojection is the voxel-pair kernel's (256^2 slice,
-// 360 angles: 16 voxels 0.85 ms against 0.91, 40 voxels 1.46 against 0.97).
-inline bool thin_volume(const tsgb_projector* p, int nz) {
-  return p->g.nz <= nz && int64_t(p->g.nx) * p->g.ny >= (int64_t(1) << 15);
-}
+// (up to 16 voxels along z a thin, wide volume keeps the voxel-pair kernel: 256^2
+// slice, 360 angles, 16 voxels 0.85 ms against 0.91, 40 voxels 1.46 against 0.97)
 inline bool flat_bp(const tsgb_projector* p) { return p->flat && !thin_volume(p, 16); }
 int64_t flat_fp_bytes(const tsgb_projector* p);
 int64_t flat_bp_bytes(const tsgb_projector* p);
