@@ -385,26 +385,71 @@ struct PairView {
   }
 };
 
-// The ray of pixel (iu, iv) at one angle, as the forward projector computes it.
-__device__ __forceinline__ Ray pixel_ray(const AngleParams& ap,
-                                         const ColumnEntry* __restrict__ columns,
-                                         const DeviceGeometry& g, int theta, int iu, int iv) {
-  const float vt = float(iv - g.ov);
-  return ap.separable ? ray_column(columns[(size_t)theta * g.cols + iu], vt)
-                      : ray_general(ap, float(iu - g.ou), vt);
+// Where the rays pass a voxel (kt, it, jt): the ray of pixel (u, v) (anchored)
+// crosses the voxel's plane at distances (ta, tb) from it along a and b, and
+//   den(u, v) (ta, tb) = be + al u + ga v,  den = e0 + e1 u + e2 v
+// (the forward projector's q_a = (ca + kt ma) . [1, u, v] / den, minus it). Halves
+// of the packed pairs: a, b.
+struct VoxelForms {
+  f32x2 al, be, ga;
+};
+
+// The forms of the voxels x8 + m of a run along x (x8 a multiple of 8 voxel
+// indexes, m < 8), at (kt, it, jt) for m = 0: linear in m. Every kernel takes
+// them from the same run, so that they round alike.
+struct RunForms {
+  VoxelForms first, step;
+};
+
+__device__ __forceinline__ RunForms run_forms(const AngleParams& ap, float kt, float it, float jt) {
+  const f32x2 k = pack2(kt, kt), ij = pack2(-it, -jt);
+  // x is one of the axes d, a, b: kt, it or jt steps by 1
+  const float dk = ap.d == 2 ? 1.0f : 0.0f, di = ap.a == 2 ? -1.0f : 0.0f;
+  const float dj = ap.b == 2 ? -1.0f : 0.0f;
+  f32x2 first[3], step[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    first[i] = fma2(ij, pack2(ap.e[i], ap.e[i]),
+                    fma2(k, pack2(ap.ma[i], ap.mb[i]), pack2(ap.ca[i], ap.cb[i])));
+    step[i] = pack2(fmaf(di, ap.e[i], dk * ap.ma[i]), fmaf(dj, ap.e[i], dk * ap.mb[i]));
+  }
+  return {{first[1], first[0], first[2]}, {step[1], step[0], step[2]}};
+}
+
+__device__ __forceinline__ VoxelForms voxel_forms(const RunForms& r, int m) {
+  const f32x2 m2 = pack2(float(m), float(m));
+  return {fma2(m2, r.step.al, r.first.al), fma2(m2, r.step.be, r.first.be),
+          fma2(m2, r.step.ga, r.first.ga)};
+}
+
+// 1 / den of pixel (u, v).
+__device__ __forceinline__ float pixel_rden(const AngleParams& ap, float u, float v) {
+  return 1.0f / fmaf(ap.e[2], v, fmaf(ap.e[1], u, ap.e[0]));
+}
+
+// The form at column u (both halves).
+__device__ __forceinline__ f32x2 form_column(const VoxelForms& f, float u) {
+  return fma2(pack2(u, u), f.al, f.be);
+}
+
+// Weight of a pixel (tent(ta) tent(tb)) at row v of that column. A tent is one
+// saturating add (1 - |t| <= 1; NaN saturates to 0); a weight of 0 adds nothing.
+__device__ __forceinline__ float pixel_weight(const VoxelForms& f, f32x2 column, float v,
+                                              float rden) {
+  float ta, tb;
+  unpack2(mul2(fma2(pack2(v, v), f.ga, column), pack2(rden, rden)), ta, tb);
+  return __saturatef(1.0f - fabsf(ta)) * __saturatef(1.0f - fabsf(tb));
 }
 
 // Matched-backprojection terms of one voxel (anchored zt, yt, xt) for one
 // angle of any geometry, added to acc: project the four corners
 // (kt, it -+ 1, jt -+ 1) of the voxel's tent footprint on its plane of the
-// dominant axis, and test every pixel of their bounding box with the forward
-// projector's ray formula. Rows outer, columns inner.
+// dominant axis, and weight every pixel of their bounding box. Rows outer,
+// columns inner.
 __device__ __forceinline__ float general_voxel_terms(const AngleParams& ap,
-                                                     const ColumnEntry* __restrict__ columns,
                                                      const float2* __restrict__ base,
                                                      const PairView& pv, const DeviceGeometry& g,
-                                                     int theta, float zt, float yt, float xt,
-                                                     float acc) {
+                                                     float zt, float yt, float xt, float acc) {
   const float kt = coord(ap.d, zt, yt, xt);
   const float it = coord(ap.a, zt, yt, xt);
   const float jt = coord(ap.b, zt, yt, xt);
@@ -431,12 +476,16 @@ __device__ __forceinline__ float general_voxel_terms(const AngleParams& ap,
   const int iu_hi = min(g.cols - 1, (int)ceilf(clamp_coord(umax)) - 1 + g.ou);
   const int iv_lo = max(0, (int)floorf(clamp_coord(vmin)) + 1 + g.ov);
   const int iv_hi = min(g.rows - 1, (int)ceilf(clamp_coord(vmax)) - 1 + g.ov);
+  const int m = (int(xt) + g.ox) & 7;
+  const float xm = xt - float(m);
+  const RunForms run = run_forms(ap, coord(ap.d, zt, yt, xm), coord(ap.a, zt, yt, xm),
+                                 coord(ap.b, zt, yt, xm));
+  const VoxelForms f = voxel_forms(run, m);
   for (int iv = iv_lo; iv <= iv_hi; ++iv) {
+    const float v = float(iv - g.ov);
     for (int iu = iu_lo; iu <= iu_hi; ++iu) {
-      const Ray r = pixel_ray(ap, columns, g, theta, iu, iv);
-      const float wa = tent(fmaf(kt, r.ma, r.Xa) - it);
-      const float wb = tent(fmaf(kt, r.mb, r.Xb) - jt);
-      const float w = wa * wb;
+      const float u = float(iu - g.ou);
+      const float w = pixel_weight(f, form_column(f, u), v, pixel_rden(ap, u, v));
       if (w > 0.0f) acc = fmaf(w, __ldg(base + iv * pv.s_row + iu * pv.s_col).x, acc);
     }
   }
@@ -445,8 +494,7 @@ __device__ __forceinline__ float general_voxel_terms(const AngleParams& ap,
 
 // One thread per voxel; any geometry (the tuning's bp_general = 1).
 __global__ void __launch_bounds__(128)
-    bp_general_kernel(const AngleParams* __restrict__ params,
-                      const ColumnEntry* __restrict__ columns, const int* __restrict__ angles,
+    bp_general_kernel(const AngleParams* __restrict__ params, const int* __restrict__ angles,
                       int n_angles, const float2* __restrict__ sinow, float* __restrict__ vol,
                       DeviceGeometry g, int additive, int zlayout) {
   const int x = blockIdx.x * 32 + threadIdx.x;
@@ -458,8 +506,8 @@ __global__ void __launch_bounds__(128)
   float acc = 0.0f;
   for (int n = 0; n < n_angles; ++n) {
     const int theta = __ldg(angles + n);
-    acc = general_voxel_terms(params[theta], columns, pv.base(sinow, g, theta, zlayout), pv, g,
-                              theta, zt, yt, xt, acc);
+    acc = general_voxel_terms(params[theta], pv.base(sinow, g, theta, zlayout), pv, g, zt, yt, xt,
+                              acc);
   }
   float* out = vol + ((size_t)z * g.ny + y) * g.nx + x;
   if (additive)
@@ -615,57 +663,57 @@ __device__ __forceinline__ void gen_region(const AngleParams& ap, const DeviceGe
 template <int kGenRunX, int kZl, int kWu, int kWv>
 __device__ __forceinline__ void gen_window_run(const AngleParams& ap, const GenRegion& R,
                                                const DeviceGeometry& g,
-                                               const float4* __restrict__ s_ray,
-                                               const float* __restrict__ s_val, float zt,
+                                               const float2* __restrict__ s_pix, float zt,
                                                float yt, float xt0, int x0,
                                                float (&acc)[kGenRunX]) {
-  const int d = ap.d, a = ap.a;
-  const float kt0 = d == 0 ? zt : (d == 1 ? yt : xt0);
-  const float it0 = a == 0 ? zt : (a == 1 ? yt : xt0);
-  const float jt0 = (d != 0 && a != 0) ? zt : ((d != 1 && a != 1) ? yt : xt0);
-  const float dk = d == 2 ? 1.0f : 0.0f, di = a == 2 ? 1.0f : 0.0f;
-  const float dj = 1.0f - dk - di;
+  // (a run of 4 starts at 0 or 4 of the forms' run of 8)
+  const int m0 = kGenRunX == 8 ? 0 : x0 & 7;
+  const float x8 = xt0 - float(m0);
+  const RunForms run = run_forms(ap, coord(ap.d, zt, yt, x8), coord(ap.a, zt, yt, x8),
+                                 coord(ap.b, zt, yt, x8));
   const float nu0 = fmaf(ap.pu[0], zt, fmaf(ap.pu[1], yt, fmaf(ap.pu[2], xt0, ap.pu[3])));
   const float nv0 = fmaf(ap.pv[0], zt, fmaf(ap.pv[1], yt, fmaf(ap.pv[2], xt0, ap.pv[3])));
   const float nw0 = fmaf(ap.pw[0], zt, fmaf(ap.pw[1], yt, fmaf(ap.pw[2], xt0, ap.pw[3])));
   const float pu2 = ap.pu[2], pv2 = ap.pv[2], pw2 = ap.pw[2];
-  // first pixel above u* - hu, as an index: floor(u* - hu) + 1 + anchor;
-  // the window is then moved inside the region if it sticks out (the
-  // footprint itself lies inside the region)
-  const float ou = float(1 + g.ou) - R.hu, ov = float(1 + g.ov) - R.hv;
-  const int u_first = R.u0 + R.nu - R.wu, v_first = R.v0 + R.nv - R.wv;
+  // first pixel above u* - hu: floor(u* - hu) + 1 (anchored coordinates; clamping to
+  // integers clamps the floor, NaN -> the first), moved inside the region if the
+  // window sticks out (the footprint itself lies inside the region)
+  const float ou = 1.0f - R.hu, ov = 1.0f - R.hv;
+  const float u_lo = float(R.u0 - g.ou), u_hi = u_lo + float(R.nu - R.wu);
+  const float v_lo = float(R.v0 - g.ov), v_hi = v_lo + float(R.nv - R.wv);
   const int su = kZl ? R.su : 1, sv = kZl ? 1 : R.sv;
+  // stage index of the anchored pixel (0, 0), from floors' kFloorMagic bits
+  const int origin = -(R.u0 - g.ou + int(kFloorBits)) * su - (R.v0 - g.ov + int(kFloorBits)) * sv;
 #pragma unroll
   for (int m = 0; m < kGenRunX; ++m) {
     if (x0 + m >= g.nx) break;
     const float fm = float(m);
-    const float kt = fmaf(fm, dk, kt0), it = fmaf(fm, di, it0), jt = fmaf(fm, dj, jt0);
     const float rw = __fdividef(1.0f, fmaf(fm, pw2, nw0));
     const float us = fmaf(fm, pu2, nu0) * rw, vs = fmaf(fm, pv2, nv0) * rw;
-    const int iu0 = min(max(__float2int_rd(us + ou), R.u0), u_first);
-    const int iv0 = min(max(__float2int_rd(vs + ov), R.v0), v_first);
-    const int st0 = (iv0 - R.v0) * sv + (iu0 - R.u0) * su;
+    const float fu = __fadd_rd(fminf(fmaxf(us + ou, u_lo), u_hi), kFloorMagic);
+    const float fv = __fadd_rd(fminf(fmaxf(vs + ov, v_lo), v_hi), kFloorMagic);
+    const int st0 = int(__float_as_uint(fv)) * sv + int(__float_as_uint(fu)) * su + origin;
+    const float u0 = fu - kFloorMagic, v0 = fv - kFloorMagic;
+    const VoxelForms f = voxel_forms(run, m0 + m);
     float acc_m = acc[m];
-    if (kWu > 0) {
+    if constexpr (kWu > 0) {
+      f32x2 column[kWu];
+#pragma unroll
+      for (int c = 0; c < kWu; ++c) column[c] = form_column(f, u0 + float(c));
 #pragma unroll
       for (int r = 0; r < kWv; ++r) {
 #pragma unroll
         for (int c = 0; c < kWu; ++c) {
-          const int st = st0 + r * sv + c * su;
-          const float4 r4 = s_ray[st];
-          const float wa = __saturatef(1.0f - fabsf(fmaf(kt, r4.y, r4.x) - it));
-          const float wb = __saturatef(1.0f - fabsf(fmaf(kt, r4.w, r4.z) - jt));
-          acc_m = fmaf(wa * wb, s_val[st], acc_m);
+          const float2 p = s_pix[st0 + r * sv + c * su];
+          acc_m = fmaf(pixel_weight(f, column[c], v0 + float(r), p.x), p.y, acc_m);
         }
       }
     } else {
       for (int r = 0; r < R.wv; ++r) {
         for (int c = 0; c < R.wu; ++c) {
-          const int st = st0 + r * sv + c * su;
-          const float4 r4 = s_ray[st];
-          const float wa = __saturatef(1.0f - fabsf(fmaf(kt, r4.y, r4.x) - it));
-          const float wb = __saturatef(1.0f - fabsf(fmaf(kt, r4.w, r4.z) - jt));
-          acc_m = fmaf(wa * wb, s_val[st], acc_m);
+          const float2 p = s_pix[st0 + r * sv + c * su];
+          acc_m = fmaf(pixel_weight(f, form_column(f, u0 + float(c)), v0 + float(r), p.x), p.y,
+                       acc_m);
         }
       }
     }
@@ -674,15 +722,13 @@ __device__ __forceinline__ void gen_window_run(const AngleParams& ap, const GenR
 }
 
 template <int kGenRunX, int kZl>
-__global__ void __launch_bounds__(kGenThreads, 4)
+__global__ void __launch_bounds__(kGenThreads, 3)
     bp_general_box_kernel(const AngleParams* __restrict__ params,
-                          const ColumnEntry* __restrict__ columns,
                           const int* __restrict__ angles, int n_angles,
                           const float2* __restrict__ sinow, float* __restrict__ vol,
                           DeviceGeometry g, int additive) {
   constexpr int zlayout = kZl;
-  __shared__ float4 s_ray[kGenStage];  // Xa, ma, Xb, mb
-  __shared__ float s_val[kGenStage];   // W y
+  __shared__ float2 s_pix[kGenStage];  // 1 / den, W y
   __shared__ GenRegion s_reg[2];       // regions of angles n and n + 1
   const int tid = threadIdx.x, warp = tid >> 5;
   constexpr int kGenBoxX = 2 * kGenRunX;
@@ -725,10 +771,9 @@ __global__ void __launch_bounds__(kGenThreads, 4)
       int q = t0 / inner, r = t0 % inner;
       for (int t = t0; t < total; t += kStagers) {
         const int iu = R.u0 + (zlayout ? q : r), iv = R.v0 + (zlayout ? r : q);
-        const Ray ray = pixel_ray(ap, columns, g, theta, iu, iv);
-        const int st = q * stride + r;
-        s_ray[st] = make_float4(ray.Xa, ray.ma, ray.Xb, ray.mb);
-        s_val[st] = __ldg(base + iv * pv.s_row + iu * pv.s_col).x;
+        s_pix[q * stride + r] =
+            make_float2(pixel_rden(ap, float(iu - g.ou), float(iv - g.ov)),
+                        __ldg(base + iv * pv.s_row + iu * pv.s_col).x);
         q += step_q;
         r += step_r;
         if (r >= inner) {
@@ -744,29 +789,25 @@ __global__ void __launch_bounds__(kGenThreads, 4)
       // the common window shapes get fully unrolled sums
       switch (R.wu * 16 + R.wv) {  // wv <= kGenWindow < 16
         case 3 * 16 + 2:
-          gen_window_run<kGenRunX, kZl, 3, 2>(ap, R, g, s_ray, s_val, zt, yt, xt0, x0, acc);
+          gen_window_run<kGenRunX, kZl, 3, 2>(ap, R, g, s_pix, zt, yt, xt0, x0, acc);
           break;
         case 2 * 16 + 2:
-          gen_window_run<kGenRunX, kZl, 2, 2>(ap, R, g, s_ray, s_val, zt, yt, xt0, x0, acc);
+          gen_window_run<kGenRunX, kZl, 2, 2>(ap, R, g, s_pix, zt, yt, xt0, x0, acc);
           break;
         case 3 * 16 + 3:
-          gen_window_run<kGenRunX, kZl, 3, 3>(ap, R, g, s_ray, s_val, zt, yt, xt0, x0, acc);
+          gen_window_run<kGenRunX, kZl, 3, 3>(ap, R, g, s_pix, zt, yt, xt0, x0, acc);
           break;
         case 2 * 16 + 3:
-          gen_window_run<kGenRunX, kZl, 2, 3>(ap, R, g, s_ray, s_val, zt, yt, xt0, x0, acc);
+          gen_window_run<kGenRunX, kZl, 2, 3>(ap, R, g, s_pix, zt, yt, xt0, x0, acc);
           break;
         default:
-          gen_window_run<kGenRunX, kZl, 0, 0>(ap, R, g, s_ray, s_val, zt, yt, xt0, x0, acc);
+          gen_window_run<kGenRunX, kZl, 0, 0>(ap, R, g, s_pix, zt, yt, xt0, x0, acc);
       }
     } else if (zy_in && R.mode == 1) {
-      // The thread's voxels run along x, which is one of the angle's axes
-      // d, a, b: their (kt, it, jt) step by 1 along that one.
-      const int d = ap.d, a = ap.a;
-      const float kt0 = d == 0 ? zt : (d == 1 ? yt : xt0);
-      const float it0 = a == 0 ? zt : (a == 1 ? yt : xt0);
-      const float jt0 = (d != 0 && a != 0) ? zt : ((d != 1 && a != 1) ? yt : xt0);
-      const float dk = d == 2 ? 1.0f : 0.0f, di = a == 2 ? 1.0f : 0.0f;
-      const float dj = 1.0f - dk - di;
+      const int a = ap.a, m0 = kGenRunX == 8 ? 0 : x0 & 7;
+      const float x8 = xt0 - float(m0);
+      const RunForms run = run_forms(ap, coord(ap.d, zt, yt, x8), coord(ap.a, zt, yt, x8),
+                                     coord(ap.b, zt, yt, x8));
       // footprint bound from the centre's projection (u*, v*) = (nu, nv) / nw
       const float Su = fabsf(ap.pu[a]) + fabsf(ap.pu[ap.b]);
       const float Sv = fabsf(ap.pv[a]) + fabsf(ap.pv[ap.b]);
@@ -784,7 +825,6 @@ __global__ void __launch_bounds__(kGenThreads, 4)
       for (int m = 0; m < kGenRunX; ++m) {
         if (x0 + m >= g.nx) break;
         const float fm = float(m);
-        const float kt = fmaf(fm, dk, kt0), it = fmaf(fm, di, it0), jt = fmaf(fm, dj, jt0);
         const float nu = fmaf(fm, pu2, nu0), nv = fmaf(fm, pv2, nv0), nw = fmaf(fm, pw2, nw0);
         const float rw = __fdividef(1.0f, nw), rm = __fdividef(1.0f, nw - Ew);
         const float us = nu * rw, vs = nv * rw;
@@ -802,17 +842,15 @@ __global__ void __launch_bounds__(kGenThreads, 4)
           iv_hi = min(iv_hi, __float2int_ru((vs + dv) + hi_v));
         }
         float acc_m = acc[m];
+        const VoxelForms f = voxel_forms(run, m0 + m);
         // stage index of (iv_lo, iu_lo), region-relative (small), then steps
         int st_row = (iv_lo - R.v0) * R.sv + (iu_lo - R.u0) * R.su;
         for (int iv = iv_lo; iv <= iv_hi; ++iv, st_row += R.sv) {
           int st = st_row;
+          const float v = float(iv - g.ov);
           for (int iu = iu_lo; iu <= iu_hi; ++iu, st += R.su) {
-            const float4 r4 = s_ray[st];
-            // tent(t) as one saturating add (1 - |t| <= 1; NaN saturates to
-            // 0); a weight of 0 adds nothing
-            const float wa = __saturatef(1.0f - fabsf(fmaf(kt, r4.y, r4.x) - it));
-            const float wb = __saturatef(1.0f - fabsf(fmaf(kt, r4.w, r4.z) - jt));
-            acc_m = fmaf(wa * wb, s_val[st], acc_m);
+            const float2 p = s_pix[st];
+            acc_m = fmaf(pixel_weight(f, form_column(f, float(iu - g.ou)), v, p.x), p.y, acc_m);
           }
         }
         acc[m] = acc_m;
@@ -821,8 +859,7 @@ __global__ void __launch_bounds__(kGenThreads, 4)
 #pragma unroll
       for (int m = 0; m < kGenRunX; ++m)
         if (x0 + m < g.nx)
-          acc[m] = general_voxel_terms(ap, columns, base, pv, g, theta, zt, yt,
-                                       float(x0 + m - g.ox), acc[m]);
+          acc[m] = general_voxel_terms(ap, base, pv, g, zt, yt, float(x0 + m - g.ox), acc[m]);
     }
     __syncthreads();  // stage reused and next region visible
   }
@@ -847,7 +884,7 @@ void launch_bp_general(const tsgb_projector* p, const int* angles, int n, const 
   const DeviceGeometry& g = p->g;
   if (p->tuning.bp_general == 1) {
     const dim3 grid((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz);
-    bp_general_kernel<<<grid, dim3(32, 4), 0, stream>>>(p->d_params, p->d_columns, angles, n,
+    bp_general_kernel<<<grid, dim3(32, 4), 0, stream>>>(p->d_params, angles, n,
                                                         pairs, vol, g, additive ? 1 : 0,
                                                         zlayout ? 1 : 0);
     return;
@@ -857,16 +894,16 @@ void launch_bp_general(const tsgb_projector* p, const int* angles, int n, const 
                   (g.nz + kGenBoxZ - 1) / kGenBoxZ);
   const int add = additive ? 1 : 0;
   if (run == 8 && zlayout)
-    bp_general_box_kernel<8, 1><<<grid, kGenThreads, 0, stream>>>(p->d_params, p->d_columns,
+    bp_general_box_kernel<8, 1><<<grid, kGenThreads, 0, stream>>>(p->d_params,
                                                                   angles, n, pairs, vol, g, add);
   else if (run == 8)
-    bp_general_box_kernel<8, 0><<<grid, kGenThreads, 0, stream>>>(p->d_params, p->d_columns,
+    bp_general_box_kernel<8, 0><<<grid, kGenThreads, 0, stream>>>(p->d_params,
                                                                   angles, n, pairs, vol, g, add);
   else if (zlayout)
-    bp_general_box_kernel<4, 1><<<grid, kGenThreads, 0, stream>>>(p->d_params, p->d_columns,
+    bp_general_box_kernel<4, 1><<<grid, kGenThreads, 0, stream>>>(p->d_params,
                                                                   angles, n, pairs, vol, g, add);
   else
-    bp_general_box_kernel<4, 0><<<grid, kGenThreads, 0, stream>>>(p->d_params, p->d_columns,
+    bp_general_box_kernel<4, 0><<<grid, kGenThreads, 0, stream>>>(p->d_params,
                                                                   angles, n, pairs, vol, g, add);
 }
 
