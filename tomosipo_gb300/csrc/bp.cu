@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(128)
 // per SM instead of 4: 35.3 ms).
 constexpr int kGenBoxZ = 16, kGenBoxY = 8;
 constexpr int kGenThreads = 256;
-constexpr int kGenStage = 2048;                           // staged pixels per angle
+constexpr int kGenStage = 4096;  // staged pixels per angle, padding included
 constexpr int kGenWindow = 9;  // largest box-wide window (pixels) summed by every voxel
 static_assert(kGenWindow < 16, "window shapes are keyed as wu * 16 + wv");
 
@@ -620,11 +620,13 @@ __device__ __forceinline__ void gen_region(const AngleParams& ap, const DeviceGe
     r.v0 = v0;
     r.nu = u1 - u0 + 1;
     r.nv = v1 - v0 + 1;
-    // staged in the sinogram's own order, so the staging reads are coalesced,
-    // with an odd stride between columns (rows) so that the two half-warps,
-    // kGenRunX voxels apart along x, read different banks
+    // staged in the sinogram's own order, so the staging reads are coalesced, with a
+    // stride of 4 or 12 (mod 16 8-byte banks) between columns (rows): the 4 x 4
+    // voxels of a half-warp then read 1.03 banks deep on average (1.9 for 16 voxels
+    // along z and an odd stride; scans tilted 0.4 rad with pixels about as large as
+    // voxels)
     const int inner = zlayout ? r.nv : r.nu, outer = zlayout ? r.nu : r.nv;
-    const int stride = inner | 1;
+    const int stride = ((inner + 3) & ~7) + 4;
     if (r.nu <= 0 || r.nv <= 0)
       r.mode = 0;
     else if ((long long)outer * stride > kGenStage)
@@ -734,8 +736,11 @@ __global__ void __launch_bounds__(kGenThreads, 3)
   constexpr int kGenBoxX = 2 * kGenRunX;
   static_assert(kGenBoxZ * kGenBoxY * kGenBoxX / kGenRunX == kGenThreads, "one thread per x run");
   const int bz = blockIdx.z * kGenBoxZ, by = blockIdx.y * kGenBoxY, bx = blockIdx.x * kGenBoxX;
-  // this thread's voxels: (z, y, x0 + m), m < kGenRunX
-  const int z = bz + (tid & 15), y = by + (tid >> 5), x0 = bx + ((tid >> 4) & 1) * kGenRunX;
+  // this thread's voxels: (z, y, x0 + m), m < kGenRunX; a half-warp is 4 (z) x 4 (y)
+  // voxels of one x run, whose candidates fall on different shared-memory banks
+  // with gen_region's stride
+  const int z = bz + (warp & 3) * 4 + (tid & 3), y = by + (warp >> 2) * 4 + ((tid >> 2) & 3);
+  const int x0 = bx + ((tid >> 4) & 1) * kGenRunX;
   const bool zy_in = z < g.nz && y < g.ny;
   const float zt = float(z - g.oz), yt = float(y - g.oy);
   // the box, clipped to the volume, in anchored coordinates (z, y, x)
