@@ -18,7 +18,8 @@ from . import vector_calc as vc
 from .geometry import VolumeGeometry, VolumeVectorGeometry, volume, from_perspective
 from .Data import Data, data
 from .links.base import link, geometry_shape
-from .projector import create_projector, direct_fp, direct_bp, direct_project_batch, BP_KINDS
+from .projector import (BP_KINDS, create_projector, device_ready, direct_bp, direct_fp,
+                        direct_project_batch, project_on_device)
 
 
 def to_astra_compatible_operator_geometry(vg, pg):
@@ -102,7 +103,24 @@ class Operator:
         self.backprojector = backprojector
         self._transpose = BackprojectionOperator(self)
 
+    def _on_device(self, src, out, src_shape, out_shape, forward):
+        """``src`` projected into ``out`` (new if None) without wrapping them in
+        links, or None if they are not device tensors the kernels take as they are
+        (the calls that remain cost about as much as a small projection)."""
+        if not device_ready(src) or tuple(src.shape) != src_shape:
+            return None
+        if out is None:
+            out = (src.new_zeros if self.additive else src.new_empty)(out_shape)
+        elif not device_ready(src, out) or tuple(out.shape) != out_shape:
+            return None
+        vol, sino = (src, out) if forward else (out, src)
+        project_on_device(self.projector, vol, sino, forward, self.additive, self.backprojector)
+        return out
+
     def _fp(self, volume, out=None):
+        done = self._on_device(volume, out, self.domain_shape, self.range_shape, True)
+        if done is not None:
+            return done
         vlink = _to_link(self.astra_compat_vg, volume)
         if out is not None:
             plink = _to_link(self.astra_compat_pg, out)
@@ -116,6 +134,9 @@ class Operator:
         return plink.data
 
     def _bp(self, projection, out=None):
+        done = self._on_device(projection, out, self.range_shape, self.domain_shape, False)
+        if done is not None:
+            return done
         plink = _to_link(self.astra_compat_pg, projection)
         if out is not None:
             vlink = _to_link(self.astra_compat_vg, out)
@@ -159,11 +180,11 @@ class Operator:
 
     @property
     def domain_shape(self):
-        return geometry_shape(self.astra_compat_vg)
+        return self.projector.vol_shape
 
     @property
     def range_shape(self):
-        return geometry_shape(self.astra_compat_pg)
+        return self.projector.sino_shape
 
 
 class BackprojectionOperator:

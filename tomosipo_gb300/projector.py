@@ -68,6 +68,7 @@ class Projector:
         self.vol_shape = tuple(vg.shape)
         self.sino_shape = (rows, vec.shape[0], cols)
         self._handles = {}
+        self._workspace_bytes = {}  # (device, forward, bp_kind) -> bytes
 
     def handle(self, device_index):
         h = self._handles.get(device_index)
@@ -88,11 +89,15 @@ class Projector:
         return h
 
     def workspace_bytes(self, device_index, forward, bp_kind="matched"):
-        lib = _native.load()
-        h = self.handle(device_index)
-        if forward:
-            return int(lib.tsgb_fp_workspace_bytes(h))
-        return int(lib.tsgb_bp_workspace_bytes(h, BP_KINDS[bp_kind]))
+        key = (device_index, forward, bp_kind)
+        nbytes = self._workspace_bytes.get(key)
+        if nbytes is None:
+            lib = _native.load()
+            h = self.handle(device_index)
+            nbytes = int(lib.tsgb_fp_workspace_bytes(h) if forward
+                         else lib.tsgb_bp_workspace_bytes(h, BP_KINDS[bp_kind]))
+            self._workspace_bytes[key] = nbytes
+        return nbytes
 
     def stats(self, device_index):
         """Plan statistics of the native projector (see tsgb_projector_stats)."""
@@ -127,6 +132,7 @@ class Projector:
         t = _native.Tuning(**cur)
         _native.check(_native.load().tsgb_projector_set_tuning(self.handle(idx), ctypes.byref(t)),
                       "tsgb_projector_set_tuning")
+        self._workspace_bytes.clear()
 
     def __del__(self):
         handles, self._handles = getattr(self, "_handles", {}), {}
@@ -369,6 +375,38 @@ def _project_pipelined(projector, forward, additive, src, dst, device):
             _end(leg, comp)
 
 
+def device_ready(*arrays):
+    """Plain float32 C-contiguous tensors on one CUDA device: what the kernels take
+    as it is. Anything else goes through the links, which convert or refuse it."""
+    first = arrays[0]
+    for t in arrays:
+        if not (type(t) is torch.Tensor and t.is_cuda and t.dtype is torch.float32
+                and t.is_contiguous() and t.device == first.device):
+            return False
+    return True
+
+
+def project_on_device(projector, vol, sino, forward, additive, bp_kind):
+    """Project between CUDA tensors (``device_ready``, of the projector's shapes) on
+    the current stream of their device."""
+    device = vol.device
+    if torch.cuda.current_device() != device.index:
+        with torch.cuda.device(device):
+            return project_on_device(projector, vol, sino, forward, additive, bp_kind)
+    lib = _native.load()
+    h = projector.handle(device.index)
+    nbytes = projector.workspace_bytes(device.index, forward, bp_kind)
+    ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=device)
+    stream = torch.cuda.current_stream(device).cuda_stream
+    if forward:
+        rc = lib.tsgb_direct_fp(h, vol.data_ptr(), sino.data_ptr(), int(bool(additive)),
+                                ws.data_ptr(), nbytes, stream)
+    else:
+        rc = lib.tsgb_direct_bp(h, vol.data_ptr(), sino.data_ptr(), int(bool(additive)),
+                                BP_KINDS[bp_kind], ws.data_ptr(), nbytes, stream)
+    _native.check(rc, "tsgb_direct_fp" if forward else "tsgb_direct_bp")
+
+
 def direct_project(projector, vol_link, proj_link, forward=None, additive=False,
                    bp_kind="matched"):
     """Forward (``forward=True``) or back project between two links."""
@@ -399,19 +437,8 @@ def direct_project(projector, vol_link, proj_link, forward=None, additive=False,
         return _project_pipelined(projector, forward, additive, src, dst, device)
     d_src, _ = _as_device_tensor(src, device, copy_in=True)
     d_dst, copy_back = _as_device_tensor(dst, device, copy_in=additive)
-    lib = _native.load()
-    with torch.cuda.device(device):
-        h = projector.handle(device.index)
-        stream = torch.cuda.current_stream(device).cuda_stream
-        nbytes = projector.workspace_bytes(device.index, forward, bp_kind)
-        ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=device)
-        if forward:
-            rc = lib.tsgb_direct_fp(h, d_src.data_ptr(), d_dst.data_ptr(), int(bool(additive)),
-                                    ws.data_ptr(), nbytes, stream)
-        else:
-            rc = lib.tsgb_direct_bp(h, d_dst.data_ptr(), d_src.data_ptr(), int(bool(additive)),
-                                    BP_KINDS[bp_kind], ws.data_ptr(), nbytes, stream)
-        _native.check(rc, "tsgb_direct_fp" if forward else "tsgb_direct_bp")
+    d_vol, d_sino = (d_src, d_dst) if forward else (d_dst, d_src)
+    project_on_device(projector, d_vol, d_sino, forward, additive, bp_kind)
     if copy_back:
         # Straight device -> host copy into the caller's buffer (a DMA when it is pinned).
         target = torch.from_numpy(dst) if isinstance(dst, np.ndarray) else dst
