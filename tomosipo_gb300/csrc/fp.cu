@@ -127,36 +127,45 @@ __device__ __forceinline__ FloorSplit floor_split(float q) {
   return {q - (m - kFloorMagic), int(__float_as_uint(m) - kFloorBits)};
 }
 
-// Bilinear sample of plane k from single voxels (four 4-byte taps) ...
+// A plane of the walk: its coordinate and the element offset of its anchored voxel,
+// both stepped from plane to plane (a product and a conversion per sample cost 1.4 %
+// at 256^3 / 360 angles, 3.4 % at 512^3 / 1024).
+struct PlaneStep {
+  float kt;
+  int offset;
+  __device__ __forceinline__ PlaneStep(int k, int stride_d) : kt(float(k)), offset(k * stride_d) {}
+  __device__ __forceinline__ PlaneStep(float kt_, int offset_) : kt(kt_), offset(offset_) {}
+  __device__ __forceinline__ PlaneStep after(float planes, int stride) const {
+    return PlaneStep(kt + planes, offset + stride);
+  }
+};
+
+// Bilinear sample of a plane from single voxels (four 4-byte taps) ... (Scalar
+// arithmetic: packed positions and interpolations took a quarter fewer instructions
+// and 13 % more time at 256^3, since the samples wait for L1, not for issue slots.)
 __device__ __forceinline__ float bilinear_sample(const float* __restrict__ base, const Ray& r,
-                                                 int k, int stride_d, int stride_a) {
-  const float kt = float(k);
-  const float qa = fmaf(kt, r.ma, r.Xa);
-  const float qb = fmaf(kt, r.mb, r.Xb);
-  const FloorSplit sa = floor_split(qa), sb = floor_split(qb);
-  const float fa = sa.frac, fb = sb.frac;
-  const float* p = base + (k * stride_d + sa.i * stride_a + sb.i);
+                                                 const PlaneStep& k, int stride_a) {
+  const FloorSplit sa = floor_split(fmaf(k.kt, r.ma, r.Xa));
+  const FloorSplit sb = floor_split(fmaf(k.kt, r.mb, r.Xb));
+  const float* p = base + (k.offset + sa.i * stride_a + sb.i);
   const float v00 = __ldg(p), v01 = __ldg(p + 1);
   const float v10 = __ldg(p + stride_a), v11 = __ldg(p + stride_a + 1);
-  const float left = fmaf(fb, v01 - v00, v00);
-  const float right = fmaf(fb, v11 - v10, v10);
-  return fmaf(fa, right - left, left);
+  const float left = fmaf(sb.frac, v01 - v00, v00);
+  const float right = fmaf(sb.frac, v11 - v10, v10);
+  return fmaf(sa.frac, right - left, left);
 }
 
 // ... or from pairs (two 8-byte taps, each holding both b neighbours); the
 // arithmetic is the same, so both give identical results.
 __device__ __forceinline__ float bilinear_sample(const float2* __restrict__ base, const Ray& r,
-                                                 int k, int stride_d, int stride_a) {
-  const float kt = float(k);
-  const float qa = fmaf(kt, r.ma, r.Xa);
-  const float qb = fmaf(kt, r.mb, r.Xb);
-  const FloorSplit sa = floor_split(qa), sb = floor_split(qb);
-  const float fa = sa.frac, fb = sb.frac;
-  const float2* p = base + (k * stride_d + sa.i * stride_a + sb.i);
+                                                 const PlaneStep& k, int stride_a) {
+  const FloorSplit sa = floor_split(fmaf(k.kt, r.ma, r.Xa));
+  const FloorSplit sb = floor_split(fmaf(k.kt, r.mb, r.Xb));
+  const float2* p = base + (k.offset + sa.i * stride_a + sb.i);
   const float2 v0 = __ldg(p), v1 = __ldg(p + stride_a);
-  const float left = fmaf(fb, v0.y - v0.x, v0.x);
-  const float right = fmaf(fb, v1.y - v1.x, v1.x);
-  return fmaf(fa, right - left, left);
+  const float left = fmaf(sb.frac, v0.y - v0.x, v0.x);
+  const float right = fmaf(sb.frac, v1.y - v1.x, v1.x);
+  return fmaf(sa.frac, right - left, left);
 }
 
 // The padded volume copy an angle samples: anchored voxel (0, 0, 0) and strides.
@@ -215,8 +224,8 @@ __device__ __forceinline__ RaySpan prepare_span(const AngleParams& ap,
 }
 
 template <typename E>
-__device__ __forceinline__ float sample(const CopyView<E>& v, const Ray& r, int k) {
-  return bilinear_sample(v.base, r, k, v.stride_d, v.stride_a);
+__device__ __forceinline__ float sample(const CopyView<E>& v, const Ray& r, const PlaneStep& k) {
+  return bilinear_sample(v.base, r, k, v.stride_a);
 }
 
 // Samples of planes k0..k1 are summed into two partial sums by the parity of
@@ -226,12 +235,18 @@ template <typename E>
 __device__ __forceinline__ void walk(const CopyView<E>& v, const Ray& r, int k0, int k1, float& e,
                                      float& o) {
   int k = k0;
-  if (k <= k1 && (k & 1)) o += sample(v, r, k++);
-  for (; k < k1; k += 2) {
-    e += sample(v, r, k);
-    o += sample(v, r, k + 1);
+  PlaneStep s(k, v.stride_d);
+  if (k <= k1 && (k & 1)) {
+    o += sample(v, r, s);
+    s = s.after(1.0f, v.stride_d);
+    ++k;
   }
-  if (k == k1) e += sample(v, r, k);
+  for (; k < k1; k += 2) {
+    e += sample(v, r, s);
+    o += sample(v, r, s.after(1.0f, v.stride_d));
+    s = s.after(2.0f, 2 * v.stride_d);
+  }
+  if (k == k1) e += sample(v, r, s);
 }
 
 // Ray sum (scaled by the plane step) of pixel (iv, iu) at angle theta. If W
@@ -269,20 +284,24 @@ __device__ __forceinline__ void fp_ray_pair(const AngleParams& apa, const AngleP
     walk(va, a.r, a.k0, lo - 1, ea, oa);
     walk(va, b.r, b.k0, lo - 1, eb, ob);
     int k = lo;
+    PlaneStep s(k, va.stride_d);
     if (k & 1) {
-      oa += sample(va, a.r, k);
-      ob += sample(va, b.r, k);
+      oa += sample(va, a.r, s);
+      ob += sample(va, b.r, s);
+      s = s.after(1.0f, va.stride_d);
       ++k;
     }
     for (; k < hi; k += 2) {
-      ea += sample(va, a.r, k);
-      eb += sample(va, b.r, k);
-      oa += sample(va, a.r, k + 1);
-      ob += sample(va, b.r, k + 1);
+      const PlaneStep next = s.after(1.0f, va.stride_d);
+      ea += sample(va, a.r, s);
+      eb += sample(va, b.r, s);
+      oa += sample(va, a.r, next);
+      ob += sample(va, b.r, next);
+      s = s.after(2.0f, 2 * va.stride_d);
     }
     if (k == hi) {
-      ea += sample(va, a.r, k);
-      eb += sample(va, b.r, k);
+      ea += sample(va, a.r, s);
+      eb += sample(va, b.r, s);
     }
     walk(va, a.r, hi + 1, a.k1, ea, oa);
     walk(va, b.r, hi + 1, b.k1, eb, ob);
