@@ -1454,14 +1454,9 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
       continue;
     }
     if (bp_uses_zlane(p)) {
-      for (int k = 0; k < m; ++k)
-        launch_bp_weight_z(p, sino + (i0 + k) * sino_elems,
-                           reinterpret_cast<float*>(workspace + k * item_bytes), 0, g.nangles,
-                           stream);
-      launch_bp_zlane_separable(p, 0, n_ax, n_ax, n_ay, reinterpret_cast<const float*>(workspace),
-                                reinterpret_cast<float*>(workspace + bp_pairs_bytes(g)),
-                                vol + i0 * vol_elems, additive ? 1 : 0, nullptr, stream, m,
-                                item_bytes);
+      const int rc = launch_bp_zlane_batch(p, vol + i0 * vol_elems, sino + i0 * sino_elems, m,
+                                           additive, workspace, stream);
+      if (rc != 0) return rc;
       continue;
     }
     for (int k = 0; k < m; ++k)

@@ -70,31 +70,59 @@ __device__ __forceinline__ float weighted_pixel_z(const AngleParams& ap, const C
 // rows of W y it needs into shared memory (reads along u, coalesced), then
 // writes the pairs along the rows (coalesced). Every padded pair is written,
 // so the buffer needs no clearing. `out` points at the angle range's first
-// column; blockIdx.z counts angles from `theta0`.
+// column; blockIdx.z counts angles from `theta0`, over groups of kItems stacked
+// sinograms: with kItems = 2 an element holds both items' pairs.
+template <int kItems>
 __global__ void __launch_bounds__(256)
     bp_weight_z_kernel(const AngleParams* __restrict__ params,
                        const ColumnEntry* __restrict__ columns, const float* __restrict__ sino,
-                       float2* __restrict__ out, DeviceGeometry g, int theta0) {
-  __shared__ float s[33][33];  // [row][column]
-  const int theta = theta0 + blockIdx.z;
+                       float2* __restrict__ out, long long group_pairs, DeviceGeometry g,
+                       int theta0, int n_angles, int groups) {
+  __shared__ float s[kItems][33][33];  // [item][row][column]
   const int iu0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int RP = g.rows + 2 * kRowPad;
-  const AngleParams& ap = params[theta];
-  {
-    const int iu = iu0 + threadIdx.x;
-    ColumnEntry ce{};
-    if (ap.separable && iu < g.cols) ce = columns[(size_t)theta * g.cols + iu];
-    for (int k = threadIdx.y; k < 33; k += 8)
-      s[k][threadIdx.x] = weighted_pixel_z(ap, ce, sino, g, r0 + k - kRowPad, iu, theta);
+  const size_t item = (size_t)g.rows * g.nangles * g.cols;
+  for (long long b = blockIdx.z; b < (long long)n_angles * groups; b += gridDim.z) {
+    const int group = int(b / n_angles), n = int(b - (long long)group * n_angles);
+    const int theta = theta0 + n;
+    const AngleParams& ap = params[theta];
+    {
+      const int iu = iu0 + threadIdx.x;
+      ColumnEntry ce{};
+      if (ap.separable && iu < g.cols) ce = columns[(size_t)theta * g.cols + iu];
+#pragma unroll
+      for (int i = 0; i < kItems; ++i)
+        for (int k = threadIdx.y; k < 33; k += 8)
+          s[i][k][threadIdx.x] = weighted_pixel_z(ap, ce, sino + (group * kItems + i) * item, g,
+                                                  r0 + k - kRowPad, iu, theta);
+    }
+    __syncthreads();
+    const int r = r0 + threadIdx.x;
+    for (int c = threadIdx.y; c < 32 && iu0 + c < g.cols && r < RP; c += 8) {
+      const size_t at = ((size_t)n * g.cols + iu0 + c) * RP + r;
+      float2 v[kItems];
+#pragma unroll
+      for (int i = 0; i < kItems; ++i)
+        v[i] = make_float2(s[i][threadIdx.x][c], s[i][threadIdx.x + 1][c]);
+      if constexpr (kItems == 2)
+        reinterpret_cast<float4*>(out + group * group_pairs)[at] =
+            make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+      else
+        out[group * group_pairs + at] = v[0];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int r = r0 + threadIdx.x;
-  if (r >= RP) return;
-  for (int c = threadIdx.y; c < 32; c += 8) {
-    const int iu = iu0 + c;
-    if (iu >= g.cols) break;
-    out[((size_t)blockIdx.z * g.cols + iu) * RP + r] =
-        make_float2(s[threadIdx.x][c], s[threadIdx.x + 1][c]);
+}
+
+// The row pairs of the kItems items at one element.
+template <int kItems>
+__device__ __forceinline__ void load_rows(const char* p, float2 (&y)[kItems]) {
+  if constexpr (kItems == 2) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    y[0] = make_float2(v.x, v.y);
+    y[1] = make_float2(v.z, v.w);
+  } else {
+    y[0] = __ldg(reinterpret_cast<const float2*>(p));
   }
 }
 
@@ -111,14 +139,15 @@ __global__ void __launch_bounds__(256)
 // time was waiting for L1 and L2 at 256^3 (5.2 -> 4.6 ms per backprojection,
 // although fewer warps fit). 16 voxels per lane leave no registers for this
 // (116 ms at 512^3 / 1024 angles, against 100 ms for two ranges of 8).
-template <int kX, int kRun, bool kClamp>
-__device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
+template <bool kClamp, int kRun, int kItems, int kX>
+__device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kItems][kX][(kRun + 1) / 2],
                                               const float4 (&list)[34][4], int n, float zt,
                                               float vmin, float vmax) {
   constexpr int kPairs = (kRun + 1) / 2;
+  constexpr size_t kElem = sizeof(float2) * kItems;
   struct Stage {
     f32x2 t[kPairs];
-    float2 ya[kPairs], yb[kPairs];
+    float2 ya[kPairs][kItems], yb[kPairs][kItems];
   } st[2];
   const auto stage = [&](Stage& S, const float4(&entry)[4]) {
     const float4 e0 = entry[0], e1 = entry[1];
@@ -140,26 +169,30 @@ __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
       S.t[jj] = add2(fma2(v0, Sl2, pack2(C0 - float(32 * ja), C0 - float(32 * jb))), Bl2);
       float fa, fb;
       unpack2(f, fa, fb);
-      S.ya[jj] = __ldg(reinterpret_cast<const float2*>(colb + size_t(__float_as_uint(fa)) * sizeof(float2)));
-      S.yb[jj] = __ldg(reinterpret_cast<const float2*>(colb + size_t(__float_as_uint(fb)) * sizeof(float2)));
+      load_rows(colb + size_t(__float_as_uint(fa)) * kElem, S.ya[jj]);
+      load_rows(colb + size_t(__float_as_uint(fb)) * kElem, S.yb[jj]);
     }
   };
   const auto finish = [&](const Stage& S, const float4(&entry)[4]) {
     const float4 e2 = entry[2];
     const float2 e3 = *reinterpret_cast<const float2*>(&entry[3]);
-    f32x2 V[kPairs];
+    f32x2 V[kItems][kPairs];
 #pragma unroll
     for (int jj = 0; jj < kPairs; ++jj) {
       float ta, tb;
       unpack2(S.t[jj], ta, tb);
       ta = fabsf(ta);
       tb = fabsf(tb);
-      V[jj] = pack2(fmaf(__saturatef(1.0f - ta), S.ya[jj].x, __saturatef(e3.y + ta) * S.ya[jj].y),
-                   fmaf(__saturatef(1.0f - tb), S.yb[jj].x, __saturatef(e3.y + tb) * S.yb[jj].y));
+      const float wa0 = __saturatef(1.0f - ta), wa1 = __saturatef(e3.y + ta);
+      const float wb0 = __saturatef(1.0f - tb), wb1 = __saturatef(e3.y + tb);
+#pragma unroll
+      for (int i = 0; i < kItems; ++i)
+        V[i][jj] = pack2(fmaf(wa0, S.ya[jj][i].x, __fmul_rn(wa1, S.ya[jj][i].y)),
+                         fmaf(wb0, S.yb[jj][i].x, __fmul_rn(wb1, S.yb[jj][i].y)));
     }
-    const auto profile = [&](int jj) { return V[jj]; };
-    window_dispatch<kX, kPairs, -1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
-                                    pack2(e2.z, e2.w));
+    const auto profile = [&](int i, int jj) { return V[i][jj]; };
+    window_dispatch<-1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
+                            pack2(e2.z, e2.w));
   };
   if (n == 0) return;
   const float4(*entry)[4] = list;
@@ -184,15 +217,16 @@ __device__ __forceinline__ void zlane_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
 // true one; NaN clamps to the low end). Loads a column ahead where the registers
 // hold two stages (2 x 2 supersampled 128 x 160 x 160 / 200: 2.21 -> 1.95 ms per
 // backprojection).
-template <int kX, int kRun>
-__device__ __forceinline__ void zlane_fine_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
+template <int kRun, int kItems, int kX>
+__device__ __forceinline__ void zlane_fine_columns(f32x2 (&acc)[kItems][kX][(kRun + 1) / 2],
                                                    const float4 (&list)[34][4], int n, float zt,
                                                    float vmin, float vmax) {
   constexpr int kPairs = (kRun + 1) / 2, kN = 2 * kPairs;
-  constexpr int kStages = kRun <= 4 ? 2 : 1;
+  constexpr int kStages = kRun * kItems <= 4 ? 2 : 1;
+  constexpr size_t kElem = sizeof(float2) * kItems;
   struct Stage {
     float t[kN];
-    float2 y01[kN], y23[kN];
+    float2 y01[kN][kItems], y23[kN][kItems];
   } st[kStages];
   const auto stage = [&](Stage& S, const float4(&entry)[4]) {
     const float4 e0 = entry[0], e1 = entry[1];
@@ -204,34 +238,39 @@ __device__ __forceinline__ void zlane_fine_columns(f32x2 (&acc)[kX][(kRun + 1) /
     for (int j = 0; j < kN; ++j) {
       const float t = fminf(fmaxf(fmaf(float(j), dv, vs0), vmin - 1.0f), vmax - 2.0f);
       const float f = __fadd_rd(t, kFloorMagic);
-      const float2* p = reinterpret_cast<const float2*>(
-          colb + size_t(__float_as_uint(f) + 1u) * sizeof(float2));
+      const char* p = colb + size_t(__float_as_uint(f) + 1u) * kElem;
       S.t[j] = fmaf(f - kFloorMagic, e0.x, C0 - float(32 * j)) + e0.z;
-      S.y01[j] = __ldg(p);
-      S.y23[j] = __ldg(p + 2);
+      load_rows(p, S.y01[j]);
+      load_rows(p + 2 * kElem, S.y23[j]);
     }
   };
   const auto finish = [&](const Stage& S, const float4(&entry)[4]) {
     const float Sl = entry[0].x;
     const float4 e2 = entry[2];
     const float f0 = entry[3].x;
-    f32x2 V[kPairs];
+    f32x2 V[kItems][kPairs];
 #pragma unroll
     for (int jj = 0; jj < kPairs; ++jj) {
-      float v[2];
+      float v[kItems][2];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int j = 2 * jj + i;
-        v[i] = __saturatef(1.0f - fabsf(S.t[j] + Sl)) * S.y01[j].x;
-        v[i] = fmaf(__saturatef(1.0f - fabsf(fmaf(2.0f, Sl, S.t[j]))), S.y01[j].y, v[i]);
-        v[i] = fmaf(__saturatef(1.0f - fabsf(fmaf(3.0f, Sl, S.t[j]))), S.y23[j].x, v[i]);
-        v[i] = fmaf(__saturatef(1.0f - fabsf(fmaf(4.0f, Sl, S.t[j]))), S.y23[j].y, v[i]);
+      for (int h = 0; h < 2; ++h) {
+        const int j = 2 * jj + h;
+        const float w0 = __saturatef(1.0f - fabsf(S.t[j] + Sl));
+        const float w1 = __saturatef(1.0f - fabsf(fmaf(2.0f, Sl, S.t[j])));
+        const float w2 = __saturatef(1.0f - fabsf(fmaf(3.0f, Sl, S.t[j])));
+        const float w3 = __saturatef(1.0f - fabsf(fmaf(4.0f, Sl, S.t[j])));
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+          v[i][h] = fmaf(w3, S.y23[j][i].y,
+                         fmaf(w2, S.y23[j][i].x,
+                              fmaf(w1, S.y01[j][i].y, __fmul_rn(w0, S.y01[j][i].x))));
       }
-      V[jj] = pack2(v[0], v[1]);
+#pragma unroll
+      for (int i = 0; i < kItems; ++i) V[i][jj] = pack2(v[i][0], v[i][1]);
     }
-    const auto profile = [&](int jj) { return V[jj]; };
-    window_dispatch<kX, kPairs, -1, kX>(acc, __float_as_int(f0), profile, pack2(e2.x, e2.y),
-                                        pack2(e2.z, e2.w));
+    const auto profile = [&](int i, int jj) { return V[i][jj]; };
+    window_dispatch<-1, kX>(acc, __float_as_int(f0), profile, pack2(e2.x, e2.y),
+                            pack2(e2.z, e2.w));
   };
   if (n == 0) return;
   if constexpr (kStages == 1) {
@@ -255,30 +294,29 @@ __device__ __forceinline__ void zlane_fine_columns(f32x2 (&acc)[kX][(kRun + 1) /
 
 // The columns of a list with rows less than half a voxel apart among them: every row
 // whose tent reaches the voxel.
-template <int kX, int kRun>
-__device__ __forceinline__ void zlane_any_columns(f32x2 (&acc)[kX][(kRun + 1) / 2],
+template <int kRun, int kItems, int kX>
+__device__ __forceinline__ void zlane_any_columns(f32x2 (&acc)[kItems][kX][(kRun + 1) / 2],
                                                   const float4 (&list)[34][4], int n, float zt,
                                                   const DeviceGeometry& g) {
-  constexpr int kPairs = (kRun + 1) / 2;
   for (int k = 0; k < n; ++k) {
     const float4 e0 = list[k][0], e1 = list[k][1], e2 = list[k][2], e3 = list[k][3];
     const float Sl = e0.x, inv = e1.x, C0 = (e1.y - zt) + e0.z;
     const float2* col = reinterpret_cast<const float2*>(  // anchored row 0
         (size_t(__float_as_uint(e1.z)) | (size_t(__float_as_uint(e1.w)) << 32)) +
-        size_t(kFloorBits) * sizeof(float2));
-    const auto rows = [&](int j) {
+        size_t(kFloorBits) * sizeof(float2) * kItems);
+    const auto rows = [&](int i, int j) {
       const float Bj = C0 - float(32 * j);
       const float v1 = (-1.0f - Bj) * inv, v2 = (1.0f - Bj) * inv;
       const int iv_lo = max(0, (int)floorf(clamp_coord(fminf(v1, v2))) + g.ov);
       const int iv_hi = min(g.rows - 1, (int)ceilf(clamp_coord(fmaxf(v1, v2))) + g.ov);
       float V = 0.0f;
       for (int iv = iv_lo; iv <= iv_hi; ++iv)
-        V = fmaf(tent(fmaf(float(iv - g.ov), Sl, Bj)), __ldg(col + (iv - g.ov)).x, V);
+        V = fmaf(tent(fmaf(float(iv - g.ov), Sl, Bj)), __ldg(col + (iv - g.ov) * kItems + i).x, V);
       return V;
     };
-    const auto profile = [&](int jj) { return pack2(rows(2 * jj), rows(2 * jj + 1)); };
-    window_dispatch<kX, kPairs, -1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
-                                        pack2(e2.z, e2.w));
+    const auto profile = [&](int i, int jj) { return pack2(rows(i, 2 * jj), rows(i, 2 * jj + 1)); };
+    window_dispatch<-1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
+                            pack2(e2.z, e2.w));
   }
 }
 
@@ -292,7 +330,7 @@ struct ZlaneArgs {
   const ColumnEntry* columns;
   const float2* sinoz;         // column-major row pairs
   float* volt[2];              // [y][x][z] sum of each pass, z rows zs apart
-  long long item_pairs, item_volt;
+  long long group_pairs, item_volt;  // strides: blockIdx.z (pairs), item (floats)
   int zs;
   DeviceGeometry g;
 };
@@ -309,7 +347,11 @@ struct ZlaneArgs {
 // shared memory (a column is then two 16-byte broadcast reads). With all lanes
 // alike this was 30 instructions per angle and 25 per column, which a run of
 // few voxels along z does not hide.
-template <int kX, int kRun, int kPlanes, int kMinBlocks>
+//
+// kItems = 2: a warp works on two stacked items at once (float4 elements): they share
+// the columns, rows and weights, and an item then costs a multiply and three
+// multiply-adds per voxel and column instead of the whole profile.
+template <int kX, int kRun, int kPlanes, int kMinBlocks, int kItems>
 __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
     bp_zlane_kernel(const __grid_constant__ ZlaneArgs A) {
   constexpr int kPairs = (kRun + 1) / 2;
@@ -331,13 +373,15 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
   const int n_angles = A.n[pass];
   const float4* __restrict__ solve = reinterpret_cast<const float4*>(A.solve[pass]);
   const float4* __restrict__ col4 = reinterpret_cast<const float4*>(A.columns);
-  const char* sino0 = reinterpret_cast<const char*>(A.sinoz + blockIdx.z * A.item_pairs +
-                                                    (kRowPad + g.ov));
-  f32x2 acc[kX][kPairs];
+  const char* sino0 = reinterpret_cast<const char*>(A.sinoz + blockIdx.z * A.group_pairs +
+                                                    (kRowPad + g.ov) * kItems);
+  f32x2 acc[kItems][kX][kPairs];
 #pragma unroll
-  for (int m = 0; m < kX; ++m)
+  for (int i = 0; i < kItems; ++i)
 #pragma unroll
-    for (int j = 0; j < kPairs; ++j) acc[m][j] = 0ull;
+    for (int m = 0; m < kX; ++m)
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j) acc[i][m][j] = 0ull;
 
   for (int n0 = 0; n0 < n_angles; n0 += 32) {
     const ColumnRanges cr = column_ranges(solve, n0 + lane, n_angles, kt, i0t - 1.0f,
@@ -371,7 +415,7 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
         const bool inside = fminf(ra, rb) >= vmin + margin && fmaxf(ra, rb) < vmax + 1.0f - margin;
         path = aSl >= 1.0f ? (inside ? 0 : 1) : aSl >= 0.5f ? 2 : 3;
         const size_t colb = reinterpret_cast<size_t>(sino0) +
-                            (ci * RP - size_t(kFloorBits)) * sizeof(float2);
+                            (ci * RP - size_t(kFloorBits)) * sizeof(float2) * kItems;
         // B as a multiple of 2^-14 plus a remainder, so that B - z is exact
         const float Bh = (B + 768.0f) - 768.0f, Bl = B - Bh;
         e0 = make_float4(Sl, Sl, Bl, Bl);
@@ -397,30 +441,33 @@ __global__ void __launch_bounds__(32 * kPlanes, kMinBlocks)
       __syncwarp();
       const int columns_in = __popc(mask);
       if (paths == 0)
-        zlane_columns<kX, kRun, false>(acc, s_list[w], columns_in, zt, vmin, vmax);
+        zlane_columns<false, kRun>(acc, s_list[w], columns_in, zt, vmin, vmax);
       else if (paths == 1)
-        zlane_columns<kX, kRun, true>(acc, s_list[w], columns_in, zt, vmin, vmax);
+        zlane_columns<true, kRun>(acc, s_list[w], columns_in, zt, vmin, vmax);
       else if (paths == 2)
-        zlane_fine_columns<kX, kRun>(acc, s_list[w], columns_in, zt, vmin, vmax);
+        zlane_fine_columns<kRun>(acc, s_list[w], columns_in, zt, vmin, vmax);
       else
-        zlane_any_columns<kX, kRun>(acc, s_list[w], columns_in, zt, g);
+        zlane_any_columns<kRun>(acc, s_list[w], columns_in, zt, g);
       __syncwarp();  // the list is rewritten
     }
   }
   // [y][x][z] scratch: lanes along z, coalesced
-  float* __restrict__ volt = A.volt[pass] + blockIdx.z * A.item_volt;
 #pragma unroll
-  for (int m = 0; m < kX; ++m) {
-    const int ia = i0 + m;
-    if (ia >= n_a) break;
-    float* out = volt + (pass ? (size_t)ia * g.nx + ip : (size_t)ip * g.nx + ia) * A.zs;
+  for (int i = 0; i < kItems; ++i) {
+    float* __restrict__ volt = A.volt[pass] + (blockIdx.z * kItems + i) * A.item_volt;
 #pragma unroll
-    for (int jj = 0; jj < kPairs; ++jj) {
-      float va, vb;
-      unpack2(acc[m][jj], va, vb);
-      const int z = z0 + 64 * jj;
-      if (z < g.nz) out[z] = va;
-      if (2 * jj + 1 < kRun && z + 32 < g.nz) out[z + 32] = vb;
+    for (int m = 0; m < kX; ++m) {
+      const int ia = i0 + m;
+      if (ia >= n_a) break;
+      float* out = volt + (pass ? (size_t)ia * g.nx + ip : (size_t)ip * g.nx + ia) * A.zs;
+#pragma unroll
+      for (int jj = 0; jj < kPairs; ++jj) {
+        float va, vb;
+        unpack2(acc[i][m][jj], va, vb);
+        const int z = z0 + 64 * jj;
+        if (z < g.nz) out[z] = va;
+        if (2 * jj + 1 < kRun && z + 32 < g.nz) out[z + 32] = vb;
+      }
     }
   }
 }
@@ -470,8 +517,8 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <int kX, int kRun, int kPlanes, int kMinBlocks>
-void launch_zlane_shape(ZlaneArgs& A, int items, cudaStream_t stream) {
+template <int kX, int kRun, int kPlanes, int kMinBlocks, int kItems = 1>
+void launch_zlane_shape(ZlaneArgs& A, int groups, cudaStream_t stream) {
   const DeviceGeometry& g = A.g;
   unsigned blocks[2];
   for (int pass = 0; pass < 2; ++pass) {
@@ -481,8 +528,8 @@ void launch_zlane_shape(ZlaneArgs& A, int items, cudaStream_t stream) {
   }
   A.blocks0 = blocks[0];
   const dim3 grid(blocks[0] + blocks[1], unsigned((g.nz + 32 * kRun - 1) / (32 * kRun)),
-                  unsigned(items));
-  bp_zlane_kernel<kX, kRun, kPlanes, kMinBlocks><<<grid, 32 * kPlanes, 0, stream>>>(A);
+                  unsigned(groups));
+  bp_zlane_kernel<kX, kRun, kPlanes, kMinBlocks, kItems><<<grid, 32 * kPlanes, 0, stream>>>(A);
 }
 
 // Warp shapes, by the voxels along z per lane (`run`, from the volume's nz: at
@@ -496,11 +543,16 @@ void launch_zlane_shape(ZlaneArgs& A, int items, cudaStream_t stream) {
 // within 2 %,
 // 128^3 / 200: 6 x 4 warps 0.407, 8 x 4 0.431. The tuning's bp_shape 3 and 4 force other windows for run 8, 5 and
 // 6 cap the run at 4 and 2; any other value takes this rule.
-void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaStream_t stream) {
+int zlane_run(const tsgb_projector* p) {
   const int shape = zlane_shape(p);
   const int most = shape == 5 ? 4 : shape == 6 ? 2 : 8;
-  const int lanes = (A.g.nz + 31) / 32, ranges = (lanes + most - 1) / most;
-  switch ((lanes + ranges - 1) / ranges) {
+  const int lanes = (p->g.nz + 31) / 32, ranges = (lanes + most - 1) / most;
+  return (lanes + ranges - 1) / ranges;
+}
+
+void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaStream_t stream) {
+  const int shape = zlane_shape(p);
+  switch (zlane_run(p)) {
     case 1: return launch_zlane_shape<4, 1, 8, 4>(A, items, stream);
     case 2: return launch_zlane_shape<4, 2, 8, 4>(A, items, stream);
     case 3: return launch_zlane_shape<8, 3, 4, 4>(A, items, stream);
@@ -513,6 +565,46 @@ void launch_zlane_passes(const tsgb_projector* p, ZlaneArgs& A, int items, cudaS
       if (shape == 4) return launch_zlane_shape<3, 8, 8, 2>(A, items, stream);
       return launch_zlane_shape<5, 8, 8, 2>(A, items, stream);
   }
+}
+
+// Two items per warp, where the registers hold both (runs of at most 4). The windows
+// are those of launch_zlane_passes: which columns share a list decides how rows of
+// about a voxel are summed, so other windows would round differently from an item
+// alone. 8 x 128^3 / 128 angles: 1.70 -> 1.05 ms.
+constexpr int kTwoItemRun = 4;
+
+void launch_zlane_two(const tsgb_projector* p, ZlaneArgs& A, int groups, cudaStream_t stream) {
+  switch (zlane_run(p)) {
+    case 1: return launch_zlane_shape<4, 1, 8, 3, 2>(A, groups, stream);
+    case 2: return launch_zlane_shape<4, 2, 8, 3, 2>(A, groups, stream);
+    case 3: return launch_zlane_shape<8, 3, 4, 3, 2>(A, groups, stream);
+    default: return launch_zlane_shape<6, 4, 4, 4, 2>(A, groups, stream);
+  }
+}
+
+// A launch over both angle lists of p (offsets into p->d_sep_angles), without its
+// sinogram and scratch volumes.
+ZlaneArgs zlane_args(const tsgb_projector* p, int off_x, int n_ax, int off_y, int n_ay) {
+  ZlaneArgs A{};
+  A.solve[0] = p->d_solve + off_x;
+  A.solve[1] = p->d_solve + off_y;
+  A.n[0] = n_ax;
+  A.n[1] = n_ay;
+  A.columns = p->d_columns;
+  A.zs = p->g.nz;
+  A.g = p->g;
+  return A;
+}
+
+template <int kItems>
+void launch_weights(const tsgb_projector* p, const float* sino, float2* out, long long group_pairs,
+                    int angle_begin, int n_angles, int groups, cudaStream_t stream) {
+  const DeviceGeometry& g = p->g;
+  const int RP = g.rows + 2 * kRowPad;
+  const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((RP + 31) / 32),
+                  unsigned(std::min<long long>((long long)n_angles * groups, 65535)));
+  bp_weight_z_kernel<kItems><<<grid, dim3(32, 8), 0, stream>>>(
+      p->d_params, p->d_columns, sino, out, group_pairs, g, angle_begin, n_angles, groups);
 }
 
 }  // namespace
@@ -544,45 +636,66 @@ int64_t bp_scratch_bytes(const tsgb_projector* p) {
   return bp_scratch_volumes(p) * bp_volume_bytes(p->g);
 }
 
-int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz_f,
-                       int angle_begin, int angle_end, void* stream_) {
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  float2* sinoz = reinterpret_cast<float2*>(sinoz_f);
+int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz,
+                       int angle_begin, int angle_end, void* stream) {
   const DeviceGeometry& g = p->g;
-  const int RP = g.rows + 2 * kRowPad;
-  for (int a0 = angle_begin; a0 < angle_end; a0 += 65535) {
-    const int n = std::min(angle_end - a0, 65535);
-    const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((RP + 31) / 32), unsigned(n));
-    bp_weight_z_kernel<<<grid, dim3(32, 8), 0, stream>>>(
-        p->d_params, p->d_columns, sino, sinoz + (size_t)a0 * g.cols * RP, g, a0);
-  }
+  float2* out = reinterpret_cast<float2*>(sinoz) +
+                (size_t)angle_begin * g.cols * (g.rows + 2 * kRowPad);
+  if (angle_end > angle_begin)
+    launch_weights<1>(p, sino, out, 0, angle_begin, angle_end - angle_begin, 1,
+                      static_cast<cudaStream_t>(stream));
   return int(cudaGetLastError());
 }
 
 bool launch_bp_zlane_separable(const tsgb_projector* p, int off_x, int n_ax, int off_y, int n_ay,
-                               const float* sinoz_f, float* volt, float* vol, int out_mode,
-                               const float* C, void* stream_, int items, int64_t item_bytes) {
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+                               const float* sinoz, float* volt, float* vol, int out_mode,
+                               const float* C, void* stream) {
   if (n_ax + n_ay == 0) return false;
-  const DeviceGeometry& g = p->g;
-  ZlaneArgs A{};
-  A.solve[0] = p->d_solve + off_x;
-  A.solve[1] = p->d_solve + off_y;
-  A.n[0] = n_ax;
-  A.n[1] = n_ay;
-  A.columns = p->d_columns;
-  A.sinoz = reinterpret_cast<const float2*>(sinoz_f);
+  ZlaneArgs A = zlane_args(p, off_x, n_ax, off_y, n_ay);
+  A.sinoz = reinterpret_cast<const float2*>(sinoz);
   // each pass has its own scratch volume; the transpose adds them
   A.volt[0] = volt;
-  A.volt[1] = n_ax > 0 ? volt + bp_volume_bytes(g) / 4 : volt;
-  A.item_pairs = item_bytes / 8;
-  A.item_volt = item_bytes / 4;
-  A.zs = g.nz;
-  A.g = g;
-  launch_zlane_passes(p, A, items, stream);
-  launch_zlane_out(g, out_mode, volt, n_ax > 0 && n_ay > 0 ? A.volt[1] : nullptr, A.item_volt, A.zs,
-                   vol, C, items, stream);
+  A.volt[1] = n_ax > 0 ? volt + bp_volume_bytes(p->g) / 4 : volt;
+  launch_zlane_passes(p, A, 1, static_cast<cudaStream_t>(stream));
+  launch_zlane_out(p->g, out_mode, volt, n_ax > 0 && n_ay > 0 ? A.volt[1] : nullptr, 0, A.zs, vol,
+                   C, 1, stream);
   return true;
+}
+
+int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino, int items,
+                          bool additive, char* workspace, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const DeviceGeometry& g = p->g;
+  const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - n_ax;
+  const size_t sino_floats = size_t(g.rows) * g.nangles * g.cols;
+  const long long pairs = bp_pairs_bytes(g) / 8, volt = bp_volume_bytes(g) / 4;
+  // weighted sinograms of all items (two items interleaved), then the scratch volumes
+  float2* sinoz = reinterpret_cast<float2*>(workspace);
+  const int two = zlane_run(p) <= kTwoItemRun ? items / 2 : 0, one = items - 2 * two;
+  if (two > 0) launch_weights<2>(p, sino, sinoz, 2 * pairs, 0, g.nangles, two, stream);
+  if (one > 0)
+    launch_weights<1>(p, sino + 2 * two * sino_floats, sinoz + 2 * two * pairs, pairs, 0, g.nangles,
+                      one, stream);
+  ZlaneArgs A = zlane_args(p, 0, n_ax, n_ax, n_ay);
+  A.item_volt = volt * bp_scratch_volumes(p);
+  A.volt[0] = reinterpret_cast<float*>(workspace + items * bp_pairs_bytes(g));
+  A.volt[1] = n_ax > 0 ? A.volt[0] + volt : A.volt[0];
+  float* first = A.volt[0];
+  const float* second = n_ax > 0 && n_ay > 0 ? A.volt[1] : nullptr;
+  if (two > 0) {
+    A.sinoz = sinoz;
+    A.group_pairs = 2 * pairs;
+    launch_zlane_two(p, A, two, stream);
+  }
+  if (one > 0) {
+    A.sinoz = sinoz + 2 * two * pairs;
+    A.group_pairs = pairs;
+    A.volt[0] += 2 * two * A.item_volt;
+    A.volt[1] += 2 * two * A.item_volt;
+    launch_zlane_passes(p, A, one, stream);
+  }
+  launch_zlane_out(g, additive ? 1 : 0, first, second, A.item_volt, A.zs, vol, nullptr, items, stream);
+  return int(cudaGetLastError());
 }
 
 }  // namespace tsgb

@@ -234,33 +234,35 @@ __device__ __forceinline__ f32x2 add2_rd(f32x2 a, f32x2 b) {
 }
 
 // Window accumulation: a column between voxels f0 and f0 + 1 of the window
-// (f0 in -1 .. kX - 1) adds wl V(z) to voxel f0 and wr V(z) to voxel f0 + 1,
-// with V(z) of the lane's voxels z0 + 32 j in pairs: profile(jj) holds those of
-// j = 2 jj and 2 jj + 1. The uniform branch on f0 sits outside the z loop, so
-// each profile pair goes straight into the two accumulators it feeds.
-template <int kX, int kPairs, int kM, typename F>
-__device__ __forceinline__ void window_apply(f32x2 (&acc)[kX][kPairs], const F& profile, f32x2 wl2,
-                                             f32x2 wr2) {
+// (f0 in -1 .. kX - 1) adds wl V(z) to voxel f0 and wr V(z) to voxel f0 + 1, for each of
+// the kItems stacked items the warp works on, with V(z) of the lane's voxels along z in
+// pairs: profile(item, jj). The uniform branch on f0 sits outside the z loop, so each
+// profile pair goes straight into the two accumulators it feeds.
+template <int kItems, int kX, int kPairs, int kM, typename F>
+__device__ __forceinline__ void window_apply(f32x2 (&acc)[kItems][kX][kPairs], const F& profile,
+                                             f32x2 wl2, f32x2 wr2) {
 #pragma unroll
-  for (int jj = 0; jj < kPairs; ++jj) {
-    const f32x2 V = profile(jj);
-    if constexpr (kM >= 0) acc[kM][jj] = fma2(wl2, V, acc[kM][jj]);
-    if constexpr (kM + 1 < kX) acc[kM + 1][jj] = fma2(wr2, V, acc[kM + 1][jj]);
-  }
+  for (int i = 0; i < kItems; ++i)
+#pragma unroll
+    for (int jj = 0; jj < kPairs; ++jj) {
+      const f32x2 V = profile(i, jj);
+      if constexpr (kM >= 0) acc[i][kM][jj] = fma2(wl2, V, acc[i][kM][jj]);
+      if constexpr (kM + 1 < kX) acc[i][kM + 1][jj] = fma2(wr2, V, acc[i][kM + 1][jj]);
+    }
 }
 
 // (kLo <= f0 < kHi: halves the candidates at each branch)
-template <int kX, int kPairs, int kLo, int kHi, typename F>
-__device__ __forceinline__ void window_dispatch(f32x2 (&acc)[kX][kPairs], int f0, const F& profile,
-                                                f32x2 wl2, f32x2 wr2) {
+template <int kLo, int kHi, int kItems, int kX, int kPairs, typename F>
+__device__ __forceinline__ void window_dispatch(f32x2 (&acc)[kItems][kX][kPairs], int f0,
+                                                const F& profile, f32x2 wl2, f32x2 wr2) {
   if constexpr (kHi - kLo == 1) {
-    window_apply<kX, kPairs, kLo>(acc, profile, wl2, wr2);
+    window_apply<kItems, kX, kPairs, kLo>(acc, profile, wl2, wr2);
   } else {
     constexpr int kMid = kLo + (kHi - kLo) / 2;
     if (f0 < kMid)
-      window_dispatch<kX, kPairs, kLo, kMid>(acc, f0, profile, wl2, wr2);
+      window_dispatch<kLo, kMid>(acc, f0, profile, wl2, wr2);
     else
-      window_dispatch<kX, kPairs, kMid, kHi>(acc, f0, profile, wl2, wr2);
+      window_dispatch<kMid, kHi>(acc, f0, profile, wl2, wr2);
   }
 }
 

@@ -370,11 +370,11 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
     const int z = z0 + r * 32 * kV;
     zoff[r] = (z < zs ? z : 0) * unsigned(sizeof(float));
   }
-  f32x2 acc[kX][kPairs];
+  f32x2 acc[1][kX][kPairs];
 #pragma unroll
   for (int m = 0; m < kX; ++m)
 #pragma unroll
-    for (int j = 0; j < kPairs; ++j) acc[m][j] = 0ull;
+    for (int j = 0; j < kPairs; ++j) acc[0][m][j] = 0ull;
   // (slots not filled yet stand for column 0)
   for (int k = lane; k < 34; k += 32) s_column[w][k] = make_int2(0, 0);
   __syncwarp();
@@ -391,8 +391,8 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
     }
   };
   const auto finish = [&](const f32x2(&V)[kPairs], int2 c, float4 e) {
-    const auto profile = [&](int j) { return V[j]; };
-    window_dispatch<kX, kPairs, -1, kX>(acc, c.x, profile, pack2(e.x, e.y), pack2(e.z, e.w));
+    const auto profile = [&](int, int j) { return V[j]; };
+    window_dispatch<-1, kX>(acc, c.x, profile, pack2(e.x, e.y), pack2(e.z, e.w));
   };
   for (int n0 = n_begin; n0 < n_end; n0 += 32) {
     const ColumnRanges cr =
@@ -453,14 +453,14 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
       if (w / kPlanes == split) {
 #pragma unroll
         for (int i = 0; i < kX * kPairs; ++i)
-          s_sum[w % kPlanes][i][lane] = acc[i / kPairs][i % kPairs];
+          s_sum[w % kPlanes][i][lane] = acc[0][i / kPairs][i % kPairs];
       }
       __syncthreads();
       if (w / kPlanes == 0) {
 #pragma unroll
         for (int i = 0; i < kX * kPairs; ++i)
-          acc[i / kPairs][i % kPairs] =
-              add2(acc[i / kPairs][i % kPairs], s_sum[w % kPlanes][i][lane]);
+          acc[0][i / kPairs][i % kPairs] =
+              add2(acc[0][i / kPairs][i % kPairs], s_sum[w % kPlanes][i][lane]);
       }
       __syncthreads();
     }
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
       if (z0 + r * 32 * kV >= zs) break;
       f32x2 x[kP];
 #pragma unroll
-      for (int i = 0; i < kP; ++i) x[i] = acc[m][r * kP + i];
+      for (int i = 0; i < kP; ++i) x[i] = acc[0][m][r * kP + i];
       store_pairs<kV>(out + r * 32 * kV, x);
     }
   }

@@ -58,9 +58,13 @@ __device__ __forceinline__ float2 copy_elem<float2>(float a, float b) {
   return make_float2(a, b);
 }
 
+// (blockIdx.y counts stacked volumes, their copies item_elems apart.)
 template <typename E>
 __global__ void fp_layout_kernel(const float* __restrict__ vol, E* __restrict__ out,
-                                 LayoutDev L, long long s_d, long long s_a, long long s_b) {
+                                 LayoutDev L, long long s_d, long long s_a, long long s_b,
+                                 long long item_elems) {
+  vol += (size_t)blockIdx.y * L.n_d * L.n_a * L.n_b;
+  out += blockIdx.y * item_elems;
   const long long n_ap = L.n_a + 2 * kPad;
   const long long n_bp = L.n_b + 2 * kPad;
   const long long total = (long long)L.n_d * n_ap * n_bp;
@@ -82,16 +86,20 @@ __global__ void fp_layout_kernel(const float* __restrict__ vol, E* __restrict__ 
 // of the remaining copy axis per blockIdx.z step, and writes 32 elements
 // along b (the 33rd b value is the last pair's second half). Reads run along x and
 // writes along b, both coalesced. Coordinates are those of the padded copy.
+// blockIdx.x counts the f tiles of the stacked volumes.
 template <typename E>
 __global__ void __launch_bounds__(256)
     fp_layout_transpose_kernel(const float* __restrict__ vol, E* __restrict__ out,
                                LayoutDev L, long long s_d, long long s_a, long long s_b,
-                               int f_is_d) {
+                               int f_is_d, long long item_elems) {
   __shared__ float tile[33][33];  // [b][f]
   const int n_ap = L.n_a + 2 * kPad, n_bp = L.n_b + 2 * kPad;
   const int f_ext = f_is_d ? L.n_d : n_ap;
   const int t_ext = f_is_d ? n_ap : L.n_d;
-  const int f0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+  const int f_tiles = (f_ext + 31) / 32, item = blockIdx.x / f_tiles;
+  const int f0 = (blockIdx.x - item * f_tiles) * 32, b0 = blockIdx.y * 32;
+  vol += (size_t)item * L.n_d * L.n_a * L.n_b;
+  out += item * item_elems;
   for (int t = blockIdx.z; t < t_ext; t += gridDim.z) {
     for (int r = threadIdx.y; r < 33; r += 8) {
       const int f = f0 + threadIdx.x, bp = b0 + r;
@@ -394,34 +402,42 @@ __global__ void __launch_bounds__(kFpRows* kFpCols, 4)
 
 namespace {
 
-// Volume copies and ray kernels with copy elements of type E (offsets and
-// strides count elements, so both types use the same plan).
+// The volume copies of `items` stacked volumes, with elements of type E (offsets and
+// strides count elements, so both types use the same plan), item_elems apart.
 template <typename E>
-void launch_fp_elems(const tsgb_projector* p, const float* vol, float* sino, bool additive,
-                     E* copies, cudaStream_t stream, const FpSirt* sirt, int angle_begin,
-                     int angle_end, bool copies_ready) {
+void launch_copies(const tsgb_projector* p, const float* vol, E* copies, int items,
+                   long long item_elems, cudaStream_t stream) {
   const DeviceGeometry& g = p->g;
   const LayoutTable lt = make_layout_table(p);
   const long long vstride[3] = {(long long)g.ny * g.nx, (long long)g.nx, 1};
-  for (int i = 0; i < lt.count && !copies_ready; ++i) {
+  for (int i = 0; i < lt.count; ++i) {
     const Layout& L = p->layouts[i];
     if (L.b == 2) {  // b is x: a plain copy reads and writes along x
       const long long total = L.n_d * (L.n_a + 2 * kPad) * (L.n_b + 2 * kPad);
       const int threads = 256;
       const long long blocks = (total + threads - 1) / threads;
-      const int grid = int(blocks < 152LL * 64 ? blocks : 152LL * 64);
+      const dim3 grid(unsigned(blocks < 152LL * 64 ? blocks : 152LL * 64), unsigned(items));
       fp_layout_kernel<E><<<grid, threads, 0, stream>>>(vol, copies, lt.l[i], vstride[L.d],
-                                                       vstride[L.a], vstride[L.b]);
+                                                       vstride[L.a], vstride[L.b], item_elems);
     } else {
       const int f_is_d = L.d == 2 ? 1 : 0;  // which copy axis is the volume's x
       const long long f_ext = f_is_d ? L.n_d : L.n_a + 2 * kPad;
       const long long t_ext = f_is_d ? L.n_a + 2 * kPad : L.n_d;
-      const dim3 grid(unsigned((f_ext + 31) / 32), unsigned((L.n_b + 2 * kPad + 31) / 32),
+      const dim3 grid(unsigned((f_ext + 31) / 32 * items), unsigned((L.n_b + 2 * kPad + 31) / 32),
                       unsigned(t_ext < 65535 ? t_ext : 65535));
       fp_layout_transpose_kernel<E><<<grid, dim3(32, 8), 0, stream>>>(
-          vol, copies, lt.l[i], vstride[L.d], vstride[L.a], vstride[L.b], f_is_d);
+          vol, copies, lt.l[i], vstride[L.d], vstride[L.a], vstride[L.b], f_is_d, item_elems);
     }
   }
+}
+
+// Volume copies and ray kernels with copy elements of type E.
+template <typename E>
+void launch_fp_elems(const tsgb_projector* p, const float* vol, float* sino, bool additive,
+                     E* copies, cudaStream_t stream, const FpSirt* sirt, int angle_begin,
+                     int angle_end, bool copies_ready) {
+  const DeviceGeometry& g = p->g;
+  if (!copies_ready) launch_copies(p, vol, copies, 1, 0, stream);
   const long long per_pair = (long long)((g.rows + kFpRows - 1) / kFpRows) *
                              ((g.cols + kFpCols - 1) / kFpCols);
   const long long chunk = fp_angle_chunk(g);
@@ -441,14 +457,13 @@ void launch_fp_elems(const tsgb_projector* p, const float* vol, float* sino, boo
 
 }  // namespace
 
-int launch_fp_copies(const tsgb_projector* p, const float* vol, float* workspace, void* stream_) {
+int launch_fp_copies(const tsgb_projector* p, const float* vol, float* workspace, void* stream_,
+                     int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  // the copies only (no angles): launch_fp_elems with an empty angle range
   if (p->tuning.fp_pair_layout)
-    launch_fp_elems(p, vol, nullptr, false, reinterpret_cast<float2*>(workspace), stream, nullptr,
-                    0, 0, false);
+    launch_copies(p, vol, reinterpret_cast<float2*>(workspace), items, item_bytes / 8, stream);
   else
-    launch_fp_elems(p, vol, nullptr, false, workspace, stream, nullptr, 0, 0, false);
+    launch_copies(p, vol, workspace, items, item_bytes / 4, stream);
   return int(cudaGetLastError());
 }
 
@@ -490,10 +505,11 @@ int launch_fp_batch(const tsgb_projector* p, const float* vol, float* sino, int6
       continue;
     }
     FpMulti fm{};
+    const int copied = launch_fp_copies(p, vol + i0 * vol_elems, reinterpret_cast<float*>(workspace),
+                                        stream, m, item_bytes);
+    if (copied != 0) return copied;
     for (int k = 0; k < m; ++k) {
       float* ws = reinterpret_cast<float*>(workspace + k * item_bytes);
-      const int rc = launch_fp_copies(p, vol + (i0 + k) * vol_elems, ws, stream);
-      if (rc != 0) return rc;
       FpMultiJob& J = fm.job[k];
       J.params = p->d_params;
       J.columns = p->d_columns;

@@ -281,8 +281,10 @@ struct BpMulti {
 // kernel arguments are limited to 32764 bytes
 static_assert(sizeof(FpMulti) <= 32764 && sizeof(BpMulti) <= 32764, "multi-job tables too large");
 
-// The padded volume copies of a forward projection, no rays (fp.cu).
-int launch_fp_copies(const tsgb_projector* p, const float* vol, float* workspace, void* stream);
+// The padded volume copies of a forward projection, no rays (fp.cu); of `items`
+// stacked volumes, their workspaces item_bytes apart.
+int launch_fp_copies(const tsgb_projector* p, const float* vol, float* workspace, void* stream,
+                     int items = 1, int64_t item_bytes = 0);
 // Whether a job's SIRT forward projection fits a multi-job launch (one angle
 // chunk), its block count, and the multi-job launch itself (fp.cu).
 bool fp_multi_eligible(const tsgb_projector* p);
@@ -340,12 +342,15 @@ int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz,
 // Both z-lane passes over the separable angle lists (offsets into
 // p->d_sep_angles) in one launch into the [y][x][z] scratch volumes at volt
 // (bp_scratch_bytes), then vol (=, +=, SIRT) from their sum (out_mode 0 / 1 / 2;
-// C for SIRT). items > 1: stacked items, item k's sinoz and volt k * item_bytes
-// further on and its vol k volumes (no SIRT). False if there are no such angles.
+// C for SIRT). False if there are no such angles.
 bool launch_bp_zlane_separable(const tsgb_projector* p, int off_x, int n_ax, int off_y, int n_ay,
                                const float* sinoz, float* volt, float* vol, int out_mode,
-                               const float* C, void* stream, int items = 1,
-                               int64_t item_bytes = 0);
+                               const float* C, void* stream);
+// The whole backprojection of `items` stacked sinograms (all angles separable) in
+// shared launches: weights, passes (two items per warp where they fit) and output.
+// Workspace: items * (bp_pairs_bytes + bp_scratch_bytes).
+int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino, int items,
+                          bool additive, char* workspace, void* stream);
 
 // [y][x][z] scratch volumes (rows of zs floats along z) to the caller's volume:
 // vol (=, +=, SIRT: out_mode 0 / 1 / 2) volt0 + volt1 (volt1 may be null) for
