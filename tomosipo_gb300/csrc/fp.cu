@@ -28,6 +28,14 @@ namespace {
 
 constexpr int kFpRows = kFpTileRows;  // threads along detector rows (one warp)
 constexpr int kFpCols = kFpTileCols;  // warps along detector columns
+// Pairs of adjacent angles per block, one warp each: two for single-voxel copies
+// (large volumes: 512^3 / 1024 angles 121.6 ms against 123.4), one for pairs along b
+// (256^3 / 360: 5.35 ms against 5.39). Blocks of 8 columns took 5.42 and 123.5 ms, 16
+// 5.64 and 127.6: a block's warps finish together, 2 columns 5.47 and 141.
+template <typename E>
+constexpr int kFpBlockPairs = sizeof(E) == sizeof(float) ? 2 : 1;
+template <typename E>
+constexpr int kFpThreads = kFpRows * kFpCols * kFpBlockPairs<E>;
 
 // Rays making more than ~89 degrees with the dominant axis are not sampled
 // (both here and, through the weighted sinogram, in the transpose).
@@ -344,9 +352,9 @@ __device__ __forceinline__ void fp_ray_tile(const AngleParams* __restrict__ para
   int rb, cb, pr;
   fp_schedule_tile(sched, block, rb, cb, pr);
   const int iv = rb * kFpRows + threadIdx.x;
-  const int iu = cb * kFpCols + threadIdx.y;
-  const int theta = angle0 + 2 * pr;
-  if (iu >= g.cols || iv >= g.rows) return;
+  const int iu = cb * kFpCols + int(threadIdx.y) % kFpCols;
+  const int theta = angle0 + 2 * (pr * kFpBlockPairs<E> + int(threadIdx.y) / kFpCols);
+  if (iu >= g.cols || iv >= g.rows || theta >= angle_end) return;
   const int slot = threadIdx.y * kFpRows + threadIdx.x;
   // the launch covers angles angle0 .. angle_end - 1: an odd count leaves the
   // last thread one angle
@@ -377,11 +385,11 @@ __device__ __forceinline__ void fp_ray_tile(const AngleParams* __restrict__ para
 }
 
 template <bool kSirt, typename E>
-__global__ void __launch_bounds__(kFpRows* kFpCols, 4)
+__global__ void __launch_bounds__(kFpThreads<E>, 1024 / kFpThreads<E>)
     fp_ray_kernel(const AngleParams* __restrict__ params, const ColumnEntry* __restrict__ columns,
                   const E* __restrict__ ws, float* __restrict__ sino, DeviceGeometry g,
                   FpSchedule sched, int angle0, int angle_end, int additive, FpSirt sirt) {
-  __shared__ volatile long long out_slot[kFpRows * kFpCols];
+  __shared__ volatile long long out_slot[kFpThreads<E>];
   fp_ray_tile<kSirt, E>(params, columns, ws, sino, g, sched, angle0, angle_end, additive, sirt,
                         blockIdx.x, out_slot);
 }
@@ -389,9 +397,9 @@ __global__ void __launch_bounds__(kFpRows* kFpCols, 4)
 // SIRT forward projections of many jobs in one launch: block b runs tile
 // b - start[j] of job j, exactly as fp_ray_kernel would for that job alone.
 template <bool kSirt, typename E>
-__global__ void __launch_bounds__(kFpRows* kFpCols, 4)
+__global__ void __launch_bounds__(kFpThreads<E>, 1024 / kFpThreads<E>)
     fp_ray_multi_kernel(const __grid_constant__ FpMulti m) {
-  __shared__ volatile long long out_slot[kFpRows * kFpCols];
+  __shared__ volatile long long out_slot[kFpThreads<E>];
   const int j = multi_job_of(m.start, m.n, blockIdx.x);
   const FpMultiJob& J = m.job[j];
   fp_ray_tile<kSirt, E>(J.params, J.columns, static_cast<const E*>(J.ws), J.sino, J.g, J.sched,
@@ -440,16 +448,17 @@ void launch_fp_elems(const tsgb_projector* p, const float* vol, float* sino, boo
   if (!copies_ready) launch_copies(p, vol, copies, 1, 0, stream);
   const long long per_pair = (long long)((g.rows + kFpRows - 1) / kFpRows) *
                              ((g.cols + kFpCols - 1) / kFpCols);
+  const dim3 block(kFpRows, kFpCols * kFpBlockPairs<E>);
   const long long chunk = fp_angle_chunk(g);
   for (long long a0 = angle_begin; a0 < angle_end; a0 += chunk) {
     const int n = int(angle_end - a0 < chunk ? angle_end - a0 : chunk);
     const FpSchedule s = fp_schedule(p, (n + 1) / 2);
     const long long blocks = per_pair * s.pairs;
     if (sirt)
-      fp_ray_kernel<true, E><<<unsigned(blocks), dim3(kFpRows, kFpCols), 0, stream>>>(
+      fp_ray_kernel<true, E><<<unsigned(blocks), block, 0, stream>>>(
           p->d_params, p->d_columns, copies, sino, g, s, int(a0), int(a0) + n, 0, *sirt);
     else
-      fp_ray_kernel<false, E><<<unsigned(blocks), dim3(kFpRows, kFpCols), 0, stream>>>(
+      fp_ray_kernel<false, E><<<unsigned(blocks), block, 0, stream>>>(
           p->d_params, p->d_columns, copies, sino, g, s, int(a0), int(a0) + n, additive ? 1 : 0,
           FpSirt{});
   }
@@ -478,7 +487,7 @@ int launch_fp_multi(const FpMulti& m, bool pair_layout, void* stream_, bool sirt
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const long long blocks = m.start[m.n];
   if (blocks <= 0) return int(cudaGetLastError());
-  const dim3 block(kFpRows, kFpCols);
+  const dim3 block(kFpRows, kFpCols * (pair_layout ? kFpBlockPairs<float2> : kFpBlockPairs<float>));
   if (sirt && pair_layout)
     fp_ray_multi_kernel<true, float2><<<unsigned(blocks), block, 0, stream>>>(m);
   else if (sirt)
@@ -560,13 +569,16 @@ long long fp_angle_chunk(const DeviceGeometry& g) {
 }
 
 FpSchedule fp_schedule(const tsgb_projector* p, int pairs) {
+  // in blocks: kFpCols columns (the tuning counts 8) and one or two angle pairs
+  const int block_pairs = p->tuning.fp_pair_layout ? kFpBlockPairs<float2> : kFpBlockPairs<float>;
   FpSchedule s;
   s.row_blocks = (p->g.rows + kFpRows - 1) / kFpRows;
   s.col_blocks = (p->g.cols + kFpCols - 1) / kFpCols;
-  s.pairs = pairs;
+  s.pairs = (pairs + block_pairs - 1) / block_pairs;
   s.patch_rows = std::min(std::max(p->tuning.fp_patch_rows, 1), s.row_blocks);
-  s.patch_cols = std::min(std::max(p->tuning.fp_patch_cols, 1), s.col_blocks);
-  s.group_pairs = std::min(std::max(p->tuning.fp_group_pairs, 1), std::max(pairs, 1));
+  s.patch_cols = int(std::min<int64_t>(int64_t(std::max(p->tuning.fp_patch_cols, 1)) * 8 / kFpCols,
+                                       s.col_blocks));
+  s.group_pairs = std::min(std::max(p->tuning.fp_group_pairs / block_pairs, 1), std::max(s.pairs, 1));
   return s;
 }
 
@@ -584,7 +596,7 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   // 512^3 cone scan with a 512 x 768 detector and 1024 angles, and within
   // 3 % of the fastest at 256^3 / 360 angles).
   t.fp_patch_rows = 256 / kFpRows;
-  t.fp_patch_cols = 32 / kFpCols;
+  t.fp_patch_cols = 32 / 8;
   t.fp_group_pairs = 32;
   // Matched backprojection: the z-lane kernel (ms per call against the
   // voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360 4.56 / 6.52,

@@ -117,7 +117,7 @@ struct DeviceGeometry {
 };
 
 // Forward-projection tile order over one chunk of angles (tsgb_tuning):
-// groups of group_pairs angle pairs, each run over the detector patch by
+// groups of group_pairs angle pairs (or, like `pairs`, of blocks of two pairs), each run over the detector patch by
 // patch (patch_rows x patch_cols tiles), row tiles fastest inside a patch.
 struct FpSchedule {
   int row_blocks, col_blocks, pairs;  // tiles along rows and columns; angle pairs
@@ -411,6 +411,6 @@ int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, b
 int launch_bp_sirt(const tsgb_projector* p, float* vol, const float* C, const float* res,
                    float* scratch, void* stream);
 constexpr int kBpRunZ = 16;  // voxels along z per matched-backprojection thread
-constexpr int kBpTileX = 32, kBpTileY = 4, kFpTileRows = 32, kFpTileCols = 8;
+constexpr int kBpTileX = 32, kBpTileY = 4, kFpTileRows = 32, kFpTileCols = 4;
 
 }  // namespace tsgb
