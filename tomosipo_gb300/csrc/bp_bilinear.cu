@@ -41,15 +41,21 @@ __global__ void __launch_bounds__(256)
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   for (int theta = blockIdx.z; theta < g.nangles; theta += gridDim.z) {
     const int iu = c0 + int(threadIdx.x) - kColPad;
-    for (int k = threadIdx.y; k < 33; k += 8) {
-      const int iv = r0 + k - kRowPad;
-      const bool in = iu >= 0 && iu < g.cols && iv >= 0 && iv < g.rows;
-      s[k][threadIdx.x] = in ? __ldg(sino + ((size_t)iv * g.nangles + theta) * g.cols + iu) : 0.0f;
+    float v[5];  // rows threadIdx.y + 8 q; the 33rd is the first warp's
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      const int k = int(threadIdx.y) + 8 * q, iv = r0 + k - kRowPad;
+      const bool in = iu >= 0 && iu < g.cols && iv >= 0 && iv < g.rows && k < 33;
+      v[q] = in ? __ldg(sino + ((size_t)iv * g.nangles + theta) * g.cols + iu) : 0.0f;
     }
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+      if (q < 4 || threadIdx.y == 0) s[threadIdx.y + 8 * q][threadIdx.x] = v[q];
     __syncthreads();
     const int r = r0 + threadIdx.x;
-    for (int c = threadIdx.y; c < 32 && c0 + c < cp; c += 8)
-      if (r < rp)
+#pragma unroll
+    for (int c = threadIdx.y, q = 0; q < 4; ++q, c += 8)
+      if (r < rp && c0 + c < cp)
         out[((size_t)theta * cp + c0 + c) * rp + r] =
             make_float2(s[threadIdx.x][c], s[threadIdx.x + 1][c]);
     __syncthreads();

@@ -51,18 +51,14 @@ namespace {
 
 constexpr float kMaxSlopeZ = 64.0f;  // must match fp.cu
 
-// W * y of pixel (iv, iu) at angle theta, 0 off the detector and for rays the
-// forward projector does not sample.
-__device__ __forceinline__ float weighted_pixel_z(const AngleParams& ap, const ColumnEntry& ce,
-                                                  const float* __restrict__ sino,
-                                                  const DeviceGeometry& g, int iv, int iu,
-                                                  int theta) {
-  if (iv < 0 || iv >= g.rows || iu >= g.cols) return 0.0f;
+// Plane step W of pixel (iv, iu), 0 for rays the forward projector does not sample.
+__device__ __forceinline__ float pixel_step_z(const AngleParams& ap, const ColumnEntry& ce,
+                                              const DeviceGeometry& g, int iv, int iu) {
   const float vt = float(iv - g.ov);
   const Ray r = ap.separable ? ray_column(ce, vt) : ray_general(ap, float(iu - g.ou), vt);
-  float w = 0.0f;
-  if (finite_ray(r) && fabsf(r.ma) <= kMaxSlopeZ && fabsf(r.mb) <= kMaxSlopeZ) w = ray_step(ap, r);
-  return w * __ldg(sino + ((size_t)iv * g.nangles + theta) * g.cols + iu);
+  const bool sampled =
+      finite_ray(r) && fabsf(r.ma) <= kMaxSlopeZ && fabsf(r.mb) <= kMaxSlopeZ;
+  return sampled ? ray_step(ap, r) : 0.0f;
 }
 
 // Column-major row-pair weighted sinogram. A block of 32 x 8 threads covers
@@ -88,17 +84,33 @@ __global__ void __launch_bounds__(256)
     const AngleParams& ap = params[theta];
     {
       const int iu = iu0 + threadIdx.x;
+      const float* y = sino + (group * kItems) * item + (size_t)theta * g.cols + iu;
+      float v[5][kItems];  // rows threadIdx.y + 8 q; the 33rd is the first warp's
+#pragma unroll
+      for (int q = 0; q < 5; ++q) {
+        const int k = int(threadIdx.y) + 8 * q, iv = r0 + k - kRowPad;
+        const bool in = iu < g.cols && iv >= 0 && iv < g.rows && k < 33;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+          v[q][i] = in ? __ldg(y + i * item + (size_t)iv * g.nangles * g.cols) : 0.0f;
+      }
       ColumnEntry ce{};
       if (ap.separable && iu < g.cols) ce = columns[(size_t)theta * g.cols + iu];
 #pragma unroll
-      for (int i = 0; i < kItems; ++i)
-        for (int k = threadIdx.y; k < 33; k += 8)
-          s[i][k][threadIdx.x] = weighted_pixel_z(ap, ce, sino + (group * kItems + i) * item, g,
-                                                  r0 + k - kRowPad, iu, theta);
+      for (int q = 0; q < 5; ++q) {
+        const int k = int(threadIdx.y) + 8 * q;
+        if (k >= 33) break;
+        const float W = pixel_step_z(ap, ce, g, r0 + k - kRowPad, iu);
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) s[i][k][threadIdx.x] = W * v[q][i];
+      }
     }
     __syncthreads();
     const int r = r0 + threadIdx.x;
-    for (int c = threadIdx.y; c < 32 && iu0 + c < g.cols && r < RP; c += 8) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = int(threadIdx.y) + 8 * q;
+      if (iu0 + c >= g.cols || r >= RP) break;
       const size_t at = ((size_t)n * g.cols + iu0 + c) * RP + r;
       float2 v[kItems];
 #pragma unroll
@@ -492,26 +504,38 @@ __global__ void __launch_bounds__(256)
   if (volt1) volt1 += item * item_volt;
   vol += (size_t)item * g.nz * g.ny * g.nx;
   for (int y = blockIdx.z; y < g.ny; y += gridDim.z) {
-    for (int k = threadIdx.y; k < 32; k += 8) {
-      const int x = x0 + k, z = z0 + threadIdx.x;
-      if (x < g.nx && z < g.nz) {
-        const size_t i = ((size_t)y * g.nx + x) * zs + z;
-        tile[k][threadIdx.x] = volt1 ? __fadd_rn(volt0[i], volt1[i]) : volt0[i];
+    float v[4], v1[4], old[4], c[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int x = x0 + int(threadIdx.y) + 8 * q, z = z0 + threadIdx.x;
+      const size_t i = ((size_t)y * g.nx + x) * zs + z;
+      const bool in = x < g.nx && z < g.nz;
+      v[q] = in ? volt0[i] : 0.0f;
+      v1[q] = in && volt1 ? volt1[i] : 0.0f;
+    }
+    if (kOut != kOutSet) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int z = z0 + int(threadIdx.y) + 8 * q, x = x0 + threadIdx.x;
+        const size_t idx = ((size_t)z * g.ny + y) * g.nx + x;
+        const bool in = x < g.nx && z < g.nz;
+        old[q] = in ? vol[idx] : 0.0f;
+        c[q] = kOut == kOutSirt && in ? __ldg(C + idx) : 0.0f;
       }
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      tile[threadIdx.y + 8 * q][threadIdx.x] = volt1 ? __fadd_rn(v[q], v1[q]) : v[q];
     __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
-      const int z = z0 + k, x = x0 + threadIdx.x;
-      if (x < g.nx && z < g.nz) {
-        const size_t idx = ((size_t)z * g.ny + y) * g.nx + x;
-        const float s = tile[threadIdx.x][k];
-        if (kOut == kOutSet)
-          vol[idx] = s;
-        else if (kOut == kOutAdd)
-          vol[idx] = __fadd_rn(vol[idx], s);
-        else
-          vol[idx] = __fadd_rn(vol[idx], __fmul_rn(s, __ldg(C + idx)));
-      }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int z = z0 + int(threadIdx.y) + 8 * q, x = x0 + threadIdx.x;
+      if (x >= g.nx || z >= g.nz) break;
+      const float s = tile[threadIdx.x][threadIdx.y + 8 * q];
+      vol[((size_t)z * g.ny + y) * g.nx + x] =
+          kOut == kOutSet   ? s
+          : kOut == kOutAdd ? __fadd_rn(old[q], s)
+                            : __fadd_rn(old[q], __fmul_rn(s, c[q]));
     }
     __syncthreads();
   }

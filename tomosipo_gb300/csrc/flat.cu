@@ -83,13 +83,18 @@ __global__ void __launch_bounds__(256)
   copy += item * item_copy;
   for (int yp = blockIdx.z; yp < nyp; yp += gridDim.z) {
     const int y = yp - kPad, x = x0 + int(threadIdx.x) - kPad;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-      const int z = z0 + k;
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int z = z0 + int(threadIdx.y) + 8 * q;
       const bool in = z < g.nz && y >= 0 && y < g.ny && x >= 0 && x < g.nx;
-      tile[k][threadIdx.x] = in ? __ldg(vol + ((size_t)z * g.ny + y) * g.nx + x) : 0.0f;
+      v[q] = in ? __ldg(vol + ((size_t)z * g.ny + y) * g.nx + x) : 0.0f;
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) tile[threadIdx.y + 8 * q][threadIdx.x] = v[q];
     __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
+#pragma unroll
+    for (int k = threadIdx.y, q = 0; q < 4; ++q, k += 8) {
       const int xp = x0 + k, z = z0 + threadIdx.x;
       if (xp < nxp && z < zs) copy[((size_t)yp * nxp + xp) * zs + z] = tile[threadIdx.x][k];
     }
@@ -219,18 +224,20 @@ __global__ void __launch_bounds__(256)
     const int iv = v0 + int(threadIdx.x);
     const float q = fmaf(float(iv - g.ov), R, P);
     const bool in = iv < g.rows && q > float(-1 - g.oz) && q < float(g.nz - g.oz);
-    const float fl = floorf(in ? q : 0.0f), f = q - fl;
+    const float fl = floorf(in ? q : 0.0f), f = in ? q - fl : 0.0f;
     const int j = int(fl) + g.oz;
     const float* s = sums + item * item_floats + (size_t)theta * g.cols * zs + j;
-    for (int c = threadIdx.y; c < 32 && u0 + c < g.cols; c += 8) {
-      float t = 0.0f;
-      if (in) {
-        const float* p = s + (size_t)(u0 + c) * zs;
-        const float a = j >= 0 ? __ldg(p) : 0.0f, d = j + 1 < g.nz ? __ldg(p + 1) : 0.0f;
-        t = fmaf(f, d - a, a);
-      }
-      tile[threadIdx.x][c] = t;
+    float a[4], d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = u0 + int(threadIdx.y) + 8 * q;
+      const float* p = s + (size_t)c * zs;
+      a[q] = in && j >= 0 && c < g.cols ? __ldg(p) : 0.0f;
+      d[q] = in && j + 1 < g.nz && c < g.cols ? __ldg(p + 1) : 0.0f;
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      tile[threadIdx.x][threadIdx.y + 8 * q] = fmaf(f, d[q] - a[q], a[q]);
     __syncthreads();
     const int iu = u0 + int(threadIdx.x);
     if (iu < g.cols) {
@@ -238,7 +245,9 @@ __global__ void __launch_bounds__(256)
       r.Xa = r.Xb = r.mb = 0.0f;
       r.ma = columns[(size_t)theta * g.cols + iu].ma;
       const float W = ray_step(ap, r);
-      for (int k = threadIdx.y; k < 32 && v0 + k < g.rows; k += 8) {
+#pragma unroll
+      for (int k = threadIdx.y, q = 0; q < 4; ++q, k += 8) {
+        if (v0 + k >= g.rows) break;
         const long long idx = ((long long)(v0 + k) * g.nangles + theta) * g.cols + iu;
         const float total = __fmul_rn(tile[k][threadIdx.x], W);
         if (kMode == 2) {
@@ -286,19 +295,29 @@ __global__ void __launch_bounds__(256)
       r.ma = columns[(size_t)theta * g.cols + iu].ma;
       W = ray_step(ap, r);
     }
-    for (int k = threadIdx.y; k < 32; k += 8) {
-      const int z = z0 + k;
-      float V = 0.0f;
-      if (iu < g.cols && z < g.nz) {
+    if (aR >= 1.0f) {
+      float t[4], y0[4], y1[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int z = z0 + int(threadIdx.y) + 8 * q;
         const float C = Ph - float(z - g.oz);
-        if (aR >= 1.0f) {
-          const float v = floorf(clamp_coord(-(C + Pl) * inv));
-          const float t = fabsf(fmaf(v, R, C) + Pl);
-          const int iv = int(v) + g.ov;
-          const float y0 = iv >= 0 && iv < g.rows ? W * __ldg(y + iv * row) : 0.0f;
-          const float y1 = iv + 1 >= 0 && iv + 1 < g.rows ? W * __ldg(y + (iv + 1) * row) : 0.0f;
-          V = fmaf(__saturatef(1.0f - t), y0, __saturatef((1.0f - aR) + t) * y1);
-        } else {
+        const float v = floorf(clamp_coord(-(C + Pl) * inv));
+        t[q] = fabsf(fmaf(v, R, C) + Pl);
+        const int iv = int(v) + g.ov;
+        const bool in = iu < g.cols && z < g.nz;
+        y0[q] = in && iv >= 0 && iv < g.rows ? __ldg(y + iv * row) : 0.0f;
+        y1[q] = in && iv + 1 >= 0 && iv + 1 < g.rows ? __ldg(y + (iv + 1) * row) : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        tile[threadIdx.y + 8 * q][threadIdx.x] = fmaf(
+            __saturatef(1.0f - t[q]), W * y0[q], __saturatef((1.0f - aR) + t[q]) * (W * y1[q]));
+    } else {
+      for (int k = threadIdx.y; k < 32; k += 8) {
+        const int z = z0 + k;
+        float V = 0.0f;
+        if (iu < g.cols && z < g.nz) {
+          const float C = Ph - float(z - g.oz);
           const float B = C + Pl;
           const float v1 = (-1.0f - B) * inv, v2 = (1.0f - B) * inv;
           const int lo = max(0, (int)floorf(clamp_coord(fminf(v1, v2))) + g.ov);
@@ -306,13 +325,14 @@ __global__ void __launch_bounds__(256)
           for (int iv = lo; iv <= hi; ++iv)
             V = fmaf(tent(fmaf(float(iv - g.ov), R, C) + Pl), W * __ldg(y + iv * row), V);
         }
+        tile[k][threadIdx.x] = V;
       }
-      tile[k][threadIdx.x] = V;
     }
     __syncthreads();
     const int z = z0 + int(threadIdx.x);
-    for (int c = threadIdx.y; c < 32 && u0 + c < g.cols; c += 8)
-      if (z < zs)
+#pragma unroll
+    for (int c = threadIdx.y, q = 0; q < 4; ++q, c += 8)
+      if (z < zs && u0 + c < g.cols)
         out[item * item_floats + ((size_t)theta * g.cols + u0 + c) * zs + z] = tile[threadIdx.x][c];
     __syncthreads();
   }

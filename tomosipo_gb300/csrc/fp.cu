@@ -109,19 +109,24 @@ __global__ void __launch_bounds__(256)
   vol += (size_t)item * L.n_d * L.n_a * L.n_b;
   out += item * item_elems;
   for (int t = blockIdx.z; t < t_ext; t += gridDim.z) {
-    for (int r = threadIdx.y; r < 33; r += 8) {
-      const int f = f0 + threadIdx.x, bp = b0 + r;
-      const int k = f_is_d ? f : t, ip = f_is_d ? t : f;
-      const int i = ip - kPad, j = bp - kPad;
-      float v = 0.0f;
-      if (f < f_ext && i >= 0 && i < L.n_a && j >= 0 && j < L.n_b)
-        v = __ldg(vol + k * s_d + i * s_a + j * s_b);
-      tile[r][threadIdx.x] = v;
+    {
+      constexpr int kReads = sizeof(E) == sizeof(float) ? 4 : 5;
+      const int f = f0 + threadIdx.x, k = f_is_d ? f : t, i = (f_is_d ? t : f) - kPad;
+      const bool in = f < f_ext && i >= 0 && i < L.n_a;
+      float v[kReads];  // b values threadIdx.y + 8 q; the 33rd is the first warp's
+#pragma unroll
+      for (int q = 0; q < kReads; ++q) {
+        const int r = int(threadIdx.y) + 8 * q, j = b0 + r - kPad;
+        v[q] = in && j >= 0 && j < L.n_b && r < 33 ? __ldg(vol + k * s_d + i * s_a + j * s_b) : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < kReads; ++q)
+        if (q < 4 || threadIdx.y == 0) tile[threadIdx.y + 8 * q][threadIdx.x] = v[q];
     }
     __syncthreads();
 #pragma unroll
-    for (int r = threadIdx.y; r < 32; r += 8) {
-      const int f = f0 + r, bp = b0 + threadIdx.x;
+    for (int q = 0; q < 4; ++q) {
+      const int r = int(threadIdx.y) + 8 * q, f = f0 + r, bp = b0 + threadIdx.x;
       const int k = f_is_d ? f : t, ip = f_is_d ? t : f;
       if (f < f_ext && bp < n_bp)
         out[L.offset + ((long long)k * n_ap + ip) * n_bp + bp] =
