@@ -51,8 +51,9 @@ constexpr int kRunZBil = 8;         // voxels along z per thread (bilinear)
 // W * y of pixel (iv, iu) at angle theta (0 for rows outside the detector and
 // for rays the forward projector does not sample). ce is the pixel's column
 // entry (read only for separable angles).
+template <bool kSpread>
 __device__ __forceinline__ float weighted_pixel(const AngleParams& ap, const ColumnEntry& ce,
-                                                const float* __restrict__ sino,
+                                                const SinoSource& sino,
                                                 const DeviceGeometry& g, int iv, int iu,
                                                 int theta) {
   if (iv < 0 || iv >= g.rows) return 0.0f;
@@ -60,7 +61,7 @@ __device__ __forceinline__ float weighted_pixel(const AngleParams& ap, const Col
   const Ray r = ap.separable ? ray_column(ce, vt) : ray_general(ap, float(iu - g.ou), vt);
   float w = 0.0f;
   if (finite_ray(r) && fabsf(r.ma) <= kMaxSlope && fabsf(r.mb) <= kMaxSlope) w = ray_step(ap, r);
-  return w * __ldg(sino + ((size_t)iv * g.nangles + theta) * g.cols + iu);
+  return w * sino_value<kSpread>(sino, g, iv, iu, theta);
 }
 
 // Row-pair weighted sinogram: element (iv, theta, iu) holds (W y[iv], W y[iv+1])
@@ -73,9 +74,10 @@ __device__ __forceinline__ float weighted_pixel(const AngleParams& ap, const Col
 // (0, 0, 0); rows are nangles * cols elements apart.
 constexpr int kWeightRows = 8;
 
+template <bool kSpread>
 __global__ void __launch_bounds__(256)
     bp_weight_kernel(const AngleParams* __restrict__ params,
-                     const ColumnEntry* __restrict__ columns, const float* __restrict__ sino,
+                     const ColumnEntry* __restrict__ columns, SinoSource sino,
                      float2* __restrict__ out, DeviceGeometry g) {
   const int iu = blockIdx.x * 32 + threadIdx.x;
   const int r0 = (blockIdx.y * 8 + threadIdx.y) * kWeightRows - 1;
@@ -84,10 +86,10 @@ __global__ void __launch_bounds__(256)
   const AngleParams& ap = params[theta];
   ColumnEntry ce{};
   if (ap.separable) ce = columns[(size_t)theta * g.cols + iu];
-  float prev = weighted_pixel(ap, ce, sino, g, r0, iu, theta);
+  float prev = weighted_pixel<kSpread>(ap, ce, sino, g, r0, iu, theta);
   const int r1 = min(r0 + kWeightRows, g.rows);
   for (int iv = r0; iv < r1; ++iv) {
-    const float next = weighted_pixel(ap, ce, sino, g, iv + 1, iu, theta);
+    const float next = weighted_pixel<kSpread>(ap, ce, sino, g, iv + 1, iu, theta);
     out[((long long)iv * g.nangles + theta) * g.cols + iu] = make_float2(prev, next);
     prev = next;
   }
@@ -1263,7 +1265,7 @@ void launch_sep_pass(const tsgb_projector* p, bool a_is_x, const int* angles, in
 // Row-major row-pair weighted sinogram of angles [angle_begin, angle_end)
 // into `pairs` (bp_weight_kernel), and the padding rows it does not write
 // zeroed: -kRowPad .. -2 and rows .. rows + kRowPad - 1.
-void launch_bp_weight_rows(const tsgb_projector* p, const float* sino, float2* pairs,
+void launch_bp_weight_rows(const tsgb_projector* p, SinoSource sino, float2* pairs,
                            int angle_begin, int angle_end, cudaStream_t stream) {
   const DeviceGeometry& g = p->g;
   const size_t rs = (size_t)g.nangles * g.cols;  // elements between rows
@@ -1273,9 +1275,10 @@ void launch_bp_weight_rows(const tsgb_projector* p, const float* sino, float2* p
     const dim3 grid((g.cols + 31) / 32, (g.rows + 1 + 8 * kWeightRows - 1) / (8 * kWeightRows),
                     n);
     // offset the angle through the pointers: rows are strided by nangles*cols
-    bp_weight_kernel<<<grid, block, 0, stream>>>(p->d_params + a0, p->d_columns + (size_t)a0 * g.cols,
-                                                 sino + (size_t)a0 * g.cols,
-                                                 pairs + kRowPad * rs + (size_t)a0 * g.cols, g);
+    const SinoSource s{sino.y + (size_t)a0 * (g.cols / sino.d), sino.d, sino.scale, sino.inv_d, sino.shift};
+    (sino.d > 1 ? bp_weight_kernel<true> : bp_weight_kernel<false>)<<<grid, block, 0, stream>>>(
+        p->d_params + a0, p->d_columns + (size_t)a0 * g.cols, s,
+        pairs + kRowPad * rs + (size_t)a0 * g.cols, g);
   }
   cudaMemsetAsync(pairs, 0, (kRowPad - 1) * rs * sizeof(float2), stream);
   cudaMemsetAsync(pairs + (kRowPad + g.rows) * rs, 0, kRowPad * rs * sizeof(float2), stream);
@@ -1294,7 +1297,7 @@ void angle_sub_range(const std::vector<int>& host_list, int lo, int hi, int a0, 
 
 }  // namespace
 
-int launch_bp_matched(const tsgb_projector* p, float* vol, const float* sino, bool additive,
+int launch_bp_matched(const tsgb_projector* p, float* vol, SinoSource sino, bool additive,
                       float* workspace, void* stream_, int angle_begin, int angle_end) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const DeviceGeometry& g = p->g;
@@ -1354,7 +1357,7 @@ int launch_bp_sirt(const tsgb_projector* p, float* vol, const float* C, const fl
   const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - p->n_sep_ax;
   const DeviceGeometry& g = p->g;
   if (flat_bp(p))  // the residual is a plain sinogram of W y
-    return launch_flat_bp(p, vol, res, true, 2, C, scratch, stream, 0, g.nangles, 1, 0);
+    return launch_flat_bp(p, vol, {res}, true, 2, C, scratch, stream, 0, g.nangles, 1, 0);
   if (p->n_general_bp > 0) {
     // Angles outside the separable backprojector (tilted detectors): the whole
     // backprojection goes into a sum volume as launch_bp_matched computes it
@@ -1447,7 +1450,7 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
   for (int64_t i0 = 0; i0 < n; i0 += group) {
     const int m = int(std::min<int64_t>(group, n - i0));
     if (flat_bp(p)) {
-      const int rc = launch_flat_bp(p, vol + i0 * vol_elems, sino + i0 * sino_elems, false,
+      const int rc = launch_flat_bp(p, vol + i0 * vol_elems, {sino + i0 * sino_elems}, false,
                                     additive ? 1 : 0, nullptr, reinterpret_cast<float*>(workspace),
                                     stream, 0, g.nangles, m, item_bytes);
       if (rc != 0) return rc;
@@ -1460,7 +1463,7 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
       continue;
     }
     for (int k = 0; k < m; ++k)
-      launch_bp_weight_rows(p, sino + (i0 + k) * sino_elems,
+      launch_bp_weight_rows(p, {sino + (i0 + k) * sino_elems},
                             reinterpret_cast<float2*>(workspace + k * item_bytes), 0, g.nangles,
                             stream);
     // the pass along x sets (or adds), the pass along y adds onto it

@@ -51,11 +51,11 @@ namespace {
 
 constexpr float kMaxSlopeZ = 64.0f;  // must match fp.cu
 
-// Plane step W of pixel (iv, iu), 0 for rays the forward projector does not sample.
-__device__ __forceinline__ float pixel_step_z(const AngleParams& ap, const ColumnEntry& ce,
-                                              const DeviceGeometry& g, int iv, int iu) {
-  const float vt = float(iv - g.ov);
-  const Ray r = ap.separable ? ray_column(ce, vt) : ray_general(ap, float(iu - g.ou), vt);
+// Plane step W of pixel (iv, iu) of an angle without column entries, 0 for rays the
+// forward projector does not sample.
+__device__ __forceinline__ float pixel_step_z(const AngleParams& ap, const DeviceGeometry& g,
+                                              int iv, int iu) {
+  const Ray r = ray_general(ap, float(iu - g.ou), float(iv - g.ov));
   const bool sampled =
       finite_ray(r) && fabsf(r.ma) <= kMaxSlopeZ && fabsf(r.mb) <= kMaxSlopeZ;
   return sampled ? ray_step(ap, r) : 0.0f;
@@ -67,60 +67,86 @@ __device__ __forceinline__ float pixel_step_z(const AngleParams& ap, const Colum
 // writes the pairs along the rows (coalesced). Every padded pair is written,
 // so the buffer needs no clearing. `out` points at the angle range's first
 // column; blockIdx.z counts angles from `theta0`, over groups of kItems stacked
-// sinograms: with kItems = 2 an element holds both items' pairs.
-template <int kItems>
+// sinograms: with kItems = 2 an element holds both items' pairs. (angles * groups
+// fits 32 bits: an angle's tables take 256 bytes, and a batch's workspace is bounded.)
+template <int kItems, bool kSpread>
 __global__ void __launch_bounds__(256)
     bp_weight_z_kernel(const AngleParams* __restrict__ params,
-                       const ColumnEntry* __restrict__ columns, const float* __restrict__ sino,
+                       const ColumnEntry* __restrict__ columns, SinoSource sino,
                        float2* __restrict__ out, long long group_pairs, DeviceGeometry g,
                        int theta0, int n_angles, int groups) {
   __shared__ float s[kItems][33][33];  // [item][row][column]
   const int iu0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int RP = g.rows + 2 * kRowPad;
-  const size_t item = (size_t)g.rows * g.nangles * g.cols;
-  for (long long b = blockIdx.z; b < (long long)n_angles * groups; b += gridDim.z) {
-    const int group = int(b / n_angles), n = int(b - (long long)group * n_angles);
-    const int theta = theta0 + n;
+  const int iu = iu0 + threadIdx.x;
+  // the source's columns and elements between its rows (kSpread: a coarser detector)
+  const int ys = kSpread ? int(source_pixel(sino, g.cols)) : g.cols;
+  const size_t rs = (size_t)g.nangles * ys, item = rs * g.rows;
+  for (unsigned b = blockIdx.z; b < unsigned(n_angles) * unsigned(groups); b += gridDim.z) {
+    const unsigned group = groups == 1 ? 0 : b / unsigned(n_angles);
+    const int n = int(b - group * unsigned(n_angles)), theta = theta0 + n;
     const AngleParams& ap = params[theta];
     {
-      const int iu = iu0 + threadIdx.x;
-      const float* y = sino + (group * kItems) * item + (size_t)theta * g.cols + iu;
+      const int iv0 = r0 + int(threadIdx.y) - kRowPad;
+      const float* y = sino.y + (size_t)group * kItems * item + (size_t)theta * ys +
+                       (kSpread ? int(source_pixel(sino, iu)) : iu);
+      if (!kSpread) y += (long long)iv0 * (long long)rs;
       float v[5][kItems];  // rows threadIdx.y + 8 q; the 33rd is the first warp's
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        const int k = int(threadIdx.y) + 8 * q, iv = r0 + k - kRowPad;
-        const bool in = iu < g.cols && iv >= 0 && iv < g.rows && k < 33;
+        const int iv = iv0 + 8 * q;
+        const bool in = iu < g.cols && iv >= 0 && iv < g.rows && (q < 4 || threadIdx.y == 0);
+        const size_t row = kSpread ? source_pixel(sino, iv) * rs : q * (8 * rs);
 #pragma unroll
-        for (int i = 0; i < kItems; ++i)
-          v[q][i] = in ? __ldg(y + i * item + (size_t)iv * g.nangles * g.cols) : 0.0f;
+        for (int i = 0; i < kItems; ++i) {
+          const float x = in ? __ldg(y + i * item + row) : 0.0f;
+          v[q][i] = kSpread ? sino.scale * x : x;
+        }
       }
+      const bool separable = ap.separable;
       ColumnEntry ce{};
-      if (ap.separable && iu < g.cols) ce = columns[(size_t)theta * g.cols + iu];
+      if (separable && iu < g.cols) ce = columns[(size_t)theta * g.cols + iu];
+      const float vd = ap.vs_d, va = ap.vs_a * ce.ma, vs_b = ap.vs_b;
+      const float vt0 = float(iv0 - g.ov);
+      const bool column_sampled = isfinite(ce.Xa) && fabsf(ce.ma) <= kMaxSlopeZ;
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
-        const int k = int(threadIdx.y) + 8 * q;
-        if (k >= 33) break;
-        const float W = pixel_step_z(ap, ce, g, r0 + k - kRowPad, iu);
+        if (q == 4 && threadIdx.y != 0) break;
+        float W = 1.0f;
+        if (separable) {  // as ray_column and ray_step, the column's part taken out
+          const float vt = vt0 + float(8 * q);
+          const float Xb = fmaf(vt, ce.R, ce.P), mb = fmaf(vt, ce.S, ce.Q), vb = vs_b * mb;
+          W = sqrtf(fmaf(vd, vd, fmaf(va, va, vb * vb)));
+          if (!column_sampled || !isfinite(Xb) || !(fabsf(mb) <= kMaxSlopeZ)) W = 0.0f;
+        }
 #pragma unroll
-        for (int i = 0; i < kItems; ++i) s[i][k][threadIdx.x] = W * v[q][i];
+        for (int i = 0; i < kItems; ++i) s[i][threadIdx.y + 8 * q][threadIdx.x] = W * v[q][i];
+      }
+      if (!separable) {
+#pragma unroll 1
+        for (int k = threadIdx.y; k < 33; k += 8) {
+          const float W = pixel_step_z(ap, g, r0 + k - kRowPad, iu);
+#pragma unroll
+          for (int i = 0; i < kItems; ++i) s[i][k][threadIdx.x] *= W;
+        }
       }
     }
     __syncthreads();
-    const int r = r0 + threadIdx.x;
+    const int r = r0 + threadIdx.x, c0 = iu0 + int(threadIdx.y);
+    float2* o = out + group * group_pairs + (((size_t)n * g.cols + c0) * RP + r) * kItems;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int c = int(threadIdx.y) + 8 * q;
-      if (iu0 + c >= g.cols || r >= RP) break;
-      const size_t at = ((size_t)n * g.cols + iu0 + c) * RP + r;
+      if (c0 + 8 * q >= g.cols || r >= RP) break;
       float2 v[kItems];
 #pragma unroll
       for (int i = 0; i < kItems; ++i)
         v[i] = make_float2(s[i][threadIdx.x][c], s[i][threadIdx.x + 1][c]);
       if constexpr (kItems == 2)
-        reinterpret_cast<float4*>(out + group * group_pairs)[at] =
-            make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        *reinterpret_cast<float4*>(o) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
       else
-        out[group * group_pairs + at] = v[0];
+        *o = v[0];
+      o += (size_t)(8 * kItems) * RP;
     }
     __syncthreads();
   }
@@ -621,14 +647,18 @@ ZlaneArgs zlane_args(const tsgb_projector* p, int off_x, int n_ax, int off_y, in
 }
 
 template <int kItems>
-void launch_weights(const tsgb_projector* p, const float* sino, float2* out, long long group_pairs,
+void launch_weights(const tsgb_projector* p, SinoSource sino, float2* out, long long group_pairs,
                     int angle_begin, int n_angles, int groups, cudaStream_t stream) {
   const DeviceGeometry& g = p->g;
   const int RP = g.rows + 2 * kRowPad;
   const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((RP + 31) / 32),
                   unsigned(std::min<long long>((long long)n_angles * groups, 65535)));
-  bp_weight_z_kernel<kItems><<<grid, dim3(32, 8), 0, stream>>>(
-      p->d_params, p->d_columns, sino, out, group_pairs, g, angle_begin, n_angles, groups);
+  if (kItems == 1 && sino.d > 1)
+    bp_weight_z_kernel<1, true><<<grid, dim3(32, 8), 0, stream>>>(
+        p->d_params, p->d_columns, sino, out, group_pairs, g, angle_begin, n_angles, groups);
+  else
+    bp_weight_z_kernel<kItems, false><<<grid, dim3(32, 8), 0, stream>>>(
+        p->d_params, p->d_columns, sino, out, group_pairs, g, angle_begin, n_angles, groups);
 }
 
 }  // namespace
@@ -660,7 +690,7 @@ int64_t bp_scratch_bytes(const tsgb_projector* p) {
   return bp_scratch_volumes(p) * bp_volume_bytes(p->g);
 }
 
-int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz,
+int launch_bp_weight_z(const tsgb_projector* p, SinoSource sino, float* sinoz,
                        int angle_begin, int angle_end, void* stream) {
   const DeviceGeometry& g = p->g;
   float2* out = reinterpret_cast<float2*>(sinoz) +
@@ -696,9 +726,9 @@ int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino
   // weighted sinograms of all items (two items interleaved), then the scratch volumes
   float2* sinoz = reinterpret_cast<float2*>(workspace);
   const int two = zlane_run(p) <= kTwoItemRun ? items / 2 : 0, one = items - 2 * two;
-  if (two > 0) launch_weights<2>(p, sino, sinoz, 2 * pairs, 0, g.nangles, two, stream);
+  if (two > 0) launch_weights<2>(p, {sino}, sinoz, 2 * pairs, 0, g.nangles, two, stream);
   if (one > 0)
-    launch_weights<1>(p, sino + 2 * two * sino_floats, sinoz + 2 * two * pairs, pairs, 0, g.nangles,
+    launch_weights<1>(p, {sino + 2 * two * sino_floats}, sinoz + 2 * two * pairs, pairs, 0, g.nangles,
                       one, stream);
   ZlaneArgs A = zlane_args(p, 0, n_ax, n_ax, n_ay);
   A.item_volt = volt * bp_scratch_volumes(p);

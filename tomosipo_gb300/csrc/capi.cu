@@ -199,7 +199,7 @@ int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
   if (bp_kind == TSGB_BP_BILINEAR)
     return p->n_bil_fast > 0 ? tsgb::bilinear_bytes(p) : 0;
   if (bp_kind != TSGB_BP_MATCHED) return fail(TSGB_ERR_INVALID, "unknown bp_kind");
-  if (p->fine) return fine_sino_bytes(p) + tsgb_bp_workspace_bytes(p->fine, bp_kind);
+  if (p->fine) return tsgb_bp_workspace_bytes(p->fine, bp_kind);
   if (tsgb::flat_bp(p)) return tsgb::flat_bp_bytes(p);
   // row-pair weighted sinogram (two floats per pixel, kRowPad padding rows),
   // then the z-lane kernel's [y][x][z] scratch volumes (either kernel may run)
@@ -260,15 +260,13 @@ int tsgb_direct_bp(tsgb_projector* p, float* vol, const float* sino, int32_t add
   if (rc != TSGB_OK) return rc;
   cudaError_t e;
   if (bp_kind == TSGB_BP_MATCHED && p->fine) {
-    // the transpose of the binning: spread each pixel / d^2 over its block,
-    // then the finer detector's matched backprojection
-    float* fine_sino = static_cast<float*>(workspace);
-    float* fine_ws = reinterpret_cast<float*>(static_cast<char*>(workspace) + fine_sino_bytes(p));
-    e = cudaError_t(tsgb::launch_ss_expand(p, sino, fine_sino, stream));
-    if (e == cudaSuccess)
-      e = cudaError_t(tsgb::launch_bp_matched(p->fine, vol, fine_sino, additive != 0, fine_ws, stream));
+    // the transpose of the binning: the finer detector's matched backprojection of
+    // each pixel / d^2 spread over its block
+    e = cudaError_t(tsgb::launch_bp_matched(p->fine, vol, tsgb::spread_source(sino, p->det_ss),
+                                            additive != 0,
+                                            static_cast<float*>(workspace), stream));
   } else if (bp_kind == TSGB_BP_MATCHED)
-    e = cudaError_t(tsgb::launch_bp_matched(p, vol, sino, additive != 0,
+    e = cudaError_t(tsgb::launch_bp_matched(p, vol, {sino}, additive != 0,
                                             static_cast<float*>(workspace), stream));
   else
     e = cudaError_t(tsgb::launch_bp_bilinear(p, vol, sino, additive != 0,
@@ -388,7 +386,7 @@ int tsgb_direct_bp_angles(tsgb_projector* p, float* vol, const float* sino, int3
                 "backprojection needs " + std::to_string(need) + " bytes of workspace");
   int rc = check_device(p);
   if (rc != TSGB_OK) return rc;
-  cudaError_t e = cudaError_t(tsgb::launch_bp_matched(p, vol, sino, additive != 0,
+  cudaError_t e = cudaError_t(tsgb::launch_bp_matched(p, vol, {sino}, additive != 0,
                                                       static_cast<float*>(workspace), stream,
                                                       int(angle_begin), int(angle_end)));
   if (e != cudaSuccess) return cuda_fail(e, "backprojection launch");

@@ -67,6 +67,20 @@ __device__ __forceinline__ Ray ray_column(const ColumnEntry& c, float vt) {
   return r;
 }
 
+// Row or column of the source that covers row or column n of the projector's detector.
+__device__ __forceinline__ unsigned source_pixel(const SinoSource& s, int n) {
+  return __umulhi(unsigned(n), s.inv_d) >> s.shift;
+}
+
+// Pixel (iv, iu) of angle theta, on the detector.
+template <bool kSpread>
+__device__ __forceinline__ float sino_value(const SinoSource& s, const DeviceGeometry& g, int iv,
+                                            int iu, int theta) {
+  if (!kSpread) return __ldg(s.y + ((size_t)iv * g.nangles + theta) * g.cols + iu);
+  return s.scale * __ldg(s.y + ((size_t)source_pixel(s, iv) * g.nangles + theta) *
+                                   source_pixel(s, g.cols) + source_pixel(s, iu));
+}
+
 // World length of the ray between consecutive planes of the dominant axis.
 __device__ __forceinline__ float ray_step(const AngleParams& ap, const Ray& r) {
   const float vd = ap.vs_d, va = ap.vs_a * r.ma, vb = ap.vs_b * r.mb;

@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(256)
   __shared__ float tile[32][33];  // [row][column]
   const int zs = flat_zs(g);
   const int u0 = blockIdx.x * 32, v0 = blockIdx.y * 32;
-  for (long long b = blockIdx.z; b < (long long)items * n_angles; b += gridDim.z) {
-    const int item = int(b / n_angles);
-    const int theta = angle_begin + int(b - (long long)item * n_angles);
+  for (unsigned b = blockIdx.z; b < unsigned(items) * unsigned(n_angles); b += gridDim.z) {
+    const int item = items == 1 ? 0 : int(b / unsigned(n_angles));
+    const int theta = angle_begin + int(b - unsigned(item) * unsigned(n_angles));
     const AngleParams& ap = params[theta];
     const float P = ap.cb[0], R = ap.cb[2];
     const int iv = v0 + int(threadIdx.x);
@@ -226,14 +226,15 @@ __global__ void __launch_bounds__(256)
     const bool in = iv < g.rows && q > float(-1 - g.oz) && q < float(g.nz - g.oz);
     const float fl = floorf(in ? q : 0.0f), f = in ? q - fl : 0.0f;
     const int j = int(fl) + g.oz;
-    const float* s = sums + item * item_floats + (size_t)theta * g.cols * zs + j;
+    const bool in_a = in && j >= 0, in_d = in && j + 1 < g.nz;
+    const int c0 = u0 + int(threadIdx.y);
+    const float* s = sums + item * item_floats + ((size_t)theta * g.cols + c0) * zs + j;
     float a[4], d[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int c = u0 + int(threadIdx.y) + 8 * q;
-      const float* p = s + (size_t)c * zs;
-      a[q] = in && j >= 0 && c < g.cols ? __ldg(p) : 0.0f;
-      d[q] = in && j + 1 < g.nz && c < g.cols ? __ldg(p + 1) : 0.0f;
+      const bool column = c0 + 8 * q < g.cols;
+      a[q] = in_a && column ? __ldg(s + q * 8 * zs) : 0.0f;
+      d[q] = in_d && column ? __ldg(s + q * 8 * zs + 1) : 0.0f;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -245,17 +246,18 @@ __global__ void __launch_bounds__(256)
       r.Xa = r.Xb = r.mb = 0.0f;
       r.ma = columns[(size_t)theta * g.cols + iu].ma;
       const float W = ray_step(ap, r);
+      const long long row = (long long)g.nangles * g.cols;
+      long long idx = (v0 + int(threadIdx.y)) * row + (long long)theta * g.cols + iu;
+      float* out = sino + item * (g.rows * row);
 #pragma unroll
       for (int k = threadIdx.y, q = 0; q < 4; ++q, k += 8) {
         if (v0 + k >= g.rows) break;
-        const long long idx = ((long long)(v0 + k) * g.nangles + theta) * g.cols + iu;
         const float total = __fmul_rn(tile[k][threadIdx.x], W);
-        if (kMode == 2) {
+        if (kMode == 2)
           sirt_residual(sirt, g, idx, total, W);
-        } else {
-          float* out = sino + (size_t)item * g.rows * g.nangles * g.cols + idx;
-          *out = kMode == 1 ? __fadd_rn(*out, total) : total;
-        }
+        else
+          out[idx] = kMode == 1 ? __fadd_rn(out[idx], total) : total;
+        idx += 8 * row;
       }
     }
     __syncthreads();
@@ -269,25 +271,35 @@ __global__ void __launch_bounds__(256)
 // the two rows around z, as saturating adds; else every row whose tent reaches z.
 // 32 (z) x 32 (column) tiles through shared memory: reads along u, writes along z.
 // blockIdx.x = column tile, blockIdx.y = z tile, blockIdx.z counts items * angles.
-template <bool kWeighted>
+template <bool kWeighted, bool kSpread>
 __global__ void __launch_bounds__(256)
     flat_resample_kernel(const AngleParams* __restrict__ params,
-                         const ColumnEntry* __restrict__ columns, const float* __restrict__ sino,
+                         const ColumnEntry* __restrict__ columns, SinoSource sino,
                          float* __restrict__ out, long long item_floats, DeviceGeometry g,
                          int angle_begin, int n_angles, int items) {
   __shared__ float tile[32][33];  // [z][column]
+  // per z: rows a voxel apart or more: both tents, the first row, which are on the
+  // detector; else P - z, the first row from the anchor, the first row, how many
+  __shared__ float4 s_z[32];
   const int zs = flat_zs(g);
   const int u0 = blockIdx.x * 32, z0 = blockIdx.y * 32;
-  const size_t row = (size_t)g.nangles * g.cols;
-  for (long long b = blockIdx.z; b < (long long)items * n_angles; b += gridDim.z) {
-    const int item = int(b / n_angles);
-    const int theta = angle_begin + int(b - (long long)item * n_angles);
+  const int iu = u0 + int(threadIdx.x);
+  // the source's columns and elements between its rows (kSpread: a coarser detector)
+  const int ys = kSpread ? int(source_pixel(sino, g.cols)) : g.cols;
+  const size_t rs = (size_t)g.nangles * ys;
+  const auto value = [&](const float* y, int iv) {
+    if (!kSpread) return __ldg(y + (long long)iv * (long long)rs);
+    return sino.scale * __ldg(y + source_pixel(sino, iv) * rs);
+  };
+  for (unsigned b = blockIdx.z; b < unsigned(items) * unsigned(n_angles); b += gridDim.z) {
+    const int item = items == 1 ? 0 : int(b / unsigned(n_angles));
+    const int theta = angle_begin + int(b - unsigned(item) * unsigned(n_angles));
     const AngleParams& ap = params[theta];
     const float P = ap.cb[0], R = ap.cb[2], inv = __frcp_rn(R), aR = fabsf(R);
     // P as a multiple of 2^-14 plus a remainder, so that P - z is exact
     const float Ph = (P + 768.0f) - 768.0f, Pl = P - Ph;
-    const int iu = u0 + int(threadIdx.x);
-    const float* y = sino + item * g.rows * row + (size_t)theta * g.cols + iu;
+    const float* y = sino.y + (size_t)item * g.rows * rs + (size_t)theta * ys +
+                     (kSpread ? int(source_pixel(sino, iu)) : iu);
     float W = 1.0f;
     if (!kWeighted && iu < g.cols) {
       Ray r;
@@ -295,39 +307,69 @@ __global__ void __launch_bounds__(256)
       r.ma = columns[(size_t)theta * g.cols + iu].ma;
       W = ray_step(ap, r);
     }
-    if (aR >= 1.0f) {
-      float t[4], y0[4], y1[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int z = z0 + int(threadIdx.y) + 8 * q;
-        const float C = Ph - float(z - g.oz);
+    // the rows that reach each z, found by the first warp: the two around it and their
+    // tents, or the first and last whose tent covers it
+    if (threadIdx.y == 0) {
+      const int z = z0 + int(threadIdx.x);
+      const float C = Ph - float(z - g.oz);
+      if (aR >= 1.0f) {
         const float v = floorf(clamp_coord(-(C + Pl) * inv));
-        t[q] = fabsf(fmaf(v, R, C) + Pl);
+        const float t = fabsf(fmaf(v, R, C) + Pl);
         const int iv = int(v) + g.ov;
-        const bool in = iu < g.cols && z < g.nz;
-        y0[q] = in && iv >= 0 && iv < g.rows ? __ldg(y + iv * row) : 0.0f;
-        y1[q] = in && iv + 1 >= 0 && iv + 1 < g.rows ? __ldg(y + (iv + 1) * row) : 0.0f;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        tile[threadIdx.y + 8 * q][threadIdx.x] = fmaf(
-            __saturatef(1.0f - t[q]), W * y0[q], __saturatef((1.0f - aR) + t[q]) * (W * y1[q]));
-    } else {
-      for (int k = threadIdx.y; k < 32; k += 8) {
-        const int z = z0 + k;
-        float V = 0.0f;
-        if (iu < g.cols && z < g.nz) {
-          const float C = Ph - float(z - g.oz);
-          const float B = C + Pl;
-          const float v1 = (-1.0f - B) * inv, v2 = (1.0f - B) * inv;
-          const int lo = max(0, (int)floorf(clamp_coord(fminf(v1, v2))) + g.ov);
-          const int hi = min(g.rows - 1, (int)ceilf(clamp_coord(fmaxf(v1, v2))) + g.ov);
-          for (int iv = lo; iv <= hi; ++iv)
-            V = fmaf(tent(fmaf(float(iv - g.ov), R, C) + Pl), W * __ldg(y + iv * row), V);
-        }
-        tile[k][threadIdx.x] = V;
+        const int in0 = z < g.nz && iv >= 0 && iv < g.rows ? 1 : 0;
+        const int in1 = z < g.nz && iv + 1 >= 0 && iv + 1 < g.rows ? 2 : 0;
+        s_z[threadIdx.x] = make_float4(__saturatef(1.0f - t), __saturatef((1.0f - aR) + t),
+                                       __int_as_float(iv), __int_as_float(in0 | in1));
+      } else {
+        const float B = C + Pl;
+        // (widened by more than v1's and v2's rounding; a row more has weight 0)
+        const float va = (-1.0f - B) * inv, vb = (1.0f - B) * inv;
+        const float v1 = clamp_coord(fminf(va, vb)), v2 = clamp_coord(fmaxf(va, vb));
+        const int lo = max(0, (int)ceilf(v1 - fmaf(fabsf(v1), 1e-6f, 0.01f)) + g.ov);
+        const int hi = min(g.rows - 1, (int)floorf(v2 + fmaf(fabsf(v2), 1e-6f, 0.01f)) + g.ov);
+        s_z[threadIdx.x] = make_float4(C, float(lo - g.ov), __int_as_float(lo),
+                                       __int_as_float(z < g.nz ? hi - lo + 1 : 0));
       }
     }
+    __syncthreads();
+    float V[4];
+    if (aR >= 1.0f) {
+      float y0[4], y1[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 e = s_z[threadIdx.y + 8 * q];
+        const int iv = __float_as_int(e.z), in = iu < g.cols ? __float_as_int(e.w) : 0;
+        y0[q] = in & 1 ? value(y, iv) : 0.0f;
+        y1[q] = in & 2 ? value(y, iv + 1) : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 e = s_z[threadIdx.y + 8 * q];
+        V[q] = fmaf(e.x, W * y0[q], e.y * (W * y1[q]));
+      }
+    } else {
+      // one row of each of the four z at a time (their loads in flight together)
+      int n[4], most = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        n[q] = iu < g.cols ? __float_as_int(s_z[threadIdx.y + 8 * q].w) : 0;
+        most = max(most, n[q]);
+        V[q] = 0.0f;
+      }
+      for (int i = 0; i < most; ++i) {
+        float yi[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          yi[q] = i < n[q] ? value(y, __float_as_int(s_z[threadIdx.y + 8 * q].z) + i) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 e = s_z[threadIdx.y + 8 * q];
+          if (i < n[q]) V[q] = fmaf(tent(fmaf(e.y + float(i), R, e.x) + Pl), W * yi[q], V[q]);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) tile[threadIdx.y + 8 * q][threadIdx.x] = V[q];
     __syncthreads();
     const int z = z0 + int(threadIdx.x);
 #pragma unroll
@@ -608,7 +650,7 @@ int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool 
   return int(cudaGetLastError());
 }
 
-int launch_flat_bp(const tsgb_projector* p, float* vol, const float* sino, bool weighted,
+int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool weighted,
                    int out_mode, const float* C, float* workspace, void* stream_, int angle_begin,
                    int angle_end, int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -619,12 +661,12 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, const float* sino, bool 
   float* profiles = workspace;
   const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((zs + 31) / 32),
                   unsigned(std::min<long long>((long long)items * n, 65535)));
-  if (weighted)
-    flat_resample_kernel<true><<<grid, dim3(32, 8), 0, stream>>>(
-        p->d_params, p->d_columns, sino, profiles, item_floats, g, angle_begin, n, items);
-  else
-    flat_resample_kernel<false><<<grid, dim3(32, 8), 0, stream>>>(
-        p->d_params, p->d_columns, sino, profiles, item_floats, g, angle_begin, n, items);
+  // (residuals are never spread)
+  const auto resample = weighted     ? flat_resample_kernel<true, false>
+                        : sino.d > 1 ? flat_resample_kernel<false, true>
+                                     : flat_resample_kernel<false, false>;
+  resample<<<grid, dim3(32, 8), 0, stream>>>(p->d_params, p->d_columns, sino, profiles, item_floats,
+                                             g, angle_begin, n, items);
   // the range's angles in each pass's list (ids increase)
   FlatBpArgs A{};
   const auto b = p->host_sep_angles.begin();

@@ -210,10 +210,9 @@ tsgb_tuning default_tuning(const tsgb_projector* p);
 int launch_bp_fdk(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
                   bool additive, float* workspace, void* stream);
 
-// Detector supersampling passes between p's detector and p->fine's (supersample.cu).
+// Detector supersampling: p->fine's sinogram binned to p's detector (supersample.cu).
 int launch_ss_bin(const tsgb_projector* p, const float* fine, float* coarse, bool additive,
                   void* stream);
-int launch_ss_expand(const tsgb_projector* p, const float* coarse, float* fine, void* stream);
 
 // Sets the calling thread's message returned by tsgb_last_error (capi.cu).
 void set_last_error(const std::string& msg);
@@ -335,9 +334,29 @@ inline int bp_scratch_volumes(const tsgb_projector* p) {
 }
 int64_t bp_scratch_bytes(const tsgb_projector* p);
 
+// The sinogram a matched backprojection reads: y itself, or (detector
+// supersampling, d > 1) a d x d times coarser one of which each of the projector's
+// pixels reads scale times the pixel that covers it. Spreading while reading instead of
+// in a pass of its own: 113 us of 4.40 ms at 2 x 2, 128 x 160 x 160 / 200 angles.
+struct SinoSource {
+  const float* y = nullptr;
+  int d = 1;
+  float scale = 1.0f;
+  // n / d = (high word of n inv_d) >> shift for 0 <= n < 2^31 (source_pixel):
+  // 2^shift < d <= 2^(shift + 1), inv_d = ceil(2^(32 + shift) / d)
+  unsigned inv_d = 0;
+  int shift = 0;
+};
+inline SinoSource spread_source(const float* y, int d) {
+  SinoSource s{y, d, 1.0f / float(d * d)};
+  while (2 << s.shift < d) ++s.shift;
+  s.inv_d = unsigned(((1ull << (32 + s.shift)) + d - 1) / d);
+  return s;
+}
+
 // Column-major row-pair weighted sinogram (float pairs) of angles
 // angle_begin .. angle_end - 1 (bp_zlane.cu).
-int launch_bp_weight_z(const tsgb_projector* p, const float* sino, float* sinoz, int angle_begin,
+int launch_bp_weight_z(const tsgb_projector* p, SinoSource sino, float* sinoz, int angle_begin,
                        int angle_end, void* stream);
 // Both z-lane passes over the separable angle lists (offsets into
 // p->d_sep_angles) in one launch into the [y][x][z] scratch volumes at volt
@@ -389,7 +408,7 @@ int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool 
                    int angle_end, bool copies_ready, int items, int64_t item_bytes);
 // weighted: sino already holds W times the values (a SIRT residual);
 // out_mode as launch_zlane_out's.
-int launch_flat_bp(const tsgb_projector* p, float* vol, const float* sino, bool weighted,
+int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool weighted,
                    int out_mode, const float* C, float* workspace, void* stream, int angle_begin,
                    int angle_end, int items, int64_t item_bytes);
 
@@ -400,7 +419,7 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, const float* sino, bool 
 int launch_fp(const tsgb_projector* p, const float* vol, float* sino, bool additive,
               float* workspace, void* stream, const FpSirt* sirt = nullptr, int angle_begin = 0,
               int angle_end = -1, bool copies_ready = false);
-int launch_bp_matched(const tsgb_projector* p, float* vol, const float* sino, bool additive,
+int launch_bp_matched(const tsgb_projector* p, float* vol, SinoSource sino, bool additive,
                       float* workspace, void* stream, int angle_begin = 0, int angle_end = -1);
 int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, bool additive,
                        float* workspace, void* stream);
