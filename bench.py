@@ -956,7 +956,7 @@ def main():
                    "the c2 workload")
     p.add_argument("--bp-kernel", choices=["auto", "pairs", "zlane"], default="auto",
                    help="matched backprojector (tuning bp_kernel; auto = the projector's default: "
-                   "z-lane warps from 448 voxels along z): to profile the voxel-pair kernel")
+                   "z-lane warps unless the volume is thin along z): to profile the voxel-pair kernel")
     args = p.parse_args()
     global N, ANGLES, DET
     N, ANGLES, DET = WORKLOADS[args.workload]

@@ -115,11 +115,10 @@ int tsgb_direct_fp_batch(tsgb_projector* p, const float* vol, float* sino, int64
  * per-slice loop of to_autograd's backward pass
  * (tomosipo/torch_support.py:70-74). With a workspace of
  * tsgb_bp_batch_workspace_bytes(p, n, bp_kind) bytes, matched
- * backprojections of the voxel-pair kernel run on multi-job launches (one
- * launch per pass over as many items as the workspace holds weighted
- * sinograms for, up to 48; they fill the GPU where one small volume does not;
- * the query keeps the workspace within 2 GiB); otherwise one item after
- * another. */
+ * backprojections of det_v-along-z angles run on launches shared by as many
+ * items as the workspace holds (up to 48: they fill the GPU where one small
+ * volume does not; the query keeps the workspace within 2 GiB); otherwise one
+ * item after another. */
 int64_t tsgb_bp_batch_workspace_bytes(const tsgb_projector* p, int64_t n, int32_t bp_kind);
 int tsgb_direct_bp_batch(tsgb_projector* p, float* vol, const float* sino, int64_t n,
                          int32_t additive, int32_t bp_kind, void* workspace,
@@ -215,16 +214,16 @@ int tsgb_sirt_batch_destroy(tsgb_sirt_batch* b);
 
 /* Launch schedule of a projector's forward projection (the order of its
  * independent tiles; a tile is 32 detector rows x 8 columns of one pair of
- * adjacent angles). The detector is cut into patches of fp_patch_rows x
+ * adjacent angles, run as blocks of 4 columns). The detector is cut into patches of fp_patch_rows x
  * fp_patch_cols tiles and the angles into groups of fp_group_pairs pairs;
  * a group's tiles over one patch run together, so the volume slab their rays
  * cross is read from HBM once and reused from L2 across the group's angles.
  * Any values >= 1 give bit-identical results. bp_kernel and bp_shape pick the
  * matched backprojector and its warp shape; they change only the order of
- * fp32 sums. bp_general picks the kernel of angles outside that backprojector. Defaults are set at creation; the Python autotuner times
- * candidates and sets the fastest. Used by tsgb_direct_fp / tsgb_direct_bp and
- * by the batched SIRT passes. No counterpart in the reference (ASTRA's launch
- * shapes are fixed). */
+ * fp32 sums. bp_general picks the kernel of angles outside that backprojector.
+ * Defaults are set at creation; the Python autotuner times candidates and sets
+ * the fastest. Used by tsgb_direct_fp / tsgb_direct_bp and by the batched SIRT
+ * passes. No counterpart in the reference (ASTRA's launch shapes are fixed). */
 typedef struct {
   int32_t fp_patch_rows;  /* tiles of 32 detector rows per patch (>= 1) */
   int32_t fp_patch_cols;  /* tiles of 8 detector columns per patch (>= 1) */

@@ -19,7 +19,8 @@ Every schedule gives bit-identical results: only the order of independent
 tiles changes. For operators with the matched backprojector the tuner then
 times the backprojection under every kernel and warp shape it offers
 (``bp_kernel``: voxel-pair threads or z-lane warps; ``bp_shape``: the z-lane
-window x z run x warps per block) and sets the fastest; these change only the
+window, z run and warps per block. Parallel scans within one slice have one kernel,
+whose times then differ by noise only) and sets the fastest; these change only the
 order of fp32 sums. Results are cached per geometry (shapes, beam kind and a
 hash of the projection vectors) in memory and, if ``cache_path`` is given, in a
 JSON file. No counterpart in the reference, whose ASTRA launch shapes are

@@ -20,10 +20,12 @@
 //     and y for others, so the angles run in two passes with different
 //     thread-to-voxel mappings, the second adding onto the first.
 //     (bp_zlane.cu holds the z-lane form of this step, with a column-major
-//     weighted sinogram; the projector's tuning picks one.)
-//  3. bp_general_kernel handles every other angle: it projects the corners of
-//     the voxel's tent footprint onto the detector and tests every pixel in
-//     their bounding box with the forward projector's own ray formula.
+//     weighted sinogram, and is the default; this kernel runs for volumes thin
+//     along z and wide, and where the tuning picks it.)
+//  3. bp_general_box_kernel handles every other angle with boxes of voxels that
+//     stage the detector region they project to; bp_general_kernel (tuning, and
+//     regions that do not fit) projects the corners of one voxel's tent
+//     footprint onto the detector and tests every pixel in their bounding box.
 //
 // Bilinear backprojection: voxel-driven, bilinear interpolation of the
 // detector at the projected voxel centre, weighted so that it approximates
@@ -530,17 +532,20 @@ __global__ void __launch_bounds__(128)
 // detector much finer than the voxels, or a source inside the box's reach), the
 // box falls back to general_voxel_terms for that angle.
 // Boxes of 16 (z) x 8 (y) x 2 kRunX (x) voxels, kRunX voxels along x per
-// thread (the kernel's template argument). kRunX = 8 measured 41.4 ms at
-// 256^3 / 360 tilted angles, 4 (boxes of 16 x 8 x 8) 47.0 ms, 16 (80
-// registers, 3 blocks per SM) 44.2 ms; the launcher takes 4 where a 16-wide
-// box's detector region would not fit the stage (detectors finer than the
-// voxels), since those angles would fall back to the per-voxel sums. The
-// sinogram layout (kZl) is a template argument too, so that one of the
-// stage's two strides is 1 at compile time, and the window shapes of
-// gen_window_run's switch (3 x 2, 2 x 2, 3 x 3, 2 x 3 pixels: over 99 % of the
-// windows of that scan) are unrolled: 34.6 ms (183.6 ms at 512^3 / 256
-// angles, against 227.8 ms with loops over the window at run time; 3 blocks
-// per SM instead of 4: 35.3 ms).
+// thread (the kernel's template argument): 8, or 4 where a 16-wide box's detector
+// region would not fit the stage (detectors finer than the voxels), since those
+// angles would fall back to the per-voxel sums. The sinogram layout (kZl) is a
+// template argument too, so that one of the stage's two strides is 1 at compile
+// time, and the window shapes of gen_window_run's switch (3 x 2, 2 x 2, 3 x 3,
+// 2 x 3 pixels: over 99 % of the windows of a scan tilted 0.4 rad) are unrolled.
+// A staged pixel is its 1 / den and its weighted value: the numerators of q_a - i
+// and q_b - j are affine in the pixel's indexes for a voxel, so a candidate takes
+// two multiply-adds and two products with 1 / den instead of the four coefficients
+// of its ray (20 bytes staged per pixel instead of 8). Measured at 256^3 / 360 tilted angles: 34.6 -> 24.7 ms, 24.4 ms with 4 x 4 voxels per
+// half-warp on rows 4 (mod 8) pixels apart; 91 ms for one thread per voxel.
+// ncu at 120 x 152 x 161 / 180 angles: issue 68 % busy at 3 blocks per SM (80
+// registers), L1 and shared memory 47 %, 136 thread instructions per voxel and
+// angle for six candidates.
 constexpr int kGenBoxZ = 16, kGenBoxY = 8;
 constexpr int kGenThreads = 256;
 constexpr int kGenStage = 4096;  // staged pixels per angle, padding included

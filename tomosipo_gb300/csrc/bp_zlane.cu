@@ -30,9 +30,10 @@
 //    Several stacked items (batched backprojection) share the launch.
 //
 // Measured (GB300; the matched backprojection, weight pass and transpose
-// included): 512^3 / 1024 angles 94.0 ms, 256^3 / 360 4.30 ms. 256^3 in ncu:
-// 20 thread instructions per voxel-angle, issue 64 %, 5.8 warps per scheduler
-// before the loads were issued a column ahead, waiting mostly for them.
+// included): 512^3 / 1024 angles 92.0 ms, 256^3 / 360 4.14 ms (voxel-pair kernel 144
+// and 6.5 ms). ncu at 256^3: 17 thread instructions per voxel-angle, issue, the
+// FMA pipe and L1 each 65 % busy at 16 warps per SM (128 registers: 40 accumulators
+// and two stages of loads), which bounds it: fixed-latency waits, 1.5 per issue.
 //
 // Arithmetic per (column, voxel) is bp_separable_kernel's: the two row tents
 // of the fast path (|slope| >= 1 rows per voxel) as saturating adds from the
@@ -69,6 +70,9 @@ __device__ __forceinline__ float pixel_step_z(const AngleParams& ap, const Devic
 // column; blockIdx.z counts angles from `theta0`, over groups of kItems stacked
 // sinograms: with kItems = 2 an element holds both items' pairs. (angles * groups
 // fits 32 bits: an angle's tables take 256 bytes, and a batch's workspace is bounded.)
+// DRAM bytes set its floor; what bounds it is issue (70-78 %) and the loads'
+// latency, so each thread has 4 to 5 loads in flight and the column's part of W is
+// taken out of the row loop (512^3 / 1024 angles 1.94 -> 1.26 ms, 0.72 at DRAM rate).
 template <int kItems, bool kSpread>
 __global__ void __launch_bounds__(256)
     bp_weight_z_kernel(const AngleParams* __restrict__ params,

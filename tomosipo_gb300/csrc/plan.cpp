@@ -345,8 +345,9 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   p->fine_rows = all_planes > 0.0 && fine_planes >= 0.25 * all_planes;
   // Detector region of a 16 x 8 x 16 voxel box at the anchor for each general
   // angle (its corners widened by one voxel along a and b, as the kernel
-  // does; pixels from floor(min) to ceil(max) of their projections, an odd
-  // stride): boxes nearer a cone's source project larger, hence the margin.
+  // does; pixels from floor(min) to ceil(max) of their projections): boxes
+  // nearer a cone's source project larger, and the kernel pads its rows to 4
+  // (mod 8) pixels, hence the margin (2048 / 1.5 of the stage's 4096 pixels).
   p->gen_box_wide = true;
   for (int t : *gen_angles) {
     const AngleParams& ap = p->host_params[t];

@@ -148,8 +148,9 @@ struct tsgb_projector {
   bool fine_rows = false;
   // The general backprojector's voxel boxes may be 16 wide along x: the
   // detector region a 16 x 8 x 16 box at the volume's centre projects to, for
-  // every general angle, stays within two thirds of the kernel's stage (else
-  // boxes 8 wide, whose regions are about half as large).
+  // every general angle, stays within a third of the kernel's stage, which
+  // also holds its padding (else boxes 8 wide, whose regions are about half as
+  // large).
   bool gen_box_wide = true;
   // Parallel beam whose rays all stay in one volume slice (no component along z,
   // det_v along z, det_u without one): flat.cu's kernels run both projections.
