@@ -71,6 +71,12 @@ def test_z_extents(dev, nz):
     _check(dev, *_scan(nz, 11, 14, max(1, int(0.9 * nz)), 21))
 
 
+@pytest.mark.parametrize("nz, n", [(192, 12), (193, 12), (385, 9), (140, 190)])
+def test_ranges_of_three_runs(dev, nz, n):
+    """Around the heights where the backprojector's z ranges are 192 voxels, not 256."""
+    _check(dev, *_scan(nz, n, n - 1, nz + 3, int(1.4 * n), angles=5))
+
+
 @pytest.mark.parametrize("nz, ny, nx", [(20, 1, 1), (20, 3, 70), (20, 70, 3), (40, 120, 130),
                                         (70, 130, 140), (130, 100, 90), (16, 190, 180), (17, 190, 180)])
 def test_planes_and_splits(dev, nz, ny, nx):

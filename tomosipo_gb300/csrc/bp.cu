@@ -633,7 +633,8 @@ __device__ __forceinline__ void gen_region(const AngleParams& ap, const DeviceGe
     // along z and an odd stride; scans tilted 0.4 rad with pixels about as large as
     // voxels)
     const int inner = zlayout ? r.nv : r.nu, outer = zlayout ? r.nu : r.nv;
-    const int stride = ((inner + 3) & ~7) + 4;
+    int stride = ((inner + 3) & ~7) + 4;
+    if ((long long)outer * stride > kGenStage) stride = inner | 1;  // (long, narrow regions)
     if (r.nu <= 0 || r.nv <= 0)
       r.mode = 0;
     else if ((long long)outer * stride > kGenStage)

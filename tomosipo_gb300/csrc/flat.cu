@@ -688,6 +688,12 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
     launch_bp_split<2, 1, 4>(A, items, stream);
   else if (zs <= 128)
     launch_bp_split<4, 1, 4>(A, items, stream);
+  else if (192 * ((zs + 191) / 192) < 256 * ((zs + 255) / 256))
+    // z ranges of 3 x 64 voxels leave fewer lanes idle than 2 x 128: nz = 140, 160, 192
+    // and 300 of 192^2 to 256^2 columns 587 -> 547, 536 -> 470, 872 -> 826 and 1853 ->
+    // 1750 us per backprojection (256, where they do not: 1702 -> 3012). The forward
+    // projection gains nothing (437 -> 447 us at 160).
+    launch_bp_split<2, 3, 3>(A, items, stream);
   else
     launch_bp_split<4, 2, 3>(A, items, stream);
   launch_zlane_out(g, out_mode, A.volt[0], A.n[0] > 0 && A.n[1] > 0 ? A.volt[1] : nullptr,
