@@ -179,12 +179,14 @@ __global__ void __launch_bounds__(32 * kWX * kWY, kMinBlocks)
       const int theta = __float_as_int(t2.w);
       const float nw = fmaf(t1.w, yt, fmaf(t2.x, xt, t2.y));
       const float inw = 1.0f / nw;
-      const float ut = fmaf(t0.x, yt, fmaf(t0.y, xt, t0.z)) * inw;
+      // (quotients, one rounding each, once per voxel column and angle: the positions'
+      // errors are most of the result's)
+      const float ut = fmaf(t0.x, yt, fmaf(t0.y, xt, t0.z)) / nw;
       const float fu0 = floorf(ut), fu = ut - fu0;
       // behind the source, or both columns off the detector: nothing to add
       ok = nw > 0.0f && fu0 >= float(-1 - g.ou) && fu0 <= float(g.cols - 1 - g.ou);
-      const float dv = t0.w * inw;
-      const float vb = fmaf(t1.x, yt, fmaf(t1.y, xt, t1.z)) * inw;  // row at z = 0
+      const float dv = t0.w / nw;
+      const float vb = fmaf(t1.x, yt, fmaf(t1.y, xt, t1.z)) / nw;  // row at z = 0
       // rows are monotone in z: inside if the warp's first and last voxel's are
       const float ra = fmaf(zw0, dv, vb), rb = fmaf(zw0 + float(32 * kRun - 1), dv, vb);
       const float margin = fmaf(4e-7f, fabsf(ra) + fabsf(rb), 0.01f);
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(32 * kWX * kWY, kMinBlocks)
           reinterpret_cast<size_t>(pairs) +
           ((size_t(theta) * cp + size_t(iu + kColPad)) * rp + size_t(kRowPad + g.ov) -
            size_t(kFloorBits)) * sizeof(float2);
-      const float wa = K * (1.0f - fu), wb = K * fu;
+      const float wa = fmaf(-fu, K, K), wb = fu * K;
       e[0] = make_float4(wa, wa, wb, wb);
       e[1] = make_float4(dv, vb, __uint_as_float(unsigned(col)), __uint_as_float(unsigned(col >> 32)));
     }
