@@ -174,8 +174,11 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   columns->assign(size_t(g.nangles) * g.cols, ColumnEntry{});
   sep_angles->clear();
   p->fine_rows = false;
-  // (the flat kernels' column lists hold 32-bit column indexes)
-  p->flat = !cone && int64_t(g.nangles) * g.cols < (int64_t(1) << 32);
+  // (the flat kernels' column lists hold 32-bit column indexes, and they step through
+  // their volume copy, with its border on both in-slice axes, in 32-bit offsets)
+  p->flat = !cone && int64_t(g.nangles) * g.cols < (int64_t(1) << 32) &&
+            int64_t(g.ny + 2 * kPad) * (g.nx + 2 * kPad) * ((g.nz + 3) / 4 * 4) <
+                (int64_t(1) << 31);
   double fine_planes = 0.0, all_planes = 0.0;  // (separable angle, column, plane) triples
   gen_angles->clear();
   bil_fast->clear();
