@@ -727,9 +727,11 @@ int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino
   const int n_ax = p->n_sep_ax, n_ay = p->n_separable_bp - n_ax;
   const size_t sino_floats = size_t(g.rows) * g.nangles * g.cols;
   const long long pairs = bp_pairs_bytes(g) / 8, volt = bp_volume_bytes(g) / 4;
-  // weighted sinograms of all items (two items interleaved), then the scratch volumes
+  // weighted sinograms of all items (two items interleaved, as 16-byte elements, in a
+  // workspace aligned to them), then the scratch volumes
   float2* sinoz = reinterpret_cast<float2*>(workspace);
-  const int two = zlane_run(p) <= kTwoItemRun ? items / 2 : 0, one = items - 2 * two;
+  const bool aligned = reinterpret_cast<uintptr_t>(workspace) % sizeof(float4) == 0;
+  const int two = aligned && zlane_run(p) <= kTwoItemRun ? items / 2 : 0, one = items - 2 * two;
   if (two > 0) launch_weights<2>(p, {sino}, sinoz, 2 * pairs, 0, g.nangles, two, stream);
   if (one > 0)
     launch_weights<1>(p, {sino + 2 * two * sino_floats}, sinoz + 2 * two * pairs, pairs, 0, g.nangles,

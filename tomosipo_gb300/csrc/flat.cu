@@ -592,6 +592,12 @@ void launch_bp_split(FlatBpArgs& A, int items, cudaStream_t stream) {
     launch_bp_windows<kFlatX, kV, kR, kMinBlocks, 1>(A, items, stream);
 }
 
+// Buffers start on 16 bytes in workspaces this package allocates. A caller's own may
+// not: its copies and columns are then read one float at a time.
+bool vectors_aligned(const void* workspace) {
+  return reinterpret_cast<uintptr_t>(workspace) % sizeof(float4) == 0;
+}
+
 int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 int64_t copy_bytes(const DeviceGeometry& g) {
   return round256(int64_t(g.ny + 2 * kPad) * (g.nx + 2 * kPad) * flat_zs(g) * 4);
@@ -627,7 +633,7 @@ int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool 
   }
   const int n = angle_end - angle_begin;
   if (n <= 0) return int(cudaGetLastError());
-  if (zs <= 32)
+  if (zs <= 32 || !vectors_aligned(workspace))
     launch_fp_tiles<1, 1>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
   else if (zs <= 64)
     launch_fp_tiles<2, 1>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
@@ -682,7 +688,7 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
   A.volt[1] = A.n[0] > 0 ? A.volt[0] + volt_bytes(g) / 4 : A.volt[0];
   A.item_floats = item_floats;
   A.g = g;
-  if (zs <= 32)
+  if (zs <= 32 || !vectors_aligned(workspace))
     launch_bp_split<1, 1, 4>(A, items, stream);
   else if (zs <= 64)
     launch_bp_split<2, 1, 4>(A, items, stream);
