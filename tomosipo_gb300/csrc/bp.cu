@@ -692,8 +692,10 @@ __device__ __forceinline__ void gen_window_run(const AngleParams& ap, const GenR
   const float u_lo = float(R.u0 - g.ou), u_hi = u_lo + float(R.nu - R.wu);
   const float v_lo = float(R.v0 - g.ov), v_hi = v_lo + float(R.nv - R.wv);
   const int su = kZl ? R.su : 1, sv = kZl ? 1 : R.sv;
-  // stage index of the anchored pixel (0, 0), from floors' kFloorMagic bits
-  const int origin = -(R.u0 - g.ou + int(kFloorBits)) * su - (R.v0 - g.ov + int(kFloorBits)) * sv;
+  // stage index of the anchored pixel (0, 0), from floors' kFloorMagic bits (unsigned:
+  // the biased products wrap around, their sum with a pixel's is its small index)
+  const unsigned origin = -(unsigned(R.u0 - g.ou) + kFloorBits) * unsigned(su) -
+                          (unsigned(R.v0 - g.ov) + kFloorBits) * unsigned(sv);
 #pragma unroll
   for (int m = 0; m < kGenRunX; ++m) {
     if (x0 + m >= g.nx) break;
@@ -702,7 +704,8 @@ __device__ __forceinline__ void gen_window_run(const AngleParams& ap, const GenR
     const float us = fmaf(fm, pu2, nu0) * rw, vs = fmaf(fm, pv2, nv0) * rw;
     const float fu = __fadd_rd(fminf(fmaxf(us + ou, u_lo), u_hi), kFloorMagic);
     const float fv = __fadd_rd(fminf(fmaxf(vs + ov, v_lo), v_hi), kFloorMagic);
-    const int st0 = int(__float_as_uint(fv)) * sv + int(__float_as_uint(fu)) * su + origin;
+    const int st0 = int(__float_as_uint(fv) * unsigned(sv) + __float_as_uint(fu) * unsigned(su) +
+                        origin);
     const float u0 = fu - kFloorMagic, v0 = fv - kFloorMagic;
     const VoxelForms f = voxel_forms(run, m0 + m);
     float acc_m = acc[m];
