@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(256)
           load_pairs<kV>(reinterpret_cast<const float*>(p1) + r * 32 * kV, v1);
 #pragma unroll
           for (int i = 0; i < kP; ++i)
-            acc[q][r][i] = fma2(w1, v1[i], fma2(w0, v0[i], acc[q][r][i]));
+            // (the plane's sample, then the sum: one rounding of the sum per plane)
+            acc[q][r][i] = add2(acc[q][r][i], fma2(w1, v1[i], mul2(w0, v0[i])));
         }
       }
     }
