@@ -278,7 +278,7 @@ int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino
     case 4: launch_run<4, 8>(p, pairs, volt, angle_w, stream); break;
     default: launch_run<5, 8>(p, pairs, volt, angle_w, stream);
   }
-  launch_zlane_out(g, additive ? 1 : 0, volt, nullptr, 0, g.nz, vol, nullptr, 1, stream);
+  launch_zlane_out(g, additive ? 1 : 0, volt, nullptr, 0, g.nz, 0, g.nz, vol, nullptr, 1, stream);
   return int(cudaGetLastError());
 }
 

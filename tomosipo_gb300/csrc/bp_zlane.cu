@@ -521,12 +521,13 @@ enum ZlaneOut { kOutSet = 0, kOutAdd = 1, kOutSirt = 2 };
 // the plain recipe's rounding. volt is the sum of both passes' scratch volumes
 // (volt1 may be null). 32 x 32 tiles of the (x, z) plane of one y through
 // shared memory: reads along z and writes along x are both coalesced.
-// blockIdx.x = item * z tiles + z tile.
+// The scratch volumes hold the slices first_z .. first_z + n_z - 1 (the others' sums
+// are 0). blockIdx.x = item * z tiles + z tile.
 template <int kOut>
 __global__ void __launch_bounds__(256)
     bp_zlane_out_kernel(const float* __restrict__ volt0, const float* __restrict__ volt1,
-                        long long item_volt, int zs, float* __restrict__ vol,
-                        const float* __restrict__ C, DeviceGeometry g) {
+                        long long item_volt, int zs, int first_z, int n_z,
+                        float* __restrict__ vol, const float* __restrict__ C, DeviceGeometry g) {
   __shared__ float tile[32][33];  // [x][z]
   const int z_tiles = (g.nz + 31) / 32, item = blockIdx.x / z_tiles;
   const int z0 = (blockIdx.x - item * z_tiles) * 32, x0 = blockIdx.y * 32;
@@ -537,9 +538,9 @@ __global__ void __launch_bounds__(256)
     float v[4], v1[4], old[4], c[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int x = x0 + int(threadIdx.y) + 8 * q, z = z0 + threadIdx.x;
+      const int x = x0 + int(threadIdx.y) + 8 * q, z = z0 + int(threadIdx.x) - first_z;
       const size_t i = ((size_t)y * g.nx + x) * zs + z;
-      const bool in = x < g.nx && z < g.nz;
+      const bool in = x < g.nx && z >= 0 && z < n_z;
       v[q] = in ? volt0[i] : 0.0f;
       v1[q] = in && volt1 ? volt1[i] : 0.0f;
     }
@@ -668,18 +669,21 @@ void launch_weights(const tsgb_projector* p, SinoSource sino, float2* out, long 
 }  // namespace
 
 void launch_zlane_out(const DeviceGeometry& g, int mode, const float* volt0, const float* volt1,
-                      long long item_volt, int zs, float* vol, const float* C, int items,
-                      void* stream_) {
+                      long long item_volt, int zs, int first_z, int n_z, float* vol,
+                      const float* C, int items, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const dim3 grid(unsigned((g.nz + 31) / 32) * items, unsigned((g.nx + 31) / 32),
                   unsigned(std::min(g.ny, 65535)));
   const dim3 block(32, 8);
   if (mode == kOutSet)
-    bp_zlane_out_kernel<kOutSet><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, vol, C, g);
+    bp_zlane_out_kernel<kOutSet><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, first_z,
+                                                             n_z, vol, C, g);
   else if (mode == kOutAdd)
-    bp_zlane_out_kernel<kOutAdd><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, vol, C, g);
+    bp_zlane_out_kernel<kOutAdd><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, first_z,
+                                                             n_z, vol, C, g);
   else
-    bp_zlane_out_kernel<kOutSirt><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, vol, C, g);
+    bp_zlane_out_kernel<kOutSirt><<<grid, block, 0, stream>>>(volt0, volt1, item_volt, zs, first_z,
+                                                              n_z, vol, C, g);
 }
 
 int64_t bp_pairs_bytes(const DeviceGeometry& g) {
@@ -715,8 +719,8 @@ bool launch_bp_zlane_separable(const tsgb_projector* p, int off_x, int n_ax, int
   A.volt[0] = volt;
   A.volt[1] = n_ax > 0 ? volt + bp_volume_bytes(p->g) / 4 : volt;
   launch_zlane_passes(p, A, 1, static_cast<cudaStream_t>(stream));
-  launch_zlane_out(p->g, out_mode, volt, n_ax > 0 && n_ay > 0 ? A.volt[1] : nullptr, 0, A.zs, vol,
-                   C, 1, stream);
+  launch_zlane_out(p->g, out_mode, volt, n_ax > 0 && n_ay > 0 ? A.volt[1] : nullptr, 0, A.zs, 0,
+                   p->g.nz, vol, C, 1, stream);
   return true;
 }
 
@@ -754,7 +758,8 @@ int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino
     A.volt[1] += 2 * two * A.item_volt;
     launch_zlane_passes(p, A, one, stream);
   }
-  launch_zlane_out(g, additive ? 1 : 0, first, second, A.item_volt, A.zs, vol, nullptr, items, stream);
+  launch_zlane_out(g, additive ? 1 : 0, first, second, A.item_volt, A.zs, 0, g.nz, vol, nullptr,
+                   items, stream);
   return int(cudaGetLastError());
 }
 

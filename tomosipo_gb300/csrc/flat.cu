@@ -16,7 +16,9 @@
 //    the in-slice weights alone.
 //
 // Lanes run along z with kV consecutive floats each, so every load is a full
-// 128 to 512 bytes.
+// 128 to 512 bytes. The kernels see only the slices that some detector row
+// interpolates: their geometry's nz and oz are those slices' (window below), the
+// volume's own only where a caller's volume is addressed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -73,13 +75,13 @@ __device__ __forceinline__ void store_pairs(float* p, const f32x2 (&v)[(kV + 1) 
 // padded with zeros to zs. Each block transposes 32 x 32 tiles of the (x, z)
 // plane through shared memory. blockIdx.x = item * z tiles + z tile.
 __global__ void __launch_bounds__(256)
-    flat_copy_kernel(const float* __restrict__ vol, float* __restrict__ copy, long long item_copy,
-                     DeviceGeometry g) {
+    flat_copy_kernel(const float* __restrict__ vol, long long item_vol, float* __restrict__ copy,
+                     long long item_copy, DeviceGeometry g) {
   __shared__ float tile[32][33];  // [z][x]
   const int zs = flat_zs(g), nxp = g.nx + 2 * kPad, nyp = g.ny + 2 * kPad;
   const int z_tiles = (zs + 31) / 32, item = blockIdx.x / z_tiles;
   const int z0 = (blockIdx.x - item * z_tiles) * 32, x0 = blockIdx.y * 32;
-  vol += (size_t)item * g.nz * g.ny * g.nx;
+  vol += item * item_vol;
   copy += item * item_copy;
   for (int yp = blockIdx.z; yp < nyp; yp += gridDim.z) {
     const int y = yp - kPad, x = x0 + int(threadIdx.x) - kPad;
@@ -548,8 +550,8 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
 
 template <int kV, int kR>
 void launch_fp_tiles(const tsgb_projector* p, const float* copy, float* sums, long long item_floats,
-                     int angle_begin, int angle_end, int items, cudaStream_t stream) {
-  const DeviceGeometry& g = p->g;
+                     const DeviceGeometry& g, int angle_begin, int angle_end, int items,
+                     cudaStream_t stream) {
   const int zs = flat_zs(g);
   const unsigned tiles = unsigned((g.cols + kFlatCols - 1) / kFlatCols) *
                          unsigned((angle_end - angle_begin + kFlatAngles - 1) / kFlatAngles);
@@ -599,6 +601,16 @@ bool vectors_aligned(const void* workspace) {
   return reinterpret_cast<uintptr_t>(workspace) % sizeof(float4) == 0;
 }
 
+// The geometry of the slices p's rows interpolate. A detector of 32 rows over 512
+// slices of 192^2 voxels, 180 angles: forward projection 933 -> 218 us, backprojection
+// 1012 -> 329 (all slices against 64).
+DeviceGeometry window(const tsgb_projector* p) {
+  DeviceGeometry g = p->g;
+  g.oz -= p->flat_z0;
+  g.nz = p->flat_nz;
+  return g;
+}
+
 int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 int64_t copy_bytes(const DeviceGeometry& g) {
   return round256(int64_t(g.ny + 2 * kPad) * (g.nx + 2 * kPad) * flat_zs(g) * 4);
@@ -612,16 +624,20 @@ int64_t volt_bytes(const DeviceGeometry& g) {
 
 }  // namespace
 
-int64_t flat_fp_bytes(const tsgb_projector* p) { return copy_bytes(p->g) + line_bytes(p->g); }
+int64_t flat_fp_bytes(const tsgb_projector* p) {
+  const DeviceGeometry g = window(p);
+  return copy_bytes(g) + line_bytes(g);
+}
 int64_t flat_bp_bytes(const tsgb_projector* p) {
-  return line_bytes(p->g) + bp_scratch_volumes(p) * volt_bytes(p->g);
+  const DeviceGeometry g = window(p);
+  return line_bytes(g) + bp_scratch_volumes(p) * volt_bytes(g);
 }
 
 int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool additive,
                    float* workspace, void* stream_, const FpSirt* sirt, int angle_begin,
                    int angle_end, bool copies_ready, int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const DeviceGeometry& g = p->g;
+  const DeviceGeometry g = window(p);
   const int zs = flat_zs(g);
   const long long item_floats = item_bytes / 4;
   float* copy = workspace;
@@ -630,18 +646,20 @@ int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool 
     const dim3 grid(unsigned((zs + 31) / 32) * unsigned(items),
                     unsigned((g.nx + 2 * kPad + 31) / 32),
                     unsigned(std::min(g.ny + 2 * kPad, 65535)));
-    flat_copy_kernel<<<grid, dim3(32, 8), 0, stream>>>(vol, copy, item_floats, g);
+    const long long slice = (long long)g.ny * g.nx;
+    flat_copy_kernel<<<grid, dim3(32, 8), 0, stream>>>(vol + p->flat_z0 * slice, p->g.nz * slice,
+                                                       copy, item_floats, g);
   }
   const int n = angle_end - angle_begin;
   if (n <= 0) return int(cudaGetLastError());
   if (zs <= 32 || !vectors_aligned(workspace))
-    launch_fp_tiles<1, 1>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
+    launch_fp_tiles<1, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
   else if (zs <= 64)
-    launch_fp_tiles<2, 1>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
+    launch_fp_tiles<2, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
   else if (zs <= 128)
-    launch_fp_tiles<4, 1>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
+    launch_fp_tiles<4, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
   else
-    launch_fp_tiles<4, 2>(p, copy, sums, item_floats, angle_begin, angle_end, items, stream);
+    launch_fp_tiles<4, 2>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
   const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((g.rows + 31) / 32),
                   unsigned(std::min<long long>((long long)items * n, 65535)));
   const dim3 block(32, 8);
@@ -661,7 +679,7 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
                    int out_mode, const float* C, float* workspace, void* stream_, int angle_begin,
                    int angle_end, int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const DeviceGeometry& g = p->g;
+  const DeviceGeometry g = window(p);
   const int zs = flat_zs(g), n = angle_end - angle_begin;
   if (n <= 0) return int(cudaGetLastError());
   const long long item_floats = item_bytes / 4;
@@ -703,8 +721,8 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
     launch_bp_split<2, 3, 3>(A, items, stream);
   else
     launch_bp_split<4, 2, 3>(A, items, stream);
-  launch_zlane_out(g, out_mode, A.volt[0], A.n[0] > 0 && A.n[1] > 0 ? A.volt[1] : nullptr,
-                   item_floats, zs, vol, C, items, stream);
+  launch_zlane_out(p->g, out_mode, A.volt[0], A.n[0] > 0 && A.n[1] > 0 ? A.volt[1] : nullptr,
+                   item_floats, zs, p->flat_z0, p->flat_nz, vol, C, items, stream);
   return int(cudaGetLastError());
 }
 

@@ -179,6 +179,7 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   p->flat = !cone && int64_t(g.nangles) * g.cols < (int64_t(1) << 32) &&
             int64_t(g.ny + 2 * kPad) * (g.nx + 2 * kPad) * ((g.nz + 3) / 4 * 4) <
                 (int64_t(1) << 31);
+  double flat_lo = g.nz, flat_hi = -1.0;       // voxels along z between which flat rows lie
   double fine_planes = 0.0, all_planes = 0.0;  // (separable angle, column, plane) triples
   gen_angles->clear();
   bil_fast->clear();
@@ -296,6 +297,12 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
     ap.bp_general = (separable && b == 0) ? 0 : 1;
     // rays within one slice, all columns' rows at the same heights
     if (ap.bp_general || mb[0] != 0.0 || cb[1] != 0.0) p->flat = false;
+    if (p->flat) {  // the first and last row, as the kernels compute them
+      const double first = g.oz + double(ap.cb[0]) - double(g.ov) * ap.cb[2];
+      const double last = g.oz + double(ap.cb[0]) + double(g.rows - 1 - g.ov) * ap.cb[2];
+      flat_lo = std::min(flat_lo, std::min(first, last));
+      flat_hi = std::max(flat_hi, std::max(first, last));
+    }
     if (ap.bp_general)
       gen_angles->push_back(t);
     else
@@ -381,6 +388,16 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
       p->gen_box_wide = false;
       break;
     }
+  }
+  // Slices that the rows of flat scans interpolate, one more on each side than their
+  // exact positions need (the kernels' are rounded), in steps of 64: lanes hold 32, 64
+  // or 128 consecutive slices.
+  if (p->flat) {
+    const double top = double(g.nz - 1);
+    const int lo = int(std::floor(std::min(std::max(flat_lo - 1.0, 0.0), top)));
+    const int hi = int(std::ceil(std::min(std::max(flat_hi + 1.0, 0.0), top)));
+    p->flat_nz = std::min(g.nz, (std::max(hi - lo, 0) + 1 + 63) / 64 * 64);
+    p->flat_z0 = std::min(lo, g.nz - p->flat_nz);
   }
   p->n_general_bp = int(gen_angles->size());
   // Separable angles grouped by their in-plane axis a (x first, then y): the

@@ -155,6 +155,9 @@ struct tsgb_projector {
   // Parallel beam whose rays all stay in one volume slice (no component along z,
   // det_v along z, det_u without one): flat.cu's kernels run both projections.
   bool flat = false;
+  // Slices flat_z0 .. flat_z0 + flat_nz - 1 hold every slice that a detector row of
+  // any angle interpolates (flat.cu works on these alone).
+  int flat_z0 = 0, flat_nz = 0;
   int n_bil_fast = 0;           // bilinear BP: angles for the z-flat kernel
   int n_bil_slow = 0;           // bilinear BP: angles for the general kernel
   tsgb::AngleParams* d_params = nullptr;
@@ -374,10 +377,11 @@ int launch_bp_zlane_batch(const tsgb_projector* p, float* vol, const float* sino
 
 // [y][x][z] scratch volumes (rows of zs floats along z) to the caller's volume:
 // vol (=, +=, SIRT: out_mode 0 / 1 / 2) volt0 + volt1 (volt1 may be null) for
-// `items` stacked items, scratch volumes item_volt floats apart (bp_zlane.cu).
+// `items` stacked items, scratch volumes item_volt floats apart (bp_zlane.cu). The
+// scratch volumes hold the slices first_z .. first_z + n_z - 1; the others' sums are 0.
 void launch_zlane_out(const DeviceGeometry& g, int out_mode, const float* volt0,
-                      const float* volt1, long long item_volt, int zs, float* vol, const float* C,
-                      int items, void* stream);
+                      const float* volt1, long long item_volt, int zs, int first_z, int n_z,
+                      float* vol, const float* C, int items, void* stream);
 
 // Volumes of at most nz voxels along z and 2^15 or more in the slice: they leave
 // most of the z-lane kernels' lanes idle, and fill the GPU without them.
