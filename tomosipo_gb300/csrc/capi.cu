@@ -437,7 +437,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
   const int64_t chunk = tsgb::fp_angle_chunk(f->g);
   // (parallel beams through flat.cu: copy, line sums, rows; resample, windows, out)
   const int64_t fp_launches =
-      f->flat ? 3 + extra
+      f->flat ? 1 + 2 * tsgb::flat_chunks(f) + extra
               : int64_t(f->layouts.size()) + (f->g.nangles + chunk - 1) / chunk + extra;
   // weight pass, both z-lane passes and the transpose out of their scratch (or
   // one launch per voxel-pair pass), the general kernel
@@ -446,7 +446,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
       : tsgb::bp_uses_zlane(f) ? 2
                                : (f->n_sep_ax > 0) + (f->n_separable_bp > f->n_sep_ax);
   const int64_t bp_launches =
-      (tsgb::flat_bp(f) ? 3
+      (tsgb::flat_bp(f) ? 1 + 2 * tsgb::flat_chunks(f)
                : chunks + sep_launches + ((f->n_general_bp > 0 || f->n_separable_bp == 0) ? 1 : 0)) +
       extra;
   const int64_t vals[8] = {int64_t(f->layouts.size()),

@@ -46,10 +46,13 @@ struct Vec<4> {
   using T = float4;
 };
 
-// kV floats at p as packed pairs (kV = 1: the second half is 0).
-template <int kV>
+// kV floats at p as packed pairs (kV = 1: the second half is 0). kConstant: memory that
+// the kernel does not write.
+template <int kV, bool kConstant = true>
 __device__ __forceinline__ void load_pairs(const float* p, f32x2 (&v)[(kV + 1) / 2]) {
-  const typename Vec<kV>::T x = __ldg(reinterpret_cast<const typename Vec<kV>::T*>(p));
+  using T = typename Vec<kV>::T;
+  const T* q = reinterpret_cast<const T*>(p);
+  const T x = kConstant ? __ldg(q) : *q;
   if constexpr (kV == 1) v[0] = pack2(x, 0.0f);
   if constexpr (kV == 2) v[0] = pack2(x.x, x.y);
   if constexpr (kV == 4) {
@@ -116,6 +119,7 @@ constexpr int kFlatPlanes = 32;  // planes prepared at a time, one per lane
 // columns with the weights 1 - fa and fa. Positions, weights and offsets of 32
 // planes at a time are computed with one lane per plane and read back from shared
 // memory. Planes alternate between two partial sums.
+// sums holds the angles from angle_begin on.
 // blockIdx.x = tile, blockIdx.y = z range, blockIdx.z = item.
 template <int kV, int kR>
 __global__ void __launch_bounds__(256)
@@ -195,7 +199,8 @@ __global__ void __launch_bounds__(256)
     }
     __syncwarp();
   }
-  float* out = sums + blockIdx.z * item_floats + ((size_t)theta * g.cols + iu) * zs + z0;
+  float* out =
+      sums + blockIdx.z * item_floats + ((size_t)(theta - angle_begin) * g.cols + iu) * zs + z0;
 #pragma unroll
   for (int r = 0; r < kR; ++r) {
     if (z0 + r * 32 * kV >= zs) break;
@@ -221,7 +226,7 @@ __global__ void __launch_bounds__(256)
   const int u0 = blockIdx.x * 32, v0 = blockIdx.y * 32;
   for (unsigned b = blockIdx.z; b < unsigned(items) * unsigned(n_angles); b += gridDim.z) {
     const int item = items == 1 ? 0 : int(b / unsigned(n_angles));
-    const int theta = angle_begin + int(b - unsigned(item) * unsigned(n_angles));
+    const int n = int(b - unsigned(item) * unsigned(n_angles)), theta = angle_begin + n;
     const AngleParams& ap = params[theta];
     const float P = ap.cb[0], R = ap.cb[2];
     const int iv = v0 + int(threadIdx.x);
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(256)
     const int j = int(fl) + g.oz;
     const bool in_a = in && j >= 0, in_d = in && j + 1 < g.nz;
     const int c0 = u0 + int(threadIdx.y);
-    const float* s = sums + item * item_floats + ((size_t)theta * g.cols + c0) * zs + j;
+    const float* s = sums + item * item_floats + ((size_t)n * g.cols + c0) * zs + j;
     float a[4], d[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -272,8 +277,8 @@ __global__ void __launch_bounds__(256)
 // V[theta][u][z] = sum over the detector rows of tent(P + v R - z) W y[v][theta][u]
 // (W = 1 when kWeighted: a SIRT residual holds W y). Rows at least a voxel apart:
 // the two rows around z, as saturating adds; else every row whose tent reaches z.
-// 32 (z) x 32 (column) tiles through shared memory: reads along u, writes along z.
-// blockIdx.x = column tile, blockIdx.y = z tile, blockIdx.z counts items * angles.
+// 32 (z) x 32 (column) tiles through shared memory: reads along u, writes along z. out
+// holds the angles from angle_begin on. blockIdx.x = column tile, blockIdx.y = z tile, blockIdx.z counts items * angles.
 template <bool kWeighted, bool kSpread>
 __global__ void __launch_bounds__(256)
     flat_resample_kernel(const AngleParams* __restrict__ params,
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(256)
   };
   for (unsigned b = blockIdx.z; b < unsigned(items) * unsigned(n_angles); b += gridDim.z) {
     const int item = items == 1 ? 0 : int(b / unsigned(n_angles));
-    const int theta = angle_begin + int(b - unsigned(item) * unsigned(n_angles));
+    const int angle = int(b - unsigned(item) * unsigned(n_angles)), theta = angle_begin + angle;
     const AngleParams& ap = params[theta];
     const float P = ap.cb[0], R = ap.cb[2], inv = __frcp_rn(R), aR = fabsf(R);
     // P as a multiple of 2^-14 plus a remainder, so that P - z is exact
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int c = threadIdx.y, q = 0; q < 4; ++q, c += 8)
       if (z < zs && u0 + c < g.cols)
-        out[item * item_floats + ((size_t)theta * g.cols + u0 + c) * zs + z] = tile[threadIdx.x][c];
+        out[item * item_floats + ((size_t)angle * g.cols + u0 + c) * zs + z] = tile[threadIdx.x][c];
     __syncthreads();
   }
 }
@@ -389,8 +394,10 @@ struct FlatBpArgs {
   int plane_blocks[2];
   unsigned blocks0;
   const ColumnEntry* columns;
-  const float* profiles;       // V[theta][u][z]
+  const float* profiles;       // V[theta][u][z] from column first_column (theta, u) on
+  unsigned first_column;
   float* volt[2];              // [y][x][z] sum of each pass
+  bool add[2];                 // onto what volt holds (angles of an earlier launch)
   long long item_floats;
   DeviceGeometry g;
 };
@@ -477,7 +484,7 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
         const float fq = __fadd_rd(qa, kFloorMagic);
         const float fa = qa - (fq - kFloorMagic);
         e = make_float4(1.0f - fa, 1.0f - fa, fa, fa);
-        c = make_int2(int(__float_as_uint(fq) - kFloorBits), int(unsigned(ci)));
+        c = make_int2(int(__float_as_uint(fq) - kFloorBits), int(unsigned(ci) - A.first_column));
       }
       const unsigned mask = __ballot_sync(0xffffffffu, ok);
       if (ok) {
@@ -543,6 +550,12 @@ __global__ void __launch_bounds__(32 * kFlatWarps, kMinBlocks)
       f32x2 x[kP];
 #pragma unroll
       for (int i = 0; i < kP; ++i) x[i] = acc[0][m][r * kP + i];
+      if (A.add[pass]) {
+        f32x2 old[kP];
+        load_pairs<kV, false>(out + r * 32 * kV, old);
+#pragma unroll
+        for (int i = 0; i < kP; ++i) x[i] = add2(old[i], x[i]);
+      }
       store_pairs<kV>(out + r * 32 * kV, x);
     }
   }
@@ -615,8 +628,17 @@ int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 int64_t copy_bytes(const DeviceGeometry& g) {
   return round256(int64_t(g.ny + 2 * kPad) * (g.nx + 2 * kPad) * flat_zs(g) * 4);
 }
+// Angles whose line sums or profiles the kernels hold at a time: about 2 GiB of them
+// (whole patches of angle groups), so that a long scan does not need its sinogram's size
+// or more once again. Pieces cost their launches and, in the backprojection, a read of
+// the scratch volumes each.
+int line_angles(const DeviceGeometry& g) {
+  constexpr int64_t kBudget = int64_t(2) << 30, kPatch = kFlatAngles * kPatchAngles;
+  const int64_t fit = kBudget / (int64_t(g.cols) * flat_zs(g) * 4) / kPatch * kPatch;
+  return int(std::min<int64_t>(g.nangles, std::max(fit, kPatch)));
+}
 int64_t line_bytes(const DeviceGeometry& g) {
-  return round256(int64_t(g.nangles) * g.cols * flat_zs(g) * 4);
+  return round256(int64_t(line_angles(g)) * g.cols * flat_zs(g) * 4);
 }
 int64_t volt_bytes(const DeviceGeometry& g) {
   return round256(int64_t(g.ny) * g.nx * flat_zs(g) * 4);
@@ -632,13 +654,16 @@ int64_t flat_bp_bytes(const tsgb_projector* p) {
   const DeviceGeometry g = window(p);
   return line_bytes(g) + bp_scratch_volumes(p) * volt_bytes(g);
 }
+int flat_chunks(const tsgb_projector* p) {
+  return (p->g.nangles - 1) / line_angles(window(p)) + 1;
+}
 
 int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool additive,
                    float* workspace, void* stream_, const FpSirt* sirt, int angle_begin,
                    int angle_end, bool copies_ready, int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const DeviceGeometry g = window(p);
-  const int zs = flat_zs(g);
+  const int zs = flat_zs(g), step = line_angles(g);
   const long long item_floats = item_bytes / 4;
   float* copy = workspace;
   float* sums = workspace + copy_bytes(g) / 4;
@@ -650,28 +675,24 @@ int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool 
     flat_copy_kernel<<<grid, dim3(32, 8), 0, stream>>>(vol + p->flat_z0 * slice, p->g.nz * slice,
                                                        copy, item_floats, g);
   }
-  const int n = angle_end - angle_begin;
-  if (n <= 0) return int(cudaGetLastError());
-  if (zs <= 32 || !vectors_aligned(workspace))
-    launch_fp_tiles<1, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
-  else if (zs <= 64)
-    launch_fp_tiles<2, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
-  else if (zs <= 128)
-    launch_fp_tiles<4, 1>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
-  else
-    launch_fp_tiles<4, 2>(p, copy, sums, item_floats, g, angle_begin, angle_end, items, stream);
-  const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((g.rows + 31) / 32),
-                  unsigned(std::min<long long>((long long)items * n, 65535)));
-  const dim3 block(32, 8);
-  if (sirt)
-    fp_flat_rows_kernel<2><<<grid, block, 0, stream>>>(p->d_params, p->d_columns, sums, item_floats,
-                                                       sino, g, angle_begin, n, items, *sirt);
-  else if (additive)
-    fp_flat_rows_kernel<1><<<grid, block, 0, stream>>>(p->d_params, p->d_columns, sums, item_floats,
-                                                       sino, g, angle_begin, n, items, FpSirt{});
-  else
-    fp_flat_rows_kernel<0><<<grid, block, 0, stream>>>(p->d_params, p->d_columns, sums, item_floats,
-                                                       sino, g, angle_begin, n, items, FpSirt{});
+  for (int a0 = angle_begin, a1; a0 < angle_end; a0 = a1) {
+    a1 = int(std::min<int64_t>(int64_t(a0) + step, angle_end));
+    if (zs <= 32 || !vectors_aligned(workspace))
+      launch_fp_tiles<1, 1>(p, copy, sums, item_floats, g, a0, a1, items, stream);
+    else if (zs <= 64)
+      launch_fp_tiles<2, 1>(p, copy, sums, item_floats, g, a0, a1, items, stream);
+    else if (zs <= 128)
+      launch_fp_tiles<4, 1>(p, copy, sums, item_floats, g, a0, a1, items, stream);
+    else
+      launch_fp_tiles<4, 2>(p, copy, sums, item_floats, g, a0, a1, items, stream);
+    const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((g.rows + 31) / 32),
+                    unsigned(std::min<long long>((long long)items * (a1 - a0), 65535)));
+    const auto rows = sirt       ? fp_flat_rows_kernel<2>
+                      : additive ? fp_flat_rows_kernel<1>
+                                 : fp_flat_rows_kernel<0>;
+    rows<<<grid, dim3(32, 8), 0, stream>>>(p->d_params, p->d_columns, sums, item_floats, sino, g, a0,
+                                           a1 - a0, items, sirt ? *sirt : FpSirt{});
+  }
   return int(cudaGetLastError());
 }
 
@@ -680,49 +701,55 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
                    int angle_end, int items, int64_t item_bytes) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const DeviceGeometry g = window(p);
-  const int zs = flat_zs(g), n = angle_end - angle_begin;
-  if (n <= 0) return int(cudaGetLastError());
-  const long long item_floats = item_bytes / 4;
-  float* profiles = workspace;
-  const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((zs + 31) / 32),
-                  unsigned(std::min<long long>((long long)items * n, 65535)));
-  // (residuals are never spread)
-  const auto resample = weighted     ? flat_resample_kernel<true, false>
-                        : sino.d > 1 ? flat_resample_kernel<false, true>
-                                     : flat_resample_kernel<false, false>;
-  resample<<<grid, dim3(32, 8), 0, stream>>>(p->d_params, p->d_columns, sino, profiles, item_floats,
-                                             g, angle_begin, n, items);
-  // the range's angles in each pass's list (ids increase)
+  const int zs = flat_zs(g), step = line_angles(g);
+  if (angle_end <= angle_begin) return int(cudaGetLastError());
   FlatBpArgs A{};
-  const auto b = p->host_sep_angles.begin();
-  for (int pass = 0; pass < 2; ++pass) {
-    const auto lo = pass ? b + p->n_sep_ax : b, hi = pass ? p->host_sep_angles.end() : b + p->n_sep_ax;
-    const auto first = std::lower_bound(lo, hi, angle_begin);
-    A.solve[pass] = p->d_solve + (first - b);
-    A.n[pass] = int(std::lower_bound(first, hi, angle_end) - first);
-  }
   A.columns = p->d_columns;
-  A.profiles = profiles;
-  A.volt[0] = workspace + line_bytes(g) / 4;
-  A.volt[1] = A.n[0] > 0 ? A.volt[0] + volt_bytes(g) / 4 : A.volt[0];
-  A.item_floats = item_floats;
+  A.profiles = workspace;
+  A.item_floats = item_bytes / 4;
   A.g = g;
-  if (zs <= 32 || !vectors_aligned(workspace))
-    launch_bp_split<1, 1, 4>(A, items, stream);
-  else if (zs <= 64)
-    launch_bp_split<2, 1, 4>(A, items, stream);
-  else if (zs <= 128)
-    launch_bp_split<4, 1, 4>(A, items, stream);
-  else if (192 * ((zs + 191) / 192) < 256 * ((zs + 255) / 256))
-    // z ranges of 3 x 64 voxels leave fewer lanes idle than 2 x 128: nz = 140, 160, 192
-    // and 300 of 192^2 to 256^2 columns 587 -> 547, 536 -> 470, 872 -> 826 and 1853 ->
-    // 1750 us per backprojection (256, where they do not: 1702 -> 3012). The forward
-    // projection gains nothing (437 -> 447 us at 160).
-    launch_bp_split<2, 3, 3>(A, items, stream);
-  else
-    launch_bp_split<4, 2, 3>(A, items, stream);
-  launch_zlane_out(p->g, out_mode, A.volt[0], A.n[0] > 0 && A.n[1] > 0 ? A.volt[1] : nullptr,
-                   item_floats, zs, p->flat_z0, p->flat_nz, vol, C, items, stream);
+  // a pass's angles in [a0, a1): where they lie in its list (ids increase), how many
+  const auto b = p->host_sep_angles.begin();
+  const auto range = [&](int pass, int a0, int a1, int* n) {
+    const auto lo = pass ? b + p->n_sep_ax : b, hi = pass ? p->host_sep_angles.end() : b + p->n_sep_ax;
+    const auto first = std::lower_bound(lo, hi, a0);
+    *n = int(std::lower_bound(first, hi, a1) - first);
+    return p->d_solve + (first - b);
+  };
+  int all[2];
+  for (int pass = 0; pass < 2; ++pass) range(pass, angle_begin, angle_end, &all[pass]);
+  A.volt[0] = workspace + line_bytes(g) / 4;
+  A.volt[1] = all[0] > 0 ? A.volt[0] + volt_bytes(g) / 4 : A.volt[0];
+  for (int a0 = angle_begin, a1; a0 < angle_end; a0 = a1) {
+    a1 = int(std::min<int64_t>(int64_t(a0) + step, angle_end));
+    const dim3 grid(unsigned((g.cols + 31) / 32), unsigned((zs + 31) / 32),
+                    unsigned(std::min<long long>((long long)items * (a1 - a0), 65535)));
+    // (residuals are never spread)
+    const auto resample = weighted     ? flat_resample_kernel<true, false>
+                          : sino.d > 1 ? flat_resample_kernel<false, true>
+                                       : flat_resample_kernel<false, false>;
+    resample<<<grid, dim3(32, 8), 0, stream>>>(p->d_params, p->d_columns, sino, workspace,
+                                               A.item_floats, g, a0, a1 - a0, items);
+    A.first_column = unsigned(a0) * unsigned(g.cols);
+    for (int pass = 0; pass < 2; ++pass) A.solve[pass] = range(pass, a0, a1, &A.n[pass]);
+    if (zs <= 32 || !vectors_aligned(workspace))
+      launch_bp_split<1, 1, 4>(A, items, stream);
+    else if (zs <= 64)
+      launch_bp_split<2, 1, 4>(A, items, stream);
+    else if (zs <= 128)
+      launch_bp_split<4, 1, 4>(A, items, stream);
+    else if (192 * ((zs + 191) / 192) < 256 * ((zs + 255) / 256))
+      // z ranges of 3 x 64 voxels leave fewer lanes idle than 2 x 128: nz = 140, 160, 192
+      // and 300 of 192^2 to 256^2 columns 587 -> 547, 536 -> 470, 872 -> 826 and 1853 ->
+      // 1750 us per backprojection (256, where they do not: 1702 -> 3012). The forward
+      // projection gains nothing (437 -> 447 us at 160).
+      launch_bp_split<2, 3, 3>(A, items, stream);
+    else
+      launch_bp_split<4, 2, 3>(A, items, stream);
+    for (int pass = 0; pass < 2; ++pass) A.add[pass] = A.add[pass] || A.n[pass] > 0;
+  }
+  launch_zlane_out(p->g, out_mode, A.volt[0], all[0] > 0 && all[1] > 0 ? A.volt[1] : nullptr,
+                   A.item_floats, zs, p->flat_z0, p->flat_nz, vol, C, items, stream);
   return int(cudaGetLastError());
 }
 

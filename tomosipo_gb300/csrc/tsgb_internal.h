@@ -401,13 +401,15 @@ int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino
 
 // Parallel beams through flat.cu (p->flat). Workspace bytes of one item's
 // forward projection (volume copy, per-slice line sums) and backprojection
-// (sinogram resampled to the slices, scratch volumes); the projections of
+// (sinogram resampled to the slices, scratch volumes), in pieces of as many angles as
+// about 2 GiB of line sums or profiles hold; the projections of
 // `items` stacked items with their workspaces item_bytes apart.
 // (up to 16 voxels along z a thin, wide volume keeps the voxel-pair kernel: 256^2
 // slice, 360 angles, 16 voxels 0.85 ms against 0.91, 40 voxels 1.46 against 0.97)
 inline bool flat_bp(const tsgb_projector* p) { return p->flat && !thin_volume(p, 16); }
 int64_t flat_fp_bytes(const tsgb_projector* p);
 int64_t flat_bp_bytes(const tsgb_projector* p);
+int flat_chunks(const tsgb_projector* p);
 int launch_flat_fp(const tsgb_projector* p, const float* vol, float* sino, bool additive,
                    float* workspace, void* stream, const FpSirt* sirt, int angle_begin,
                    int angle_end, bool copies_ready, int items, int64_t item_bytes);
