@@ -218,9 +218,11 @@ int tsgb_sirt_batch_destroy(tsgb_sirt_batch* b);
  * fp_patch_cols tiles and the angles into groups of fp_group_pairs pairs;
  * a group's tiles over one patch run together, so the volume slab their rays
  * cross is read from HBM once and reused from L2 across the group's angles.
- * Any values >= 1 give bit-identical results. bp_kernel and bp_shape pick the
- * matched backprojector and its warp shape; they change only the order of
- * fp32 sums. bp_general picks the kernel of angles outside that backprojector.
+ * Any values >= 1 give bit-identical results; they have no effect on parallel
+ * scans whose rays stay in one slice, whose projector has no such order.
+ * bp_kernel and bp_shape pick the matched backprojector and its warp shape; they
+ * change only the order of fp32 sums. bp_general picks the kernel of angles
+ * outside that backprojector.
  * Defaults are set at creation; the Python autotuner times candidates and sets
  * the fastest. Used by tsgb_direct_fp / tsgb_direct_bp and by the batched SIRT
  * passes. No counterpart in the reference (ASTRA's launch shapes are fixed). */
@@ -232,7 +234,9 @@ typedef struct {
                              loads per sample), 0: single voxels (four 4-byte) */
   int32_t bp_kernel;      /* matched backprojection of det_v-along-z angles:
                              1: z-lane warps over a column-major weighted
-                             sinogram, 0: voxel-pair threads over a row-major one */
+                             sinogram (parallel scans whose rays stay in one
+                             slice: the slice kernels, without bp_shape),
+                             0: voxel-pair threads over a row-major one */
   int32_t bp_shape;       /* z-lane warp shape: 0, 1, 2: chosen from the volume's
                              z extent (at most 8 voxels along z per lane);
                              3: 4-voxel windows, 16 planes per block and 4:
@@ -267,7 +271,7 @@ int tsgb_fdk_backproject(tsgb_projector* p, float* vol, const float* filtered,
 int tsgb_projector_shapes(const tsgb_projector* p, int64_t vol_shape[3],
                           int64_t sino_shape[3]);
 
-/* Plan statistics, written to out[0..n-1] (n <= 8):
+/* Plan statistics, written to out[0..n-1] (n <= 10):
  *   [0] padded volume copies the forward projector builds (axis permutations)
  *   [1] angles backprojected by the separable (det_v along z) gather kernel
  *   [2] angles backprojected by the general gather kernel
@@ -275,6 +279,9 @@ int tsgb_projector_shapes(const tsgb_projector* p, int64_t vol_shape[3],
  *   [4] kernel launches per matched tsgb_direct_bp call
  *   [5] kernel launches per bilinear tsgb_direct_bp call
  *   [6] forward workspace bytes, [7] matched backprojection workspace bytes
+ *   [8] forward kernel: 0 rays, 1 slice by slice (parallel beams within slices)
+ *   [9] matched backprojection of det_v-along-z angles: 0 none, 1 voxel-pair
+ *       threads, 2 z-lane warps, 3 slice by slice
  * No counterpart in ASTRA's projector; used for measurement and tests. */
 int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n);
 

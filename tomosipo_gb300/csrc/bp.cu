@@ -1307,11 +1307,12 @@ void angle_sub_range(const std::vector<int>& host_list, int lo, int hi, int a0, 
 }  // namespace
 
 int launch_bp_matched(const tsgb_projector* p, float* vol, SinoSource sino, bool additive,
-                      float* workspace, void* stream_, int angle_begin, int angle_end) {
+                      float* workspace, void* stream_, bool slices, int angle_begin,
+                      int angle_end) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const DeviceGeometry& g = p->g;
   if (angle_end < 0) angle_end = g.nangles;
-  if (flat_bp(p))
+  if (flat_bp(p) || slices)
     return launch_flat_bp(p, vol, sino, false, additive ? 1 : 0, nullptr, workspace, stream,
                           angle_begin, angle_end, 1, 0);
   // the angles of [angle_begin, angle_end) in each of the three angle lists

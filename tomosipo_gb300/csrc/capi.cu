@@ -180,18 +180,34 @@ int64_t fine_sino_bytes(const tsgb_projector* p) {
   return (int64_t(f.rows) * f.nangles * f.cols * int64_t(sizeof(float)) + 255) / 256 * 256;
 }
 
+// What batched SIRT's backprojection keeps in the forward workspace: the slice kernels'
+// profiles and scratch volumes, or the voxel-pair kernel's first sum; else a sum volume
+// and the z-lane kernel's scratch volumes.
+int64_t sirt_scratch_bytes(const tsgb_projector* p) {
+  const int64_t volume = tsgb::bp_volume_bytes(p->g);
+  return p->flat ? std::max(tsgb::flat_bp_bytes(p), volume) : volume + tsgb::bp_scratch_bytes(p);
+}
+
+// The least workspace of a matched backprojection (p runs it: the finer projector of a
+// supersampled detector). Scans within slices run slice by slice, whatever the tuning
+// says, in workspaces that hold no row pairs.
+int64_t bp_bytes(const tsgb_projector* p) {
+  return p->flat ? tsgb::flat_bp_bytes(p) : tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED);
+}
+bool slices_only(const tsgb_projector* p, int64_t workspace_bytes) {
+  return p->flat && workspace_bytes < tsgb::bp_pairs_bytes(p->g);
+}
+
 }  // namespace
 
 int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p) {
   if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
   if (p->fine) return fine_sino_bytes(p) + tsgb_fp_workspace_bytes(p->fine);
-  // (batched SIRT backprojects in the forward workspace)
-  const int64_t sirt_bytes = tsgb::flat_bp(p) ? tsgb::flat_bp_bytes(p)
-                                              : tsgb::bp_volume_bytes(p->g) + tsgb::bp_scratch_bytes(p);
-  if (p->flat) return std::max(tsgb::flat_fp_bytes(p), sirt_bytes);
-  // volume copies (pairs of floats); batched SIRT also keeps its sum volume and
-  // the backprojection's scratch volumes there
-  return std::max(p->fp_workspace_elems * int64_t(2 * sizeof(float)), sirt_bytes);
+  // volume copies (pairs of floats), or the slice kernels' copy and line sums; batched
+  // SIRT backprojects there, by whichever kernel the tuning picks
+  return std::max(p->flat ? tsgb::flat_fp_bytes(p)
+                          : p->fp_workspace_elems * int64_t(2 * sizeof(float)),
+                  sirt_scratch_bytes(p));
 }
 
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
@@ -200,9 +216,12 @@ int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
     return p->n_bil_fast > 0 ? tsgb::bilinear_bytes(p) : 0;
   if (bp_kind != TSGB_BP_MATCHED) return fail(TSGB_ERR_INVALID, "unknown bp_kind");
   if (p->fine) return tsgb_bp_workspace_bytes(p->fine, bp_kind);
+  // the slice kernels' profiles and scratch volumes (and what the voxel-pair kernel
+  // needs, where the tuning picks that), or the row-pair weighted sinogram (two floats
+  // per pixel, kRowPad padding rows) and the z-lane kernel's [y][x][z] scratch volumes,
+  // whichever kernel runs
   if (tsgb::flat_bp(p)) return tsgb::flat_bp_bytes(p);
-  // row-pair weighted sinogram (two floats per pixel, kRowPad padding rows),
-  // then the z-lane kernel's [y][x][z] scratch volumes (either kernel may run)
+  if (p->flat) return std::max(tsgb::flat_bp_bytes(p), tsgb::bp_pairs_bytes(p->g));
   return tsgb::bp_pairs_bytes(p->g) + tsgb::bp_scratch_bytes(p);
 }
 
@@ -252,22 +271,21 @@ int tsgb_direct_bp(tsgb_projector* p, float* vol, const float* sino, int32_t add
   if (!p || !vol || !sino) return fail(TSGB_ERR_INVALID, "NULL projector or data pointer");
   if (bp_kind != TSGB_BP_MATCHED && bp_kind != TSGB_BP_BILINEAR)
     return fail(TSGB_ERR_INVALID, "unknown bp_kind");
-  const int64_t need = tsgb_bp_workspace_bytes(p, bp_kind);
+  const tsgb_projector* f = p->fine ? p->fine : p;  // (matched only)
+  const int64_t need =
+      bp_kind == TSGB_BP_MATCHED ? bp_bytes(f) : tsgb_bp_workspace_bytes(p, bp_kind);
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(TSGB_ERR_WORKSPACE,
                 "backprojection needs " + std::to_string(need) + " bytes of workspace");
   int rc = check_device(p);
   if (rc != TSGB_OK) return rc;
   cudaError_t e;
-  if (bp_kind == TSGB_BP_MATCHED && p->fine) {
-    // the transpose of the binning: the finer detector's matched backprojection of
-    // each pixel / d^2 spread over its block
-    e = cudaError_t(tsgb::launch_bp_matched(p->fine, vol, tsgb::spread_source(sino, p->det_ss),
-                                            additive != 0,
-                                            static_cast<float*>(workspace), stream));
-  } else if (bp_kind == TSGB_BP_MATCHED)
-    e = cudaError_t(tsgb::launch_bp_matched(p, vol, {sino}, additive != 0,
-                                            static_cast<float*>(workspace), stream));
+  if (bp_kind == TSGB_BP_MATCHED)
+    // (supersampled: the transpose of the binning, the finer detector's matched
+    // backprojection of each pixel / d^2 spread over its block)
+    e = cudaError_t(tsgb::launch_bp_matched(
+        f, vol, p->fine ? tsgb::spread_source(sino, p->det_ss) : tsgb::SinoSource{sino},
+        additive != 0, static_cast<float*>(workspace), stream, slices_only(f, workspace_bytes)));
   else
     e = cudaError_t(tsgb::launch_bp_bilinear(p, vol, sino, additive != 0,
                                              static_cast<float*>(workspace), stream));
@@ -380,7 +398,7 @@ int tsgb_direct_bp_angles(tsgb_projector* p, float* vol, const float* sino, int3
   if (p->fine) return fail(TSGB_ERR_INVALID, "angle ranges need detector supersampling 1");
   if (angle_begin < 0 || angle_end > p->g.nangles || angle_begin >= angle_end)
     return fail(TSGB_ERR_INVALID, "angle range outside 0 .. num_angles");
-  const int64_t need = tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED);
+  const int64_t need = bp_bytes(p);
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(TSGB_ERR_WORKSPACE,
                 "backprojection needs " + std::to_string(need) + " bytes of workspace");
@@ -388,6 +406,7 @@ int tsgb_direct_bp_angles(tsgb_projector* p, float* vol, const float* sino, int3
   if (rc != TSGB_OK) return rc;
   cudaError_t e = cudaError_t(tsgb::launch_bp_matched(p, vol, {sino}, additive != 0,
                                                       static_cast<float*>(workspace), stream,
+                                                      slices_only(p, workspace_bytes),
                                                       int(angle_begin), int(angle_end)));
   if (e != cudaSuccess) return cuda_fail(e, "backprojection launch");
   return TSGB_OK;
@@ -428,7 +447,7 @@ int tsgb_fdk_backproject(tsgb_projector* p, float* vol, const float* filtered, c
 }
 
 int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
-  if (!p || !out || n < 0 || n > 8) return fail(TSGB_ERR_INVALID, "bad stats arguments");
+  if (!p || !out || n < 0 || n > 10) return fail(TSGB_ERR_INVALID, "bad stats arguments");
   // FP and matched BP run on the finer detector when it is supersampled, plus
   // one binning / spreading launch
   const tsgb_projector* f = p->fine ? p->fine : p;
@@ -449,7 +468,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
       (tsgb::flat_bp(f) ? 1 + 2 * tsgb::flat_chunks(f)
                : chunks + sep_launches + ((f->n_general_bp > 0 || f->n_separable_bp == 0) ? 1 : 0)) +
       extra;
-  const int64_t vals[8] = {int64_t(f->layouts.size()),
+  const int64_t vals[10] = {int64_t(f->layouts.size()),
                            f->n_separable_bp,
                            f->n_general_bp,
                            fp_launches,
@@ -457,7 +476,12 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
                            (p->n_bil_fast > 0 ? (tsgb::bilinear_thin(p) ? 2 : 3) : 0) +
                                ((p->n_bil_slow > 0 || p->n_bil_fast == 0) ? 1 : 0),
                            tsgb_fp_workspace_bytes(p),
-                           tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED)};
+                           tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED),
+                           f->flat ? 1 : 0,
+                           f->n_separable_bp == 0   ? 0
+                           : tsgb::flat_bp(f)       ? 3
+                           : tsgb::bp_uses_zlane(f) ? 2
+                                                    : 1};
   for (int i = 0; i < n; ++i) out[i] = vals[i];
   return TSGB_OK;
 }

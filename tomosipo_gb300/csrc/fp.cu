@@ -607,8 +607,9 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   // voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360 4.56 / 6.52,
   // 64^3 / 96 0.057 / 0.241), except for thin, wide volumes, whose few voxels
   // along z leave its lanes idle (256^2 x 16 / 360 1.79 / 0.86, 256^2 x 40 1.95 /
-  // 1.57).
-  t.bp_kernel = thin_volume(p, 48) ? 0 : 1;
+  // 1.57). The slice kernels of parallel scans the same, on thinner volumes (256^2 x 16
+  // 0.91 / 0.85, 256^2 x 40 0.97 / 1.46).
+  t.bp_kernel = thin_volume(p, p->flat ? 16 : 48) ? 0 : 1;
   t.bp_shape = 2;
   return t;
 }

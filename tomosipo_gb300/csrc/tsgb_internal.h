@@ -316,7 +316,8 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
                             bool additive, char* workspace, int64_t item_bytes, int group,
                             void* stream);
 
-// The matched backprojector of det_v-along-z angles is the z-lane kernel
+// The matched backprojector of det_v-along-z angles, where it does not run slice by
+// slice (flat_bp), is the z-lane kernel
 // (bp_zlane.cu, column-major weighted sinogram) unless the tuning picks the
 // voxel-pair kernel (bp.cu, row-major) or the volume's (y, x) plane is too
 // large for the z-lane grid (fewer than 2^32 voxel columns keep its two passes
@@ -404,9 +405,9 @@ int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino
 // (sinogram resampled to the slices, scratch volumes), in pieces of as many angles as
 // about 2 GiB of line sums or profiles hold; the projections of
 // `items` stacked items with their workspaces item_bytes apart.
-// (up to 16 voxels along z a thin, wide volume keeps the voxel-pair kernel: 256^2
-// slice, 360 angles, 16 voxels 0.85 ms against 0.91, 40 voxels 1.46 against 0.97)
-inline bool flat_bp(const tsgb_projector* p) { return p->flat && !thin_volume(p, 16); }
+// (the tuning's bp_kernel 0 picks the voxel-pair backprojector, the default of thin,
+// wide volumes)
+inline bool flat_bp(const tsgb_projector* p) { return p->flat && p->tuning.bp_kernel == 1; }
 int64_t flat_fp_bytes(const tsgb_projector* p);
 int64_t flat_bp_bytes(const tsgb_projector* p);
 int flat_chunks(const tsgb_projector* p);
@@ -426,8 +427,10 @@ int launch_flat_bp(const tsgb_projector* p, float* vol, SinoSource sino, bool we
 int launch_fp(const tsgb_projector* p, const float* vol, float* sino, bool additive,
               float* workspace, void* stream, const FpSirt* sirt = nullptr, int angle_begin = 0,
               int angle_end = -1, bool copies_ready = false);
+// slices: slice by slice whatever the tuning picks (p->flat).
 int launch_bp_matched(const tsgb_projector* p, float* vol, SinoSource sino, bool additive,
-                      float* workspace, void* stream, int angle_begin = 0, int angle_end = -1);
+                      float* workspace, void* stream, bool slices = false, int angle_begin = 0,
+                      int angle_end = -1);
 int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, bool additive,
                        float* workspace, void* stream);
 

@@ -102,12 +102,12 @@ class Projector:
     def stats(self, device_index):
         """Plan statistics of the native projector (see tsgb_projector_stats)."""
         lib = _native.load()
-        out = (ctypes.c_int64 * 8)()
-        _native.check(lib.tsgb_projector_stats(self.handle(device_index), out, 8),
+        out = (ctypes.c_int64 * 10)()
+        _native.check(lib.tsgb_projector_stats(self.handle(device_index), out, 10),
                       "tsgb_projector_stats")
         keys = ["layouts", "separable_bp_angles", "general_bp_angles", "fp_launches",
                 "bp_matched_launches", "bp_bilinear_launches", "fp_workspace_bytes",
-                "bp_workspace_bytes"]
+                "bp_workspace_bytes", "fp_kernel", "bp_matched_kernel"]
         return dict(zip(keys, [int(v) for v in out]))
 
     TUNING_KEYS = ("fp_patch_rows", "fp_patch_cols", "fp_group_pairs", "fp_pair_layout",
