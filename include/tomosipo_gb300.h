@@ -74,9 +74,12 @@ int tsgb_projector_create(const tsgb_volume_desc* vol,
  * to garbage collection). Synchronises the projector's device. */
 int tsgb_projector_destroy(tsgb_projector* p);
 
-/* Bytes of device workspace ``tsgb_direct_fp`` / ``tsgb_direct_bp`` need
+/* Bytes of device workspace that suffice for ``tsgb_direct_fp`` and as the
+ * ``fp_workspace`` of a batched SIRT job, and that ``tsgb_direct_bp`` needs
  * (0 if none); a negative error code for a NULL projector or an unknown
- * bp_kind. No counterpart in the reference (ASTRA allocates internally). */
+ * bp_kind. A forward projection alone needs
+ * ``tsgb_fp_batch_workspace_bytes(p, 1)``. No counterpart in the reference
+ * (ASTRA allocates internally). */
 int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p);
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind);
 
@@ -104,7 +107,7 @@ int tsgb_direct_bp(tsgb_projector* p, float* vol, const float* sino,
  * launches: one ray launch over as many items as the workspace holds volume
  * copies for (up to 48; the query keeps that within 2 GiB, so projectors
  * whose copies are larger run one item after another); with
- * tsgb_fp_workspace_bytes, one after another on ``stream``. */
+ * tsgb_fp_batch_workspace_bytes(p, 1), one after another on ``stream``. */
 int64_t tsgb_fp_batch_workspace_bytes(const tsgb_projector* p, int64_t n);
 int tsgb_direct_fp_batch(tsgb_projector* p, const float* vol, float* sino, int64_t n,
                          int32_t additive, void* workspace, int64_t workspace_bytes,

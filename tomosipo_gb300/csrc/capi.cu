@@ -180,6 +180,13 @@ int64_t fine_sino_bytes(const tsgb_projector* p) {
   return (int64_t(f.rows) * f.nangles * f.cols * int64_t(sizeof(float)) + 255) / 256 * 256;
 }
 
+// A forward projection's own need: volume copies (pairs of floats), or the slice kernels'
+// copy and line sums, after the finer sinogram of a supersampled detector.
+int64_t fp_bytes(const tsgb_projector* p) {
+  if (p->fine) return fine_sino_bytes(p) + fp_bytes(p->fine);
+  return p->flat ? tsgb::flat_fp_bytes(p) : p->fp_workspace_elems * int64_t(2 * sizeof(float));
+}
+
 // What batched SIRT's backprojection keeps in the forward workspace: the slice kernels'
 // profiles and scratch volumes, or the voxel-pair kernel's first sum; else a sum volume
 // and the z-lane kernel's scratch volumes.
@@ -202,12 +209,9 @@ bool slices_only(const tsgb_projector* p, int64_t workspace_bytes) {
 
 int64_t tsgb_fp_workspace_bytes(const tsgb_projector* p) {
   if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
-  if (p->fine) return fine_sino_bytes(p) + tsgb_fp_workspace_bytes(p->fine);
-  // volume copies (pairs of floats), or the slice kernels' copy and line sums; batched
-  // SIRT backprojects there, by whichever kernel the tuning picks
-  return std::max(p->flat ? tsgb::flat_fp_bytes(p)
-                          : p->fp_workspace_elems * int64_t(2 * sizeof(float)),
-                  sirt_scratch_bytes(p));
+  // batched SIRT (without supersampling) backprojects in its forward workspace too, by
+  // whichever kernel the tuning picks
+  return p->fine ? fp_bytes(p) : std::max(fp_bytes(p), sirt_scratch_bytes(p));
 }
 
 int64_t tsgb_bp_workspace_bytes(const tsgb_projector* p, int32_t bp_kind) {
@@ -244,7 +248,7 @@ int tsgb_direct_fp(tsgb_projector* p, const float* vol, float* sino, int32_t add
                    void* workspace, int64_t workspace_bytes, void* stream) {
   g_last_error.clear();
   if (!p || !vol || !sino) return fail(TSGB_ERR_INVALID, "NULL projector or data pointer");
-  const int64_t need = tsgb_fp_workspace_bytes(p);
+  const int64_t need = fp_bytes(p);
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(TSGB_ERR_WORKSPACE, "forward projection needs " + std::to_string(need) +
                                         " bytes of workspace");
@@ -294,7 +298,8 @@ int tsgb_direct_bp(tsgb_projector* p, float* vol, const float* sino, int32_t add
 }
 
 int64_t tsgb_fp_batch_workspace_bytes(const tsgb_projector* p, int64_t n) {
-  const int64_t one = tsgb_fp_workspace_bytes(p);
+  if (!p) return fail(TSGB_ERR_INVALID, "projector is NULL");
+  const int64_t one = fp_bytes(p);
   if (one <= 0 || n <= 1 || p->fine || !tsgb::fp_multi_eligible(p)) return one;
   const int64_t group = tsgb::batch_group(n, one);
   return group > 1 ? group * one : one;
@@ -309,7 +314,7 @@ int tsgb_direct_fp_batch(tsgb_projector* p, const float* vol, float* sino, int64
   const size_t sino_elems = size_t(p->g.rows) * p->g.nangles * p->g.cols;
   // multi-job launches when the workspace holds the volume copies of every
   // item of a group (tsgb_fp_batch_workspace_bytes); else one after another
-  const int64_t one = tsgb_fp_workspace_bytes(p);
+  const int64_t one = fp_bytes(p);
   const int64_t group = one > 0 && workspace ? std::min<int64_t>({n, int64_t(tsgb::kMaxMultiJobs),
                                                                  workspace_bytes / one})
                                              : 0;
@@ -377,7 +382,7 @@ int tsgb_direct_fp_angles(tsgb_projector* p, const float* vol, float* sino, int3
   if (p->fine) return fail(TSGB_ERR_INVALID, "angle ranges need detector supersampling 1");
   if (angle_begin < 0 || angle_end > p->g.nangles || angle_begin >= angle_end)
     return fail(TSGB_ERR_INVALID, "angle range outside 0 .. num_angles");
-  const int64_t need = tsgb_fp_workspace_bytes(p);
+  const int64_t need = fp_bytes(p);
   if (need > 0 && (!workspace || workspace_bytes < need))
     return fail(TSGB_ERR_WORKSPACE, "forward projection needs " + std::to_string(need) +
                                         " bytes of workspace");

@@ -89,12 +89,14 @@ class Projector:
         return h
 
     def workspace_bytes(self, device_index, forward, bp_kind="matched"):
+        """Workspace of one projection (a batched SIRT job's: ``stats``'s
+        ``fp_workspace_bytes``, which holds its backprojection too)."""
         key = (device_index, forward, bp_kind)
         nbytes = self._workspace_bytes.get(key)
         if nbytes is None:
             lib = _native.load()
             h = self.handle(device_index)
-            nbytes = int(lib.tsgb_fp_workspace_bytes(h) if forward
+            nbytes = int(lib.tsgb_fp_batch_workspace_bytes(h, 1) if forward
                          else lib.tsgb_bp_workspace_bytes(h, BP_KINDS[bp_kind]))
             self._workspace_bytes[key] = nbytes
         return nbytes

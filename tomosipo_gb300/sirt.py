@@ -71,7 +71,7 @@ class SirtJobState:
             # the backprojector's row-pair layout (two floats per pixel) with two
             # zero detector rows above and below, read as padding
             self.res = torch.zeros(2 * (rows + 4) * angles * cols, device=device)
-            nbytes = A.projector.workspace_bytes(device.index, True)
+            nbytes = A.projector.stats(device.index)["fp_workspace_bytes"]
             self.ws = torch.empty(max(nbytes, 4) // 4, device=device)
 
     def tensors(self):
