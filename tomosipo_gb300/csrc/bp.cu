@@ -31,7 +31,7 @@
 // detector at the projected voxel centre, weighted so that it approximates
 // the transpose (voxel volume / pixel area / ray obliquity, times the cone
 // magnification squared). Angles whose projection keeps u and the depth along z
-// take bp_bilinear.cu (thin, wide volumes bp_bilinear_z_kernel here), the others
+// take bp_bilinear.cu or bp_bilinear_z_kernel here (bilinear_zlane), the others
 // bp_bilinear_kernel.
 #include <cuda_runtime.h>
 
@@ -1024,8 +1024,8 @@ __device__ __forceinline__ float detector_or_zero(const float* __restrict__ sino
   return __ldg(sino + ((size_t)iv * g.nangles + t) * g.cols + iu);
 }
 
-// Thin, wide volumes (thin_volume(p, 32)): the lanes of bp_bilinear.cu's kernel
-// would idle, so a thread owns a voxel column of 16 voxels along z instead.
+// Where bp_bilinear.cu's kernel would leave lanes idle or spend its time on the scratch
+// volume (bilinear_zlane), a thread owns a voxel column of 16 voxels along z instead.
 //
 // Quad copy of the sinogram for bp_bilinear_z_kernel: element (iv, t, iu) for
 // iv in -kRowPad .. rows + kRowPad - 1 and iu in -kColPad .. cols + kColPad - 1
@@ -1526,8 +1526,8 @@ void launch_bil_z(const tsgb_projector* p, const float4* quads, float* vol, bool
   launch_bil_z_tile<kWeight, 8>(p, quads, vol, additive, angle_w, stream);
 }
 
-// Quad copy and the z-flat kernel of thin, wide volumes.
-void launch_bil_thin(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
+// Quad copy and the z-flat kernel of one thread per 16 voxels along z.
+void launch_bil_quads(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
                      bool additive, float* workspace, cudaStream_t stream) {
   const DeviceGeometry& g = p->g;
   const long long total = (long long)(g.rows + 2 * kRowPad) * g.nangles * (g.cols + 2 * kColPad);
@@ -1546,8 +1546,10 @@ void launch_bil_thin(const tsgb_projector* p, float* vol, const float* sino, con
 // The z-flat angles of the bilinear backprojection (angle_w: FDK's weights).
 void launch_bil_fast(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
                      bool additive, float* workspace, cudaStream_t stream) {
-  if (bilinear_thin(p))
-    launch_bil_thin(p, vol, sino, angle_w, additive, workspace, stream);
+  const BilWeight weight =
+      angle_w ? kBilFdk : p->g.kind == TSGB_CONE ? kBilCone : kBilParallel;
+  if (!bilinear_zlane(p, weight))
+    launch_bil_quads(p, vol, sino, angle_w, additive, workspace, stream);
   else
     launch_bilinear_zlane(p, vol, sino, angle_w, additive, workspace, stream);
 }

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "device_common.cuh"
 
@@ -249,16 +250,53 @@ void launch_run(const tsgb_projector* p, const float2* pairs, float* volt, const
         table, p->n_bil_fast, pairs, volt, g, nullptr);
 }
 
+// Ranges along z and voxels per lane: at most 5, ranges of near-equal length.
+int z_ranges(const DeviceGeometry& g) { return ((g.nz + 31) / 32 + 4) / 5; }
+int z_run(const DeviceGeometry& g) {
+  const int ranges = z_ranges(g);
+  return ((g.nz + 31) / 32 + ranges - 1) / ranges;
+}
+
 int64_t pairs_bytes(const DeviceGeometry& g) {
   return (int64_t(padded_rows(g)) * padded_cols(g) * g.nangles * 8 + 255) / 256 * 256;
 }
 
 }  // namespace
 
+// The times of this kernel over those of one thread per 16 voxels and quads, as factors:
+//  * a voxel, cone 0.87, FDK 0.70, parallel 0.58 of the quads' time (256^3 / 360 angles:
+//    5.63 / 6.35, 4.56 / 6.0 and 4.20 / 9.8 ms), 1.15 times that with 2 voxels a lane;
+//  * lanes past the end of the volume and of the quads' runs of 16 (400 voxels take 480);
+//  * rows finer than half a voxel: a load's 32 lanes spread over more lines (128 x 192^2 /
+//    90 cone angles: 3, 4 and 6 rows a voxel 0.64 / 0.61, 0.75 / 0.67, 1.09 / 0.72 ms);
+//  * the scratch volume, written and read once, as much as 4.7 angles (256^3, 1, 3, 16
+//    and 64 cone angles: 110 / 35, 140 / 67, 337 / 277 and 1079 / 1117 us);
+//  * the quad kernel's threads, too few for the GPU below about 3e5 (64^3 / 180: 85 / 474).
+// Over 1140 sizes, angle counts and weights the faster of the two was missed by more than
+// 5 % at 31, and by 27 % at most. Up to 32 voxels along z a wide slice keeps the quads
+// (256^2 / 360: 16 voxels 0.79 ms against 1.09, 32 0.92 / 1.06); a slice or two on their
+// own a less wide one (180 angles: 176^2 0.24 ms against 0.29, 150^2 0.24 / 0.21).
+bool bilinear_zlane(const tsgb_projector* p, BilWeight weight) {
+  const DeviceGeometry& g = p->g;
+  if (thin_volume(p, 32) || (g.nz <= 2 && int64_t(g.nx) * g.ny > 24000)) return false;
+  const int run = z_run(g), quad_runs = (g.nz + 15) / 16;
+  const double lanes = 32.0 * run * z_ranges(g) / (16.0 * quad_runs);
+  const double voxel = (weight == kBilCone ? 0.87 : weight == kBilFdk ? 0.70 : 0.58) *
+                       (run == 2 ? 1.15 : 1.0);
+  const double rows = 1.0 + 0.37 * std::max(0.0, p->bil_row_step - 2.0);
+  const double fill = std::min(1.0, std::cbrt(double(g.nx) * g.ny * quad_runs / 3e5));
+  return fill * (voxel * lanes * rows + 4.7 / std::max(1, p->n_bil_fast)) < 1.0;
+}
+
 int64_t bilinear_bytes(const tsgb_projector* p) {
-  if (bilinear_thin(p))  // quad copy: four floats per element
-    return int64_t(padded_rows(p->g)) * p->g.nangles * padded_cols(p->g) * int64_t(4 * sizeof(float));
-  return pairs_bytes(p->g) + bp_volume_bytes(p->g);
+  // (a cone's projector serves the bilinear weights and FDK's)
+  const bool cone = p->g.kind == TSGB_CONE;
+  const bool a = bilinear_zlane(p, cone ? kBilCone : kBilParallel);
+  const bool b = cone ? bilinear_zlane(p, kBilFdk) : a;
+  const int64_t quads = int64_t(padded_rows(p->g)) * p->g.nangles * padded_cols(p->g) *
+                        int64_t(4 * sizeof(float));
+  return std::max(a && b ? int64_t(0) : quads,
+                  a || b ? pairs_bytes(p->g) + bp_volume_bytes(p->g) : int64_t(0));
 }
 
 int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino,
@@ -270,8 +308,7 @@ int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino
   const dim3 grid(unsigned((padded_cols(g) + 31) / 32), unsigned((padded_rows(g) + 31) / 32),
                   unsigned(std::min(g.nangles, 65535)));
   bilinear_pairs_kernel<<<grid, dim3(32, 8), 0, stream>>>(sino, pairs, g);
-  const int lanes = (g.nz + 31) / 32, ranges = (lanes + 4) / 5;
-  switch ((lanes + ranges - 1) / ranges) {
+  switch (z_run(g)) {
     case 1: launch_run<1, 12>(p, pairs, volt, angle_w, stream); break;
     case 2: launch_run<2, 10>(p, pairs, volt, angle_w, stream); break;
     case 3: launch_run<3, 8>(p, pairs, volt, angle_w, stream); break;

@@ -473,12 +473,14 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
       (tsgb::flat_bp(f) ? 1 + 2 * tsgb::flat_chunks(f)
                : chunks + sep_launches + ((f->n_general_bp > 0 || f->n_separable_bp == 0) ? 1 : 0)) +
       extra;
+  const tsgb::BilWeight bil =
+      p->g.kind == TSGB_CONE ? tsgb::kBilCone : tsgb::kBilParallel;
   const int64_t vals[10] = {int64_t(f->layouts.size()),
                            f->n_separable_bp,
                            f->n_general_bp,
                            fp_launches,
                            bp_launches,
-                           (p->n_bil_fast > 0 ? (tsgb::bilinear_thin(p) ? 2 : 3) : 0) +
+                           (p->n_bil_fast > 0 ? (tsgb::bilinear_zlane(p, bil) ? 3 : 2) : 0) +
                                ((p->n_bil_slow > 0 || p->n_bil_fast == 0) ? 1 : 0),
                            tsgb_fp_workspace_bytes(p),
                            tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED),

@@ -408,6 +408,8 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   p->n_sep_ax = int(std::count_if(sep_angles->begin(), sep_angles->end(),
                                   [&](int t) { return p->host_params[t].a == 2; }));
   p->n_bil_fast = int(bil_fast->size());
+  p->bil_row_step = 0.0;
+  for (int t : *bil_fast) p->bil_row_step += std::fabs(double(p->host_params[t].pv[0])) / p->n_bil_fast;
   p->n_bil_slow = int(bil_slow->size());
   return std::string();
 }

@@ -160,6 +160,7 @@ struct tsgb_projector {
   int flat_z0 = 0, flat_nz = 0;
   int n_bil_fast = 0;           // bilinear BP: angles for the z-flat kernel
   int n_bil_slow = 0;           // bilinear BP: angles for the general kernel
+  double bil_row_step = 0.0;    // detector rows per voxel along z (mean over n_bil_fast angles)
   tsgb::AngleParams* d_params = nullptr;
   tsgb::ColumnEntry* d_columns = nullptr;  // [nangles][cols]
   int* d_sep_angles = nullptr;             // angle ids for the separable BP kernel
@@ -393,10 +394,9 @@ inline bool thin_volume(const tsgb_projector* p, int nz) {
 // with FDK's weights angle_w (by angle id) or, if null, the bilinear ones; its
 // workspace (padded row pairs, scratch volume).
 int64_t bilinear_bytes(const tsgb_projector* p);
-// Thin, wide volumes keep one thread per voxel column (bp.cu) and a quad copy of
-// the sinogram (256^2 slice, 360 cone angles: 16 voxels along z 0.79 ms against
-// 1.09, 32 0.92 / 1.06, 48 1.84 / 1.69).
-inline bool bilinear_thin(const tsgb_projector* p) { return thin_volume(p, 32); }
+// Whether that kernel runs under these weights, or one thread per 16 voxels along z and a
+// quad copy of the sinogram (bp.cu).
+bool bilinear_zlane(const tsgb_projector* p, BilWeight weight);
 int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino,
                           const float* angle_w, bool additive, float* workspace, void* stream);
 
