@@ -592,10 +592,15 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   // Pairs along b halve the sampler's load instructions (the gather is bound
   // by L1 wavefronts) but double the copies' footprint: at 256^3 they are 11 %
   // faster, at 512^3 (a 1.1 GB pair copy) 12 % slower because the schedule's
-  // volume slab then spills L2. Default: pairs while a pair copy is <= 512 MB.
+  // volume slab then spills L2. Rows 4 to 28 voxels apart fetch as many lines from
+  // single voxels as from pairs, and twice as many voxels to a line: single voxels take
+  // 0.72 of 1.63 ms at 512 x 192^2 / 180 angles and 16 voxels, 1.15 of 1.32 at 4, 0.64
+  // of 0.81 at 24 (1.42 of 1.42 at 3, 0.66 of 0.56 at 32, where no two rows share a line).
+  // Default: pairs while a pair copy is <= 512 MB and rows are nearer or farther.
   int64_t largest = 0;
   for (const auto& L : p->layouts) largest = std::max<int64_t>(largest, L.elems());
-  t.fp_pair_layout = largest * 8 <= (int64_t(512) << 20) ? 1 : 0;
+  const bool spread_rows = p->row_pitch > 3.5 && p->row_pitch < 28.0;
+  t.fp_pair_layout = largest * 8 <= (int64_t(512) << 20) && !spread_rows ? 1 : 0;
   // Patches of 256 detector rows x 32 columns and groups of 64 angles: the
   // volume slab such a group crosses stays in L2 while it runs (fastest on a
   // 512^3 cone scan with a 512 x 768 detector and 1024 angles, and within

@@ -353,6 +353,11 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   // supersampled or fine detector; about 0.6 % of it for the benchmark's cone
   // scans): the voxel-pair kernel then runs as its fine-row variant.
   p->fine_rows = all_planes > 0.0 && fine_planes >= 0.25 * all_planes;
+  p->row_pitch = 0.0;
+  for (int t : *sep_angles) {
+    const AngleParams& ap = p->host_params[t];
+    p->row_pitch += std::fabs(double(ap.cb[2]) / ap.e[0]) / double(sep_angles->size());
+  }
   // Detector region of a 16 x 8 x 16 voxel box at the anchor for each general
   // angle (its corners widened by one voxel along a and b, as the kernel
   // does; pixels from floor(min) to ceil(max) of their projections): boxes

@@ -146,6 +146,9 @@ struct tsgb_projector {
   // detector rows lie closer than one voxel apart (|q_b step per row| < 1):
   // the voxel-pair kernel then runs as its fine-row variant.
   bool fine_rows = false;
+  // Voxels along z between detector rows at the volume's centre (mean over the separable
+  // angles, 0 if there are none).
+  double row_pitch = 0.0;
   // The general backprojector's voxel boxes may be 16 wide along x: the
   // detector region a 16 x 8 x 16 box at the volume's centre projects to, for
   // every general angle, stays within a third of the kernel's stage, which
