@@ -335,11 +335,14 @@ __device__ __forceinline__ void zlane_fine_columns(f32x2 (&acc)[kItems][kX][(kRu
 }
 
 // The columns of a list with rows less than half a voxel apart among them: every row
-// whose tent reaches the voxel.
+// whose tent reaches the voxel. The profile is built before the window's branch: inside
+// it every branch held the row loops of all the lane's voxels (128 x 192^2 /
+// 180 cone angles, 500 rows: 20.2 ms, now 7.2; the voxel-pair kernel 11.8).
 template <int kRun, int kItems, int kX>
 __device__ __forceinline__ void zlane_any_columns(f32x2 (&acc)[kItems][kX][(kRun + 1) / 2],
                                                   const float4 (&list)[34][4], int n, float zt,
                                                   const DeviceGeometry& g) {
+  constexpr int kPairs = (kRun + 1) / 2;
   for (int k = 0; k < n; ++k) {
     const float4 e0 = list[k][0], e1 = list[k][1], e2 = list[k][2], e3 = list[k][3];
     const float Sl = e0.x, inv = e1.x, C0 = (e1.y - zt) + e0.z;
@@ -356,7 +359,13 @@ __device__ __forceinline__ void zlane_any_columns(f32x2 (&acc)[kItems][kX][(kRun
         V = fmaf(tent(fmaf(float(iv - g.ov), Sl, Bj)), __ldg(col + (iv - g.ov) * kItems + i).x, V);
       return V;
     };
-    const auto profile = [&](int i, int jj) { return pack2(rows(i, 2 * jj), rows(i, 2 * jj + 1)); };
+    f32x2 V[kItems][kPairs];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+#pragma unroll
+      for (int jj = 0; jj < kPairs; ++jj)
+        V[i][jj] = pack2(rows(i, 2 * jj), 2 * jj + 1 < kRun ? rows(i, 2 * jj + 1) : 0.0f);
+    const auto profile = [&](int i, int jj) { return V[i][jj]; };
     window_dispatch<-1, kX>(acc, __float_as_int(e3.x), profile, pack2(e2.x, e2.y),
                             pack2(e2.z, e2.w));
   }
