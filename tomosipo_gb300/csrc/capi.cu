@@ -184,7 +184,7 @@ int64_t fine_sino_bytes(const tsgb_projector* p) {
 // copy and line sums, after the finer sinogram of a supersampled detector.
 int64_t fp_bytes(const tsgb_projector* p) {
   if (p->fine) return fine_sino_bytes(p) + fp_bytes(p->fine);
-  return p->flat ? tsgb::flat_fp_bytes(p) : p->fp_workspace_elems * int64_t(2 * sizeof(float));
+  return tsgb::flat_fp(p) ? tsgb::flat_fp_bytes(p) : p->fp_workspace_elems * int64_t(2 * sizeof(float));
 }
 
 // What batched SIRT's backprojection keeps in the forward workspace: the slice kernels'
@@ -461,7 +461,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
   const int64_t chunk = tsgb::fp_angle_chunk(f->g);
   // (parallel beams through flat.cu: copy, line sums, rows; resample, windows, out)
   const int64_t fp_launches =
-      f->flat ? 1 + 2 * tsgb::flat_chunks(f) + extra
+      tsgb::flat_fp(f) ? 1 + 2 * tsgb::flat_chunks(f) + extra
               : int64_t(f->layouts.size()) + (f->g.nangles + chunk - 1) / chunk + extra;
   // weight pass, both z-lane passes and the transpose out of their scratch (or
   // one launch per voxel-pair pass), the general kernel
@@ -484,7 +484,7 @@ int tsgb_projector_stats(const tsgb_projector* p, int64_t* out, int32_t n) {
                                ((p->n_bil_slow > 0 || p->n_bil_fast == 0) ? 1 : 0),
                            tsgb_fp_workspace_bytes(p),
                            tsgb_bp_workspace_bytes(p, TSGB_BP_MATCHED),
-                           f->flat ? 1 : 0,
+                           tsgb::flat_fp(f) ? 1 : 0,
                            f->n_separable_bp == 0   ? 0
                            : tsgb::flat_bp(f)       ? 3
                            : tsgb::bp_uses_zlane(f) ? 2

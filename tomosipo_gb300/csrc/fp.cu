@@ -511,7 +511,7 @@ int launch_fp_batch(const tsgb_projector* p, const float* vol, float* sino, int6
   const size_t sino_elems = size_t(g.rows) * g.nangles * g.cols;
   for (int64_t i0 = 0; i0 < n; i0 += group) {
     const int m = int(std::min<int64_t>(group, n - i0));
-    if (p->flat) {
+    if (flat_fp(p)) {
       const int rc = launch_flat_fp(p, vol + i0 * vol_elems, sino + i0 * sino_elems, additive,
                                     reinterpret_cast<float*>(workspace), stream, nullptr, 0,
                                     g.nangles, false, m, item_bytes);
@@ -553,7 +553,7 @@ int launch_fp(const tsgb_projector* p, const float* vol, float* sino, bool addit
               int angle_end, bool copies_ready) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (angle_end < 0) angle_end = p->g.nangles;
-  if (p->flat)
+  if (flat_fp(p))
     return launch_flat_fp(p, vol, sino, additive, workspace, stream, sirt, angle_begin, angle_end,
                           copies_ready, 1, 0);
   if (p->tuning.fp_pair_layout)

@@ -161,6 +161,9 @@ struct tsgb_projector {
   // Slices flat_z0 .. flat_z0 + flat_nz - 1 hold every slice that a detector row of
   // any angle interpolates (flat.cu works on these alone).
   int flat_z0 = 0, flat_nz = 0;
+  // The forward projection sums every one of those slices' lines (flat.cu); else, few
+  // rows far apart, each row's ray (fp.cu).
+  bool flat_forward = false;
   int n_bil_fast = 0;           // bilinear BP: angles for the z-flat kernel
   int n_bil_slow = 0;           // bilinear BP: angles for the general kernel
   double bil_row_step = 0.0;    // detector rows per voxel along z (mean over n_bil_fast angles)
@@ -410,6 +413,7 @@ int launch_bilinear_zlane(const tsgb_projector* p, float* vol, const float* sino
 // `items` stacked items with their workspaces item_bytes apart.
 // (the tuning's bp_kernel 0 picks the voxel-pair backprojector, the default of thin,
 // wide volumes)
+inline bool flat_fp(const tsgb_projector* p) { return p->flat && p->flat_forward; }
 inline bool flat_bp(const tsgb_projector* p) { return p->flat && p->tuning.bp_kernel == 1; }
 int64_t flat_fp_bytes(const tsgb_projector* p);
 int64_t flat_bp_bytes(const tsgb_projector* p);
