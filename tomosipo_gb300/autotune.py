@@ -17,11 +17,12 @@ job's operator tunes its part of the batch.
 
 Every schedule gives bit-identical results: only the order of independent
 tiles changes. For operators with the matched backprojector the tuner then
-times the backprojection under every kernel and warp shape it offers
-(``bp_kernel``: voxel-pair threads or z-lane warps; ``bp_shape``: the z-lane
-window, z run and warps per block. Parallel scans within one slice have one kernel,
-whose times then differ by noise only) and sets the fastest; these change only the
-order of fp32 sums. Results are cached per geometry (shapes, beam kind and a
+times the backprojection under every kernel and warp shape that differs for the
+operator (``bp_kernel``: voxel-pair threads, or z-lane warps or, for parallel scans
+within slices, the slice kernels; ``bp_shape``: the z-lane window, z run and warps per
+block) and sets the fastest; these change only the order of fp32 sums. What has no
+effect is not timed: the schedule of projections that run slice by slice, shapes that
+select the same launch. Results are cached per geometry (shapes, beam kind and a
 hash of the projection vectors) in memory and, if ``cache_path`` is given, in a
 JSON file. No counterpart in the reference, whose ASTRA launch shapes are
 fixed.
@@ -46,6 +47,23 @@ BP_CANDIDATES = ({"bp_kernel": 0, "bp_shape": 0},) + tuple(
     {"bp_kernel": 1, "bp_shape": k} for k in range(7))
 
 _cache = {}
+
+
+def bp_candidates(kernel, nz):
+    """The candidates of ``BP_CANDIDATES`` whose launches differ, for a projector that
+    runs ``kernel`` (``stats``'s ``bp_matched_kernel``) under ``bp_kernel`` 1 on volumes
+    of ``nz`` voxels along z (include/tomosipo_gb300.h, tsgb_tuning.bp_shape)."""
+    if kernel == 0:  # no angle takes these kernels
+        return ()
+    shapes = {2}
+    if kernel == 2:
+        lanes = (nz + 31) // 32
+        ranges = (lanes + 7) // 8
+        run = (lanes + ranges - 1) // ranges  # voxels along z per lane
+        shapes |= {3, 4} if run == 8 else set()
+        shapes |= {5} if run > 4 else set()
+        shapes |= {6} if run > 2 else set()
+    return tuple(c for c in BP_CANDIDATES if c["bp_kernel"] == 0 or c["bp_shape"] in shapes)
 
 
 def geometry_key(projector):
@@ -174,8 +192,12 @@ def autotune(A, device=None, repeats=None, cache_path=None, verbose=False, key=N
                 print(f"autotune {key}: {tuning} {ms:.3f} ms")
             return ms
 
-        best, best_ms, default_ms, trials = coordinate_descent(proj.get_tuning(dev.index),
-                                                               measure)
+        best = proj.get_tuning(dev.index)
+        if hasattr(proj, "stats") and proj.stats(dev.index)["fp_kernel"] == 1:
+            best_ms = default_ms = measure(best)  # slice by slice: no schedule
+            trials = 1
+        else:
+            best, best_ms, default_ms, trials = coordinate_descent(best, measure)
         proj.set_tuning(dev.index, **best)
         result = {"tuning": best, "ms": best_ms, "default_ms": default_ms, "trials": trials}
         if getattr(A, "backprojector", None) == "matched":
@@ -190,7 +212,10 @@ def autotune(A, device=None, repeats=None, cache_path=None, verbose=False, key=N
                     print(f"autotune {key}: {tuning} BP {ms:.3f} ms")
                 return ms
 
-            best, bp_ms, bp_default_ms, bp_trials = fastest_candidate(best, BP_CANDIDATES,
+            proj.set_tuning(dev.index, bp_kernel=1)
+            candidates = bp_candidates(proj.stats(dev.index)["bp_matched_kernel"],
+                                       proj.vol_shape[0])
+            best, bp_ms, bp_default_ms, bp_trials = fastest_candidate(best, candidates,
                                                                       measure_bp)
             proj.set_tuning(dev.index, **best)
             result.update(tuning=best, bp_ms=bp_ms, bp_default_ms=bp_default_ms,
