@@ -73,6 +73,7 @@ struct tsgb_sirt_batch {
   int device = -1;
   std::vector<tsgb_sirt_job> jobs;  // largest first
   std::vector<int> index;           // jobs[k] is the caller's job index[k]
+  std::vector<int> layout;          // the layout job k's residual was last written in (-1: none)
   std::vector<Unit> units;          // largest first; unit u runs on stream u % streams
   std::vector<cudaStream_t> streams;
   std::vector<cudaEvent_t> joins;
@@ -127,6 +128,7 @@ int tsgb_sirt_batch_create(const tsgb_sirt_job* jobs, int32_t n_jobs, tsgb_sirt_
   for (int i : order) {
     b->jobs.push_back(jobs[i]);
     b->index.push_back(i);
+    b->layout.push_back(-1);
   }
   // units: each large job alone; the small ones by copy layout, in groups of
   // at most kMaxMultiJobs (a group of one is a plain unit)
@@ -179,11 +181,31 @@ int tsgb_sirt_batch_create(const tsgb_sirt_job* jobs, int32_t n_jobs, tsgb_sirt_
 
 namespace {
 
+// Layouts of a job's residual: row-major pairs, column-major pairs, a plain sinogram.
+enum { kRowPairs = 0, kColumnPairs = 1, kPlain = 2 };
+
+// Before job J's residual is written in a layout other than the last one's (the tuning
+// was changed between iterations): the padding of one holds values of another.
+cudaError_t enter_layout(const tsgb_sirt_job& J, int layout, int& last, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  if (last >= 0 && last != layout) {
+    const tsgb::DeviceGeometry& g = J.projector->g;
+    e = cudaMemsetAsync(J.residual, 0,
+                        size_t(g.rows + 2 * tsgb::kRowPad) * g.nangles * g.cols * sizeof(float2), s);
+  }
+  last = layout;
+  return e;
+}
+
 // One SIRT iteration of job J on its own launches.
-cudaError_t iterate_job(const tsgb_sirt_job& J, cudaStream_t s) {
-  const tsgb::FpSirt sirt{J.sino, J.R, J.residual, tsgb::bp_uses_zlane(J.projector) ? 1 : 0,
-                          tsgb::flat_bp(J.projector) ? 1 : 0};
-  cudaError_t e = cudaError_t(tsgb::launch_fp(J.projector, J.vol, nullptr, false, J.fp_workspace, s, &sirt));
+cudaError_t iterate_job(const tsgb_sirt_job& J, int& last_layout, cudaStream_t s) {
+  const int layout = tsgb::flat_bp(J.projector)        ? kPlain
+                     : tsgb::bp_uses_zlane(J.projector) ? kColumnPairs
+                                                        : kRowPairs;
+  const tsgb::FpSirt sirt{J.sino, J.R, J.residual, layout == kColumnPairs, layout == kPlain};
+  cudaError_t e = enter_layout(J, layout, last_layout, s);
+  if (e == cudaSuccess)
+    e = cudaError_t(tsgb::launch_fp(J.projector, J.vol, nullptr, false, J.fp_workspace, s, &sirt));
   // the forward workspace is free once the residual is written: it holds the
   // first backprojection pass's sum
   if (e == cudaSuccess)
@@ -263,19 +285,28 @@ int iterate_counts(tsgb_sirt_batch* b, const std::vector<int>& count, cudaStream
   // job's iterations stay in order on its stream, units never wait for each
   // other.
   std::vector<const tsgb_sirt_job*> members;
+  std::vector<int> member_ids;
   for (int it = 0; it < iterations && e == cudaSuccess; ++it) {
     for (size_t u = 0; u < b->units.size() && e == cudaSuccess; ++u) {
       const Unit& U = b->units[u];
       cudaStream_t s = b->streams[u % K];
       members.clear();
+      member_ids.clear();
       for (int k : U.jobs)
-        if (it < count[k]) members.push_back(&b->jobs[k]);
+        if (it < count[k]) {
+          members.push_back(&b->jobs[k]);
+          member_ids.push_back(k);
+        }
       if (members.empty()) continue;
-      if (U.multi && members.size() > 1)
-        e = iterate_group(members, U.pair_layout, s);
-      else
-        for (size_t m = 0; m < members.size() && e == cudaSuccess; ++m)
-          e = iterate_job(*members[m], s);
+      // (jobs tuned off the group's kernels since take launches of their own)
+      bool group = U.multi && members.size() > 1;
+      for (const tsgb_sirt_job* J : members)
+        group = group && multi_eligible(J->projector) &&
+                (J->projector->tuning.fp_pair_layout != 0) == U.pair_layout;
+      for (size_t m = 0; m < members.size() && e == cudaSuccess; ++m)
+        e = group ? enter_layout(*members[m], kRowPairs, b->layout[member_ids[m]], s)
+                  : iterate_job(*members[m], b->layout[member_ids[m]], s);
+      if (group && e == cudaSuccess) e = iterate_group(members, U.pair_layout, s);
     }
   }
   for (int k = 0; k < K && e == cudaSuccess; ++k) {
