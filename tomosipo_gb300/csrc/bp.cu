@@ -1543,15 +1543,30 @@ void launch_bil_quads(const tsgb_projector* p, float* vol, const float* sino, co
     launch_bil_z<kBilParallel>(p, quads, vol, additive, nullptr, stream);
 }
 
-// The z-flat angles of the bilinear backprojection (angle_w: FDK's weights).
+// Bilinear backprojection of any angles (ids of n of them), without a workspace.
+void launch_bil_general(const tsgb_projector* p, const int* angles, int n, float* vol,
+                        const float* sino, const float* angle_w, bool additive,
+                        cudaStream_t stream) {
+  const DeviceGeometry& g = p->g;
+  const dim3 grid((g.nx + kBpX - 1) / kBpX, (g.ny + kBpY - 1) / kBpY,
+                  (g.nz + kRunZBil - 1) / kRunZBil);
+  bp_bilinear_kernel<<<grid, dim3(kBpX, kBpY), 0, stream>>>(p->d_params, angles, n, sino, vol, g,
+                                                            additive ? 1 : 0, angle_w);
+}
+
+// The z-flat angles of the bilinear backprojection (angle_w: FDK's weights). Quads are
+// 16-byte loads: in a caller's workspace that does not start on 16 bytes the general
+// kernel runs instead.
 void launch_bil_fast(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
                      bool additive, float* workspace, cudaStream_t stream) {
   const BilWeight weight =
       angle_w ? kBilFdk : p->g.kind == TSGB_CONE ? kBilCone : kBilParallel;
-  if (!bilinear_zlane(p, weight))
-    launch_bil_quads(p, vol, sino, angle_w, additive, workspace, stream);
-  else
+  if (bilinear_zlane(p, weight))
     launch_bilinear_zlane(p, vol, sino, angle_w, additive, workspace, stream);
+  else if (reinterpret_cast<uintptr_t>(workspace) % sizeof(float4) != 0)
+    launch_bil_general(p, p->d_bil_fast, p->n_bil_fast, vol, sino, angle_w, additive, stream);
+  else
+    launch_bil_quads(p, vol, sino, angle_w, additive, workspace, stream);
 }
 
 }  // namespace
@@ -1559,39 +1574,29 @@ void launch_bil_fast(const tsgb_projector* p, float* vol, const float* sino, con
 int launch_bp_bilinear(const tsgb_projector* p, float* vol, const float* sino, bool additive,
                        float* workspace, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const DeviceGeometry& g = p->g;
-  const dim3 block(kBpX, kBpY);
   bool written = false;
   if (p->n_bil_fast > 0) {
     launch_bil_fast(p, vol, sino, nullptr, additive, workspace, stream);
     written = true;
   }
-  if (p->n_bil_slow > 0 || !written) {
-    const dim3 grid((g.nx + kBpX - 1) / kBpX, (g.ny + kBpY - 1) / kBpY,
-                    (g.nz + kRunZBil - 1) / kRunZBil);
-    bp_bilinear_kernel<<<grid, block, 0, stream>>>(p->d_params, p->d_bil_slow, p->n_bil_slow, sino,
-                                                   vol, g, (additive || written) ? 1 : 0, nullptr);
-  }
+  if (p->n_bil_slow > 0 || !written)
+    launch_bil_general(p, p->d_bil_slow, p->n_bil_slow, vol, sino, nullptr, additive || written,
+                       stream);
   return int(cudaGetLastError());
 }
 
 int launch_bp_fdk(const tsgb_projector* p, float* vol, const float* sino, const float* angle_w,
                   bool additive, float* workspace, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const DeviceGeometry& g = p->g;
   bool written = false;
   if (p->n_bil_fast > 0) {
     launch_bil_fast(p, vol, sino, angle_w, additive, workspace, stream);
     written = true;
   }
-  if (p->n_bil_slow > 0 || !written) {
-    // angles whose projection depends on z (tilted detectors, rotated scans)
-    const dim3 grid((g.nx + kBpX - 1) / kBpX, (g.ny + kBpY - 1) / kBpY,
-                    (g.nz + kRunZBil - 1) / kRunZBil);
-    bp_bilinear_kernel<<<grid, dim3(kBpX, kBpY), 0, stream>>>(
-        p->d_params, p->d_bil_slow, p->n_bil_slow, sino, vol, g, (additive || written) ? 1 : 0,
-        angle_w);
-  }
+  // angles whose projection depends on z (tilted detectors, rotated scans)
+  if (p->n_bil_slow > 0 || !written)
+    launch_bil_general(p, p->d_bil_slow, p->n_bil_slow, vol, sino, angle_w, additive || written,
+                       stream);
   return int(cudaGetLastError());
 }
 
