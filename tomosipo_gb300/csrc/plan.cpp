@@ -198,7 +198,7 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
   p->layouts.clear();
   columns->assign(size_t(g.nangles) * g.cols, ColumnEntry{});
   sep_angles->clear();
-  p->fine_rows = false;
+  p->fine_rows = p->half_rows = false;
   // (the flat kernels' column lists hold 32-bit column indexes, and they step through
   // their volume copy, with its border on both in-slice axes, in 32-bit offsets)
   p->flat = !cone && int64_t(g.nangles) * g.cols < (int64_t(1) << 32) &&
@@ -340,6 +340,10 @@ std::string build_plan(const tsgb_volume_desc* vol, const tsgb_projection_desc* 
       for (int iu = 0; iu < g.cols; ++iu) {
         const ColumnEntry& c = (*columns)[size_t(t) * g.cols + iu];
         double lo = k_lo, hi = k_hi;
+        // (nearest at one end, or where the step changes sign)
+        const double end_lo = double(c.R) + k_lo * c.S, end_hi = double(c.R) + k_hi * c.S;
+        p->half_rows = p->half_rows || end_lo * end_hi <= 0.0 ||
+                       std::min(std::fabs(end_lo), std::fabs(end_hi)) < 0.501;
         if (c.S != 0.0f) {
           const double a = (-1.0 - double(c.R)) / double(c.S), b = (1.0 - double(c.R)) / double(c.S);
           lo = std::max(lo, std::floor(std::min(a, b)) + 1.0);

@@ -146,6 +146,8 @@ struct tsgb_projector {
   // detector rows lie closer than one voxel apart (|q_b step per row| < 1):
   // the voxel-pair kernel then runs as its fine-row variant.
   bool fine_rows = false;
+  // On some of them rows lie less than half a voxel apart.
+  bool half_rows = false;
   // Voxels along z between detector rows at the volume's centre (mean over the separable
   // angles, 0 if there are none).
   double row_pitch = 0.0;
