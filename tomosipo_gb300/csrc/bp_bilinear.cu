@@ -278,7 +278,7 @@ int64_t pairs_bytes(const DeviceGeometry& g) {
 // own a less wide one (180 angles: 176^2 0.24 ms against 0.29, 150^2 0.24 / 0.21).
 bool bilinear_zlane(const tsgb_projector* p, BilWeight weight) {
   const DeviceGeometry& g = p->g;
-  if (thin_volume(p, 32) || (g.nz <= 2 && int64_t(g.nx) * g.ny > 24000)) return false;
+  if (thin_volume(p, 32, 1 << 15) || (g.nz <= 2 && int64_t(g.nx) * g.ny > 24000)) return false;
   const int run = z_run(g), quad_runs = (g.nz + 15) / 16;
   const double lanes = 32.0 * run * z_ranges(g) / (16.0 * quad_runs);
   const double voxel = (weight == kBilCone ? 0.87 : weight == kBilFdk ? 0.70 : 0.58) *

@@ -608,13 +608,24 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   t.fp_patch_rows = 256 / kFpRows;
   t.fp_patch_cols = 32 / 8;
   t.fp_group_pairs = 32;
-  // Matched backprojection: the z-lane kernel (ms per call against the
-  // voxel-pair kernel: 512^3 / 1024 angles 99.7 / 144.5, 256^3 / 360 4.56 / 6.52,
-  // 64^3 / 96 0.057 / 0.241), except for thin, wide volumes, whose few voxels
-  // along z leave its lanes idle (256^2 x 16 / 360 1.79 / 0.86, 256^2 x 40 1.95 /
-  // 1.57). The slice kernels of parallel scans the same, on thinner volumes (256^2 x 16
-  // 0.91 / 0.85, 256^2 x 40 0.97 / 1.46).
-  t.bp_kernel = thin_volume(p, p->flat ? 16 : 48) ? 0 : 1;
+  // Matched backprojection: the z-lane kernel, or the slice kernels, except for volumes
+  // so thin that most of a warp's 32 lanes along z idle, and so wide that the voxel-pair
+  // kernel's threads fill the GPU all the same. Times over the voxel-pair kernel's, 60 to
+  // 360 angles:
+  //    voxels along z        16            32            48            64
+  //    184^2  z-lane        0.64          0.61          0.56          0.49
+  //           slices        0.55          0.55          0.57          0.52
+  //    256^2  z-lane     1.29 - 1.35   1.05 - 1.11   0.79 - 0.84   0.61 - 0.68
+  //           slices     0.96 - 1.03   0.86 - 0.90   0.68 - 0.69   0.44 - 0.51
+  //    384^2  z-lane        2.48          1.35          1.01          0.78
+  //           slices        1.86          0.96          0.76          0.58
+  //    512^2  z-lane     2.37 - 2.59   1.48 - 1.61   1.06 - 1.15   0.82 - 0.89
+  //           slices     1.72 - 1.73   0.99 - 1.11   0.74 - 0.85   0.57 - 0.65
+  // (one call alone. Stacked items and batched SIRT jobs share the voxel-pair kernel's
+  // launches, which then fill the GPU with narrower volumes too: batched SIRT of 8 jobs of 184^2, 90
+  // angles, 16, 32 and 48 voxels: 1.68, 1.28 and 1.11, slices 1.51, 1.10 and 0.91.)
+  t.bp_kernel = p->flat ? !(thin_volume(p, 16, 1 << 15) || thin_volume(p, 32, 1 << 18))
+                        : !thin_volume(p, 48, 1 << 15);
   t.bp_shape = 2;
   return t;
 }

@@ -393,10 +393,10 @@ void launch_zlane_out(const DeviceGeometry& g, int out_mode, const float* volt0,
                       const float* volt1, long long item_volt, int zs, int first_z, int n_z,
                       float* vol, const float* C, int items, void* stream);
 
-// Volumes of at most nz voxels along z and 2^15 or more in the slice: they leave
+// Volumes of at most nz voxels along z and `columns` or more in the slice: they leave
 // most of the z-lane kernels' lanes idle, and fill the GPU without them.
-inline bool thin_volume(const tsgb_projector* p, int nz) {
-  return p->g.nz <= nz && int64_t(p->g.nx) * p->g.ny >= (int64_t(1) << 15);
+inline bool thin_volume(const tsgb_projector* p, int nz, int64_t columns) {
+  return p->g.nz <= nz && int64_t(p->g.nx) * p->g.ny >= columns;
 }
 // Bilinear backprojection of the z-flat angles (bp_bilinear.cu): vol (= or +=),
 // with FDK's weights angle_w (by angle id) or, if null, the bilinear ones; its
