@@ -173,6 +173,12 @@ def autotune(A, device=None, repeats=None, cache_path=None, verbose=False, key=N
     if hit is None and cache_path and os.path.exists(cache_path):
         hit = _load_file(cache_path).get(key)
     if hit is not None:
+        if hit["tuning"].get("bp_kernel") == 0 and "bp_candidates" not in hit:
+            # stored when slice scans ran the slice kernels whatever the tuning said, or
+            # before there were any: its times did not choose between the two
+            proj.set_tuning(dev.index, bp_kernel=1)
+            if proj.stats(dev.index)["bp_matched_kernel"] == 3:
+                hit = dict(hit, tuning=dict(hit["tuning"], bp_kernel=1))
         proj.set_tuning(dev.index, **hit["tuning"])
         _cache[key] = hit
         return dict(hit, cached=True)
@@ -219,7 +225,7 @@ def autotune(A, device=None, repeats=None, cache_path=None, verbose=False, key=N
                                                                       measure_bp)
             proj.set_tuning(dev.index, **best)
             result.update(tuning=best, bp_ms=bp_ms, bp_default_ms=bp_default_ms,
-                          bp_trials=bp_trials)
+                          bp_trials=bp_trials, bp_candidates=len(candidates))
     _cache[key] = result
     if cache_path:
         data = _load_file(cache_path)
