@@ -217,8 +217,8 @@ int tsgb_sirt_batch_destroy(tsgb_sirt_batch* b);
 
 /* Launch schedule of a projector's forward projection (the order of its
  * independent tiles; a tile is 32 detector rows x 8 columns of one pair of
- * adjacent angles, run as blocks of 4 columns). The detector is cut into patches of fp_patch_rows x
- * fp_patch_cols tiles and the angles into groups of fp_group_pairs pairs;
+ * adjacent angles, run as blocks of 4 columns). The detector is cut into
+ * patches of fp_patch_rows x fp_patch_cols tiles and the angles into groups of fp_group_pairs pairs;
  * a group's tiles over one patch run together, so the volume slab their rays
  * cross is read from HBM once and reused from L2 across the group's angles.
  * Any values >= 1 give bit-identical results; they have no effect on parallel

@@ -11,17 +11,19 @@
 // plus two kernels, with no element-wise passes.
 //
 // Small jobs on the voxel-pair backprojector (at most 128^3 voxels, no tilted
-// detectors; by default volumes thin along z and wide) are grouped, up to kMaxMultiJobs at a time, into multi-job
-// launches: one forward launch and one launch per backprojection pass cover
-// the whole group, each block running one tile of one job exactly as that
-// job's own launch would (the job descriptors travel as __grid_constant__
-// kernel arguments, so the per-job kernels keep their registers). A small
-// job's voxel-pair backprojection alone fills a fraction of the SMs for a time set
+// detectors; by default volumes thin along z and wide) are grouped, up to
+// kMaxMultiJobs at a time, into multi-job launches: one forward launch and one
+// launch per backprojection pass cover the whole group, each block running one
+// tile of one job exactly as that job's own launch would (the job descriptors
+// travel as __grid_constant__ kernel arguments, so the per-job kernels keep their
+// registers). A small job's voxel-pair backprojection alone fills a fraction of the SMs for a time set
 // by its angle count, whatever its volume; in a group its blocks queue behind the
-// others' and the SMs stay busy. Other jobs keep their own launches, on several streams: the z-lane
-// and slice kernels fill more of the GPU with a small volume alone (36 jobs of side
-// <= 128, 30 iterations: 0.77 s here and 0.83 s one after another; on the voxel-pair
-// kernel 1.13 s in groups and 1.76 s).
+// others' and the SMs stay busy. Other jobs keep their own launches, on several
+// streams: the z-lane and slice kernels fill more of the GPU with a small volume alone
+// (36 jobs of side <= 128, 30 iterations: 0.77 s here and 0.83 s one after another; on
+// the voxel-pair kernel 1.13 s in groups and 1.76 s). Volumes of a few slices leave
+// those kernels' lanes idle, and groups would be faster (24 cone jobs of 1 x 128^2 / 90:
+// 3.3 ms an iteration, in groups 1.8).
 //
 // Work units (a large job, or a group of small ones) are spread over a small
 // pool of streams (largest first, round robin), forked from and joined back

@@ -541,8 +541,9 @@ __global__ void __launch_bounds__(128)
 // A staged pixel is its 1 / den and its weighted value: the numerators of q_a - i
 // and q_b - j are affine in the pixel's indexes for a voxel, so a candidate takes
 // two multiply-adds and two products with 1 / den instead of the four coefficients
-// of its ray (20 bytes staged per pixel instead of 8). Measured at 256^3 / 360 tilted angles: 34.6 -> 24.7 ms, 24.4 ms with 4 x 4 voxels per
-// half-warp on rows 4 (mod 8) pixels apart; 91 ms for one thread per voxel.
+// of its ray (20 bytes staged per pixel instead of 8). Measured at 256^3 / 360 tilted
+// angles: 34.6 -> 24.7 ms, 24.4 ms with 4 x 4 voxels per half-warp on rows 4 (mod 8)
+// pixels apart; 91 ms for one thread per voxel.
 // ncu at 120 x 152 x 161 / 180 angles: issue 68 % busy at 3 blocks per SM (80
 // registers), L1 and shared memory 47 %, 136 thread instructions per voxel and
 // angle for six candidates.

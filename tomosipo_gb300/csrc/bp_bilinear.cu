@@ -16,9 +16,9 @@
 // voxel columns (the block's other warps) read the same detector columns from L1.
 // Results go to a z-fastest scratch volume, which launch_zlane_out transposes.
 //
-// The two 8-byte loads per voxel bound it: about 80 % of the L1 data pipe at 320^3 /
-// 500 FDK angles, 10.6 ms against 14.5 for one thread per voxel column and 16-byte
-// quads (14 ms before the blocks ran in patches: a quarter of the L2 reads missed).
+// The two 8-byte loads per voxel bound it: 95 % of the L1 data pipe at 320^3 / 500 FDK
+// angles, 10.6 ms against 14.5 for one thread per voxel column and 16-byte quads (14 ms
+// before the blocks ran in patches: a quarter of the L2 reads missed).
 #include <cuda_runtime.h>
 
 #include <algorithm>

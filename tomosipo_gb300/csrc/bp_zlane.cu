@@ -405,8 +405,8 @@ struct ZlaneArgs {
 // lane per angle or column instead of by all lanes alike: 32 angles' column
 // ranges at a time, then the ranges flattened into a list and each list entry's
 // table entry, window position, row step and address by its own lane, kept in
-// shared memory (a column is then two 16-byte broadcast reads). With all lanes
-// alike this was 30 instructions per angle and 25 per column, which a run of
+// shared memory (a column is then three 16-byte broadcast reads and an 8-byte one). With
+// all lanes alike this was 30 instructions per angle and 25 per column, which a run of
 // few voxels along z does not hide.
 //
 // kItems = 2: a warp works on two stacked items at once (float4 elements): they share
@@ -612,14 +612,24 @@ void launch_zlane_shape(ZlaneArgs& A, int groups, cudaStream_t stream) {
 // Warp shapes, by the voxels along z per lane (`run`, from the volume's nz: at
 // most 8, ranges of near-equal length along z). Wider windows share a column's
 // profile between more voxels ((kX + 1) / kX columns per voxel), as long as the
-// accumulators and the two load stages fit the registers. Measured (GB300):
-// run 8, 512^3 / 1024 angles: 5 x 8 warps 94.0 ms, 3 x 8 101.0, 4 x 8 95.5,
-// 6 x 8 over 100; run 6, helical 170 x 190 x 181 / 257: 6 x 4 warps
-// 2.76 ms (forward projection included), 5 x 4 2.80, 4 x 4 2.88; run 3, SIRT at
-// 96^3: 8 x 4 warps 1.61 ms, 4 x 4 1.66, 6 x 4 1.71; run 4, 8 x 128^3: all
-// within 2 %,
-// 128^3 / 200: 6 x 4 warps 0.407, 8 x 4 0.431. The tuning's bp_shape 3 and 4 force other windows for run 8, 5 and
-// 6 cap the run at 4 and 2; any other value takes this rule.
+// accumulators and the two load stages fit the registers. Measured (GB300, window x
+// warps per block; runs 3, 4, 6 and 8 when each was chosen, before later steps that
+// serve all windows alike):
+//   run 8, 512^3 / 1024 angles: 5 x 8 94.0 ms, 4 x 8 95.5, 3 x 8 101.0, 6 x 8 over 100
+//   run 7, 224 x 224^2 / 200: 5 x 8 2.39 ms, 6 x 8 2.34, 4 x 8 2.41, 3 x 8 2.76;
+//          224 x 100^2 / 120: 0.364 ms, 0.392, 0.395, 0.399
+//   run 6, helical 170 x 190 x 181 / 257, forward projection included: 6 x 4 2.76 ms,
+//          5 x 4 2.80, 4 x 4 2.88
+//   run 5, 160 x 160^2 / 200: 6 x 4 1.02 ms, 5 x 4 1.07, 4 x 4 1.01, 8 x 4 1.01;
+//          160 x 96^2 / 120: 0.284 ms, 0.273, 0.252, 0.235
+//   run 4, 128^3 / 200: 6 x 4 0.407 ms, 8 x 4 0.431; 8 x 128^3: all within 2 %
+//   run 3, SIRT at 96^3: 8 x 4 1.61 ms, 4 x 4 1.66, 6 x 4 1.71
+//   run 2, 64^3 / 96: 4 x 8 66 us, 3 x 8 73, 6 x 8 87, 8 x 8 89; 64 x 192^2 / 180:
+//          657 us, 675, 640, 617
+//   run 1, 32 x 64^2 / 96: 4 x 8 64 us, 3 x 8 70, 6 x 8 83, 8 x 8 83; 32 x 192^2 / 180:
+//          643 us, 659, 621, 600
+// The tuning's bp_shape 3 and 4 force other windows for run 8, 5 and 6 cap the run at 4
+// and 2; any other value takes this rule.
 int zlane_run(const tsgb_projector* p) {
   const int shape = zlane_shape(p);
   const int most = shape == 5 ? 4 : shape == 6 ? 2 : 8;

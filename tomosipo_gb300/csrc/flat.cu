@@ -7,9 +7,10 @@
 //  * A ray's position along z, q_b = P + v R, is the same on every plane, so its
 //    plane sum over the four voxels around it is the z interpolation of two
 //    in-slice line sums. fp_flat_kernel computes the line sums S[theta][u][z] of
-//    every slice, two coalesced loads and two multiply-adds per plane and voxel
+//    every slice, two coalesced loads, a sample and its addition per plane and voxel
 //    along z, from one z-fastest copy of the volume; fp_flat_rows_kernel
-//    interpolates them to the detector rows.
+//    interpolates them to the detector rows. (Where the rows are few and lie far
+//    apart fp.cu follows their rays instead: flat_lines_pay in plan.cpp.)
 //  * The transpose: a detector column's vertical profile V(z) does not depend on
 //    the plane, so flat_resample_kernel computes it once per (angle, column)
 //    instead of once per plane, and bp_flat_kernel adds it to the voxels with
@@ -278,7 +279,8 @@ __global__ void __launch_bounds__(256)
 // (W = 1 when kWeighted: a SIRT residual holds W y). Rows at least a voxel apart:
 // the two rows around z, as saturating adds; else every row whose tent reaches z.
 // 32 (z) x 32 (column) tiles through shared memory: reads along u, writes along z. out
-// holds the angles from angle_begin on. blockIdx.x = column tile, blockIdx.y = z tile, blockIdx.z counts items * angles.
+// holds the angles from angle_begin on. blockIdx.x = column tile, blockIdx.y = z tile,
+// blockIdx.z counts items * angles.
 template <bool kWeighted, bool kSpread>
 __global__ void __launch_bounds__(256)
     flat_resample_kernel(const AngleParams* __restrict__ params,

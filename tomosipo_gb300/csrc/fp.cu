@@ -622,8 +622,9 @@ tsgb_tuning default_tuning(const tsgb_projector* p) {
   //    512^2  z-lane     2.37 - 2.59   1.48 - 1.61   1.06 - 1.15   0.82 - 0.89
   //           slices     1.72 - 1.73   0.99 - 1.11   0.74 - 0.85   0.57 - 0.65
   // (one call alone. Stacked items and batched SIRT jobs share the voxel-pair kernel's
-  // launches, which then fill the GPU with narrower volumes too: batched SIRT of 8 jobs of 184^2, 90
-  // angles, 16, 32 and 48 voxels: 1.68, 1.28 and 1.11, slices 1.51, 1.10 and 0.91.)
+  // launches, which then fill the GPU with narrower volumes too: batched SIRT of 8 jobs of
+  // 184^2, 90 angles, 16, 32 and 48 voxels: 1.68, 1.28 and 1.11, slices 1.51, 1.10 and
+  // 0.91.)
   t.bp_kernel = p->flat ? !(thin_volume(p, 16, 1 << 15) || thin_volume(p, 32, 1 << 18))
                         : !thin_volume(p, 48, 1 << 15);
   t.bp_shape = 2;

@@ -117,8 +117,9 @@ struct DeviceGeometry {
 };
 
 // Forward-projection tile order over one chunk of angles (tsgb_tuning):
-// groups of group_pairs angle pairs (or, like `pairs`, of blocks of two pairs), each run over the detector patch by
-// patch (patch_rows x patch_cols tiles), row tiles fastest inside a patch.
+// groups of group_pairs angle pairs (or, like `pairs`, of blocks of two pairs), each run
+// over the detector patch by patch (patch_rows x patch_cols tiles), row tiles fastest
+// inside a patch.
 struct FpSchedule {
   int row_blocks, col_blocks, pairs;  // tiles along rows and columns; angle pairs
   int patch_rows, patch_cols, group_pairs;
@@ -326,11 +327,11 @@ int launch_bp_matched_batch(const tsgb_projector* p, float* vol, const float* si
                             void* stream);
 
 // The matched backprojector of det_v-along-z angles, where it does not run slice by
-// slice (flat_bp), is the z-lane kernel
-// (bp_zlane.cu, column-major weighted sinogram) unless the tuning picks the
-// voxel-pair kernel (bp.cu, row-major) or the volume's (y, x) plane is too
-// large for the z-lane grid (fewer than 2^32 voxel columns keep its two passes
-// below 2^31 blocks for every shape, which hold at least 16 columns per block).
+// slice (flat_bp), is the z-lane kernel (bp_zlane.cu, column-major weighted sinogram)
+// unless the tuning picks the voxel-pair kernel (bp.cu, row-major) or the volume's
+// (y, x) plane is too large for the z-lane grid (fewer than 2^32 voxel columns keep its
+// two passes below 2^31 blocks for every shape, which hold at least 16 columns per
+// block).
 inline bool bp_uses_zlane(const tsgb_projector* p) {
   return p->tuning.bp_kernel == 1 &&
          int64_t(p->g.nx) * p->g.ny < (int64_t(1) << 32);
